@@ -12,40 +12,62 @@
 //   r >= num_samples is the reference's OutOfSamplesException (src/sketch.cpp:111-113,173-177).
 //
 // All rounds run inside one persistent kernel (k_boruvka), so a query is one launch and one
-// read-back instead of a host round trip per round.  Its blocks are co-resident (cooperative
-// launch) and meet at a grid barrier between phases; every barrier wait is bounded and reports
-// GS_DEV_ERR_TIMEOUT instead of spinning forever.  Several independent graphs ("tenants", each with
-// its own geometry and seed) can share one launch: their vertices are disjoint ranges of one vertex
-// space, their rounds advance together, and a tenant whose round was unmodified stops taking part,
-// so each tenant's partition, round count and out-of-samples status equal a query run alone.
+// read-back instead of a host round trip per round.  A graph's blocks meet at a barrier between
+// phases, in one of two scopes:
+//   cluster   one thread-block cluster per graph: the barrier is the hardware's, and any number of
+//             graphs share a launch without waiting for one another;
+//   grid      one graph over the whole GPU (cooperative launch); the barrier is a counter in
+//             global memory, and every wait on it is bounded and reports GS_DEV_ERR_TIMEOUT.
 //
-// Per round (five grid barriers):
-//   sizes       component sizes from the compressed parent array (warp-aggregated atomics); the
-//               size array also freezes the round's root set for sampling and unions
-//   accumulate  warps take runs of vertices from a shared counter, stage the members' column r and
-//               deterministic bucket in shared memory with cp.async, and XOR them into a register
-//               accumulator per component, flushed with red.global.xor when the component changes
-//   sample      round 0: every vertex samples its own sketch (an octet of lanes per vertex for one
-//               graph, a thread per vertex for many); later rounds: one warp per listed root, lane j
-//               checking bucket j (and j+32) with one XXH3 each (Bucket_Boruvka::is_good,
-//               include/bucket.h:65-67).  The deterministic bucket is zero / good first, else the first
-//               good bucket by depth (Sketch::sample, src/sketch.cpp:110-132); the component's
-//               accumulator row is zeroed once read, so rows are all zero between rounds and launches
-//   union       one thread per root unions its sampled edge, so thousands of DSU walks overlap
-//   compress    full path compression, sizes cleared, per-tenant stop / out-of-samples decisions
+// A round after round 0 (barriers between the phases):
+//   compress  parent[v] = root(v); in the same pass every component's size, every vertex's rank in
+//             its component and the largest component
+//   allocate  a root takes a run of the member list and one task per kPiece members
+//   place     every vertex writes itself at its component's run, at its rank
+//   gather    a warp per task loads its members' column r and deterministic bucket straight into
+//             registers, XORs them and - when the task is the whole component - samples the result
+//             and unions the sampled edge; pieces of larger components are XORed into their
+//             accumulator row
+//   big       components of several pieces (and the largest one) are sampled from their rows, which
+//             are zeroed once read: rows are all zero between rounds and launches
+// Sample (Bucket_Boruvka::is_good, include/bucket.h:65-67; Sketch::sample, src/sketch.cpp:110-132): the
+// deterministic bucket is zero / good first, else the first good bucket by depth, one lane per bucket.
+//
+// Complement (sketch sets that XOR to zero, because every update reached both endpoints): the XOR of
+// ALL of a graph's vertex sketches is zero, so its largest component's merged column equals the XOR of
+// the columns of every vertex outside it.  The largest component's members are then never listed or
+// read, and every gathered piece is folded into the largest component's row as well.
+//
+// Bound: latency.  A round is a chain of about a dozen dependent loads and five barriers, whatever the
+// graph's size, until the graph is large enough for the member columns' bytes to matter.
+// Measured (one query, us): V = 1024 199 -> 84, 16384 345 -> 195, 100003 835 -> 400, 131072 (R-MAT) 1062 ->
+// 560, 1000003 4810 -> 2020; 256 graphs of 256 to 16384 vertices 2230 -> 1080.  Before, every phase of every
+// graph was a grid phase of 444 blocks, all members were XORed into their component's row by atomics (82 of
+// them per vertex and round at V = 10^6), and roots were appended to a list, so that a round had six barriers.
 // DSU: CAS hooking of the larger root under the smaller (include/dsu.h:155-167 unions by random
 // priority instead), so every component's root is its minimum vertex id and labels are deterministic;
 // every walk is bounded by V+64 steps and reports GS_DEV_ERR_DSU_LIMIT.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
 #include "gs_dsu.cuh"
 #include "gs_internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
 constexpr uint32_t kGood = 0, kZero = 1, kFail = 2;
-constexpr uint32_t kAccRun = 16;                 // vertices a warp stages in shared memory at once
-constexpr uint32_t kAccGrab = 64;                // vertices a warp takes from the shared work counter
-constexpr uint32_t kThreads = 256;
-constexpr uint32_t kWarps = kThreads / 32;
+// Threads of a block.  Grid scope: one block per SM, so that the barrier has few arrivals.  Narrow
+// clusters: two blocks per SM, because a small graph's block mostly waits and another's fills in (256 graphs
+// of up to 16384 vertices: 1.08 ms against 1.23 with wide ones).  Wide clusters: few graphs, whose largest
+// one sets the time (8 graphs of up to 65536: 0.53 against 0.61 ms).
+enum Scope { kGrid = 0, kNarrow = 1, kWide = 2 };
+constexpr uint32_t threads_of(int scope) { return scope == kNarrow ? 512u : 1024u; }
+constexpr uint32_t kPiece = 16;                  // members of a component that one warp gathers
+constexpr uint32_t kGroup = 4;                   // member rows a warp asks for together
+constexpr uint32_t kRing = 2 * kGroup;           // member rows a warp has room for
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
@@ -55,14 +77,6 @@ __device__ __forceinline__ GsBucket ld_bucket_cg(const GsBucket* p) {
   const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(p));
   return GsBucket{v.x, v.y};
 }
-
-// 16-byte global -> shared copy that completes asynchronously (waited for with cp_async_wait_all)
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 __device__ __forceinline__ bool is_good(const GsBucket& b, uint64_t csmix) {
   return gs_hash_tail(gs_key_mix(b.alpha) ^ csmix) == b.gamma;
@@ -93,96 +107,162 @@ __device__ __forceinline__ void sample_warp(const GsBucket* col, const GsBucket*
   *idx = 0;
 }
 
-// Sketch::sample by one thread (round 0 of multi-graph launches, whose vertices are mostly sparse
-// and decide at the deterministic bucket): the column by depth, four buckets per batch of loads.
-__device__ __forceinline__ void sample_thread(const GsBucket* col, const GsBucket* det, uint32_t bkt, uint64_t csmix,
-                                              uint32_t* code, uint64_t* idx) {
-  const GsBucket d = ld_bucket_cg(det);
-  if (d.alpha == 0 && d.gamma == 0) { *code = kZero; *idx = 0; return; }
-  if (is_good(d, csmix)) { *code = kGood; *idx = d.alpha; return; }
-  for (uint32_t j0 = 0; j0 < bkt; j0 += 4) {
-    GsBucket b[4];
+// Sketch::sample of two vertices by an octet of lanes (round 0, where every vertex samples its own
+// sketch: eight vertices per warp).  Lane k of the octet checks depths k, k+8, ...; a vertex's answer is
+// the lowest good depth among the octet's lanes.  The deterministic buckets and the first eight depths of
+// both vertices are loaded together: most vertices are decided by them, and a pass is one DRAM latency.
+// Every lane of the warp runs the same passes (bkt is the graph's) and reaches every full-warp collective.
+__device__ __forceinline__ void sample_octet2(const GsBucket* const col[2], const GsBucket* const det[2], uint32_t bkt,
+                                              uint64_t csmix, const bool active[2], uint32_t code[2], uint64_t idx[2]) {
+  const uint32_t lane = lane_id(), sub = lane & 7u, oct = lane >> 3;
+  GsBucket d[2], b[2];
+  bool decided[2];
 #pragma unroll
-    for (int k = 0; k < 4; k++) b[k] = j0 + k < bkt ? ld_bucket_cg(col + j0 + k) : GsBucket{0, 0};
+  for (int u = 0; u < 2; u++) {
+    d[u] = active[u] ? ld_bucket_cg(det[u]) : GsBucket{0, 0};
+    b[u] = active[u] && sub < bkt ? ld_bucket_cg(col[u] + sub) : GsBucket{0, 0};
+  }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (j0 + k < bkt && is_good(b[k], csmix)) {
-        *code = kGood;
-        *idx = b[k].alpha;
-        return;
+  for (int u = 0; u < 2; u++) {
+    code[u] = kFail;
+    idx[u] = 0;
+    decided[u] = !active[u];
+    if (active[u]) {
+      if (d[u].alpha == 0 && d[u].gamma == 0) { code[u] = kZero; decided[u] = true; }
+      else if (is_good(d[u], csmix)) { code[u] = kGood; idx[u] = d[u].alpha; decided[u] = true; }
+    }
+  }
+  for (uint32_t j0 = 0; j0 < bkt; j0 += 8) {
+    if (__all_sync(0xffffffffu, decided[0] && decided[1])) break;
+    const uint32_t j = j0 + sub;
+    if (j0 > 0) {
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+        if (!decided[u] && j < bkt) b[u] = ld_bucket_cg(col[u] + j);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const uint32_t m = __ballot_sync(0xffffffffu, !decided[u] && j < bkt && is_good(b[u], csmix));
+      const uint32_t mine = (m >> (8u * oct)) & 0xffu;
+      const uint64_t a = __shfl_sync(0xffffffffu, b[u].alpha, mine ? 8u * oct + (uint32_t)(__ffs(mine) - 1) : lane);
+      if (!decided[u] && mine) {
+        code[u] = kGood;
+        idx[u] = a;
+        decided[u] = true;
       }
     }
   }
-  *code = kFail;
-  *idx = 0;
 }
 
-// Sketch::sample by an octet of lanes (round 0, where every vertex samples its own sketch: four
-// vertices per warp).  Lane k of the octet checks depths k, k+8, ...; an octet's answer is the lowest
-// good depth among its lanes.  The octets of a warp may belong to graphs with different bkt, so the
-// pass count is the warp's largest bkt: every lane runs the same passes and reaches every
-// full-warp collective.
-__device__ __forceinline__ void sample_octet(const GsBucket* col, const GsBucket* det, uint32_t bkt, uint64_t csmix,
-                                             bool active, uint32_t* code, uint64_t* idx) {
-  const uint32_t lane = lane_id(), sub = lane & 7u, oct = lane >> 3;
-  bool decided = !active;
-  *code = kFail;
-  *idx = 0;
-  if (active) {
-    const GsBucket d = ld_bucket_cg(det);
-    if (d.alpha == 0 && d.gamma == 0) { *code = kZero; decided = true; }
-    else if (is_good(d, csmix)) { *code = kGood; *idx = d.alpha; decided = true; }
+// A parent entry through L1.  Within a phase a cached entry may be behind, but what it names is still an
+// ancestor; the barrier that ends a phase makes every block's earlier writes visible to these loads.  The
+// entries near a giant component's root are read by nearly every walk, and through L2 alone those reads
+// queue on one slice.
+__device__ __forceinline__ uint32_t ld_parent(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// root of x, writing nothing (each parent entry has one writer in the compress phase)
+__device__ __forceinline__ uint32_t cached_root(const uint32_t* parent, uint32_t x, uint32_t limit, uint32_t* err) {
+  for (uint32_t it = 0; it < limit; it++) {
+    const uint32_t p = ld_parent(parent + x);
+    if (p == x) return x;
+    x = p;
   }
-  const uint32_t bmax = __reduce_max_sync(0xffffffffu, bkt);
-  for (uint32_t j0 = 0; j0 < bmax; j0 += 8) {
-    if (__all_sync(0xffffffffu, decided)) break;
-    const uint32_t j = j0 + sub;
-    GsBucket b = GsBucket{0, 0};
-    const bool look = !decided && j < bkt;
-    if (look) b = ld_bucket_cg(col + j);
-    const uint32_t m = __ballot_sync(0xffffffffu, look && is_good(b, csmix));
-    const uint32_t mine = (m >> (8u * oct)) & 0xffu;
-    const uint64_t a = __shfl_sync(0xffffffffu, b.alpha, mine ? 8u * oct + (uint32_t)(__ffs(mine) - 1) : lane);
-    if (!decided && mine) {
-      *code = kGood;
-      *idx = a;
-      decided = true;
+  atomicOr(err, (uint32_t)GS_DEV_ERR_DSU_LIMIT);
+  return x;
+}
+
+// Union of the components of s and d: the vertex that was hooked (its component's root until then), or ~0
+// when they were one component already.  The parents were compressed when the phase began, so the first
+// entries read are the roots unless another union hooked them since - then the CAS fails and both walks go
+// on, from fresh loads.  A lower root that is out of date does no harm: parents are smaller than their
+// children, so the larger root cannot lie above it.
+__device__ __forceinline__ uint32_t cached_union(uint32_t* parent, uint32_t s, uint32_t d, uint32_t limit, uint32_t* err) {
+  uint32_t a = ld_parent(parent + s), b = ld_parent(parent + d);
+  for (uint32_t it = 0; it < limit; it++) {
+    if (a == b) return 0xffffffffu;
+    if (a < b) { const uint32_t t = a; a = b; b = t; }
+    if (atomicCAS(&parent[a], a, b) == a) return a;
+    for (; it < limit; it++) {
+      const uint32_t pa = ld_volatile(parent + a), pb = ld_volatile(parent + b);
+      if (pa == a && pb == b) break;
+      a = pa;
+      b = pb;
+      if (a == b) return 0xffffffffu;
     }
   }
+  atomicOr(err, (uint32_t)GS_DEV_ERR_DSU_LIMIT);
+  return 0xffffffffu;
 }
 
-// Grid-wide barrier of a co-resident launch.  Returns false when any block gave up waiting.  The
-// waiting thread backs off exponentially (32 ns .. 1 us) so that hundreds of pollers do not saturate
-// the L2 slice that holds the generation word.
-// wait_ns: how long (summed sleep time) a block waits for the others before it reports
-// GS_DEV_ERR_TIMEOUT and gives up
-__device__ bool grid_sync(uint32_t* count, uint32_t* gen, uint32_t* err, uint64_t wait_ns) {
+// 16-byte global -> shared copy that completes asynchronously
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// What the blocks of one graph share in a round; two sets, used in turn, so that one can be reset
+// while the other is still read.
+struct BorCounters {
+  unsigned long long largest;  // (size << 32) | ~root of the largest component
+  unsigned long long alloc;    // (members listed << 32) | tasks
+  uint32_t nbig;
+  uint32_t modified;           // some sample of the round failed or some union succeeded
+};
+
+struct BorArgs {
+  const GsBucket* sk;          // sketch base the tenants' sk_off index into
+  const GsBorTenant* tenants;  // device table, or nullptr: the single graph t0
+  GsBorTenant t0;
+  const uint32_t* qlist;       // cluster scope with a table: the tenant of every cluster
+  uint32_t tenant;             // grid scope with a table: the tenant
+  uint32_t W;                  // accumulator row width, >= bkt_per_col + 1
+  uint32_t R;                  // ring row width: the launch's largest bkt_per_col + 1
+  uint32_t* parent;            // per vertex: DSU parent (vertex ids of the whole vertex space)
+  uint32_t* size;              // per root: members
+  uint32_t* rank;              // per vertex: place among its component's members
+  uint32_t* off;               // per root: first member in list
+  uint32_t* list;              // members grouped by component
+  uint32_t* big;               // roots sampled from their accumulator row
+  uint4* tasks;                // {root, first list position, members, pieces of the root}
+  GsBucket* acc;               // [vertex][W]
+  uint64_t* edge;              // per hooked vertex: the edge that joined its component to another; may be null
+  uint32_t* status;            // [0] error bits [4] forest edges (with `edge`)
+  uint32_t* tstate;            // [tenant][4]: done, -, rounds, out of samples
+  BorCounters* ctr;            // grid scope: [2], zero at launch
+  uint32_t* barrier;           // grid scope: arrivals, zero at launch
+  uint64_t wait_ns;            // grid scope: limit of one barrier wait
+  uint32_t complement;         // the graph's sketches XOR to zero
+};
+
+// Barrier of a co-resident grid: arrivals are counted up and never reset, barrier k is complete at
+// k * gridDim.x.  A wait polls (each poll is a round trip to L2, counted as kPollNs) and gives up
+// after wait_ns or when another block did; the answer is the same for the whole block.
+constexpr uint64_t kPollNs = 250;
+__device__ bool grid_barrier(uint32_t* count, uint32_t target, uint32_t* err, uint64_t wait_ns) {
   __shared__ uint32_t s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t ok = 1;
-    const uint32_t g = ld_volatile(gen);
+    uint32_t ok = 1, n;
     __threadfence();
-    if (atomicAdd(count, 1u) == gridDim.x - 1) {
-      atomicExch(count, 0u);
-      __threadfence();
-      atomicAdd(gen, 1u);
-    } else {
-      uint32_t sleep_ns = 32, it = 0;
-      uint64_t waited = 0;
-      while (ld_volatile(gen) == g) {
-        __nanosleep(sleep_ns);
-        waited += sleep_ns;
-        // back-off capped at 256 ns: a block that waited long notices the release within a
-        // quarter microsecond (1024 ns made the 10-round query 1% slower)
-        if (sleep_ns < 256) sleep_ns <<= 1;
-        if ((++it & 63u) == 0 && (ld_volatile(err) & GS_DEV_ERR_TIMEOUT)) { ok = 0; break; }
-        if (waited > wait_ns) {
-          atomicOr(err, (uint32_t)GS_DEV_ERR_TIMEOUT);
-          ok = 0;
-          break;
-        }
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    uint64_t waited = 0;
+    for (uint32_t it = 0;; it++) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(count) : "memory");
+      if ((int32_t)(n - target) >= 0) break;
+      waited += kPollNs;
+      if (waited > wait_ns) {
+        atomicOr(err, (uint32_t)GS_DEV_ERR_TIMEOUT);
+        ok = 0;
+        break;
       }
+      if ((it & 63u) == 63u && (ld_volatile(err) & GS_DEV_ERR_TIMEOUT)) { ok = 0; break; }
     }
     __threadfence();
     s_ok = ok && !(ld_volatile(err) & GS_DEV_ERR_TIMEOUT);
@@ -191,502 +271,611 @@ __device__ bool grid_sync(uint32_t* count, uint32_t* gen, uint32_t* err, uint64_
   return s_ok != 0;
 }
 
-struct BorArgs {
-  const GsBucket* sk;          // sketch base the tenants' sk_off index into
-  const GsBorTenant* tenants;  // [T] (device), or nullptr: the single tenant t0
-  GsBorTenant t0;
-  const uint32_t* vtenant;     // [V] tenant of each vertex, nullptr when T == 1
-  uint32_t T, V, W;            // W: accumulator row width, max bkt_per_col + 1
-  uint32_t vlo;                // the kernel works on vertices [vlo, V)
-  uint32_t max_rounds;         // max num_samples over the tenants
-  uint32_t* parent;            // [V]
-  uint32_t* size;              // [V]
-  GsBucket* acc;               // [V][W]
-  uint64_t* samp;              // [V] sampled edge of each root this round (global ids), ~0 = none
-  uint32_t* roots;             // [V] this round's roots, status[3] of them
-  uint32_t* forest;            // [2 * forest_cap]
-  uint32_t forest_cap;
-  uint32_t* status;            // [0] error bits [3] roots [4] forest edges [5] active tenants [6,7] barrier
-                               // [12] accumulate work counter
-  uint32_t* tstate;            // [T][4]: done, modified this round, rounds, out of samples
-  uint64_t wait_ns;            // grid-barrier wait limit
-  uint32_t complement;         // every tenant's sketch set XORs to zero: see the accumulate phase
-  unsigned long long* largest; // [T] (size << 32) | ~root of each tenant's largest component this round
-};
-
-// root of tenant t's largest component this round, or ~0 when it has no component of two or more
-__device__ __forceinline__ uint32_t largest_root(const BorArgs& A, uint32_t t) {
-  const unsigned long long k = *reinterpret_cast<const volatile unsigned long long*>(A.largest + t);
-  return (k >> 32) > 1ull ? 0xffffffffu - (uint32_t)k : 0xffffffffu;
+__device__ __forceinline__ uint64_t ld_volatile64(const unsigned long long* p) {
+  return *reinterpret_cast<const volatile unsigned long long*>(p);
 }
 
-__device__ __forceinline__ const GsBorTenant& tenant_of(const BorArgs& A, uint32_t t) {
-  return A.tenants ? A.tenants[t] : A.t0;
+__device__ __forceinline__ void xor_row(GsBucket* row, uint32_t j, uint64_t a, uint64_t g) {
+  atomicXor(reinterpret_cast<unsigned long long*>(&row[j].alpha), (unsigned long long)a);
+  atomicXor(reinterpret_cast<unsigned long long*>(&row[j].gamma), (unsigned long long)g);
 }
 
-__device__ __forceinline__ void flush_acc(const BorArgs& A, uint32_t cur, uint32_t w, const uint64_t* a,
-                                          const uint64_t* gm) {
+// exclusive scan over the block (every thread calls it), and the block's total
+template <uint32_t kWarps>
+__device__ __forceinline__ unsigned long long block_scan(unsigned long long x, unsigned long long* s_sums,
+                                                         unsigned long long* total) {
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  unsigned long long inc = x;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (uint32_t)o) inc += y;
+  }
+  if (lane == 31) s_sums[w] = inc;
+  __syncthreads();
+  unsigned long long all = lane < kWarps ? s_sums[lane] : 0ull, before = lane < w ? all : 0ull;
+  for (int o = 16; o > 0; o >>= 1) {
+    all += __shfl_xor_sync(0xffffffffu, all, o);
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+  }
+  *total = all;
+  return before + inc - x;
+}
+
+// SLOTS: buckets of a row (bkt_per_col + 1) per lane; at most 64 registers in either scope.  Dynamic shared
+// memory: kRing rows of R buckets per warp.
+template <int SCOPE, int SLOTS>
+__global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k_boruvka(const BorArgs A) {
+  constexpr bool CLUSTER = SCOPE != kGrid;
+  constexpr uint32_t kThreads = threads_of(SCOPE), kWarps = kThreads / 32;
+  constexpr uint32_t kTable = 2 * kThreads;        // slots of a block's table of roots
+  extern __shared__ __align__(16) GsBucket s_ring[];
+  __shared__ BorCounters s_ctr[2];                 // cluster scope: the first block's are the cluster's
+  __shared__ uint32_t s_row[4][SLOTS * 32];        // the block's share of the largest component's row
+  __shared__ uint32_t s_key[kTable], s_cnt[kTable];  // roots among a block's vertices, and their members there
+  __shared__ unsigned long long s_sums[kWarps], s_best, s_base;
+  __shared__ uint32_t s_mod, s_hooked;             // a sample failed, unions of the phase
+  const uint32_t lane = lane_id();
+
+  BorCounters* ctr;
+  uint32_t t, block, blocks;
+  if constexpr (CLUSTER) {
+    cg::cluster_group cl = cg::this_cluster();
+    block = cl.block_rank();
+    blocks = cl.num_blocks();
+    ctr = cl.map_shared_rank(s_ctr, 0);
+    t = A.qlist ? A.qlist[blockIdx.x / blocks] : 0u;
+  } else {
+    block = blockIdx.x;
+    blocks = gridDim.x;
+    ctr = A.ctr;
+    t = A.tenant;
+  }
+  const GsBorTenant T = A.tenants ? A.tenants[t] : A.t0;
+  const uint32_t vlo = T.vbase, span = T.V, vend = T.vbase + T.V;
+  const uint32_t bkt = T.bkt, W = A.W, R = A.R;
+  const uint32_t gtid = block * kThreads + threadIdx.x, gthreads = blocks * kThreads;
+  const uint32_t gwarp = gtid >> 5, gwarps = gthreads >> 5;
+  const uint32_t limit = span + 64;
+  uint32_t* const err = A.status;
+  uint32_t* const list = A.list + vlo;
+  uint32_t* const big = A.big + vlo;
+  uint4* const tasks = A.tasks + vlo;
+  const GsBucket* const sk = A.sk + T.sk_off;
+  uint32_t* const ts = A.tstate + 4 * t;
+  uint32_t barriers = 0;
+
+  // Everything the block did becomes visible to the graph's other blocks; false: a wait gave up.
+  // `flag`, when given, is set to one if a sample of the block failed or one of its unions succeeded.
+  auto meet = [&](uint32_t* flag) -> bool {
+    if (flag) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        if (s_mod | s_hooked) *reinterpret_cast<volatile uint32_t*>(flag) = 1u;
+        if (s_hooked && A.edge) atomicAdd(&A.status[4], s_hooked);
+        s_mod = 0;
+        s_hooked = 0;
+      }
+    }
+    if constexpr (CLUSTER) {
+      cg::this_cluster().sync();
+      return true;
+    } else {
+      barriers += blocks;
+      return grid_barrier(A.barrier, barriers, err, A.wait_ns);
+    }
+  };
+  // the edge of a sample, or ~0: anything but a pair of distinct vertices is a checksum collision
+  auto edge_of = [&](uint64_t idx) -> uint64_t {
+    const uint32_t s = (uint32_t)(idx >> 32), d = (uint32_t)idx;
+    return s < span && d < span && s != d ? ((uint64_t)(vlo + s) << 32) | (vlo + d) : ~0ull;
+  };
+  // every lane unions its edge (~0: none), so that up to 32 overlap.  A vertex is hooked once at most: its
+  // edge is kept at its place, and the hooked vertices' edges are the forest.
+  auto unite = [&](uint64_t e) {
+    if (e == ~0ull) return;
+    const uint32_t hooked = cached_union(A.parent, (uint32_t)(e >> 32), (uint32_t)e, limit, err);
+    if (hooked == 0xffffffffu) return;
+    atomicAdd(&s_hooked, 1u);
+    if (A.edge) A.edge[hooked] = e;
+  };
+
+  if (threadIdx.x == 0) { s_mod = 0; s_hooked = 0; s_best = 0; }
+  if (CLUSTER && threadIdx.x < 2 * sizeof(BorCounters) / sizeof(uint32_t))
+    reinterpret_cast<uint32_t*>(s_ctr)[threadIdx.x] = 0;
+  for (uint32_t i = threadIdx.x; i < 4 * SLOTS * 32; i += kThreads) (&s_row[0][0])[i] = 0;
+  for (uint32_t v = vlo + gtid; v < vend; v += gthreads) {
+    A.parent[v] = v;
+    A.size[v] = 0;
+  }
+  if (T.round0_col >= T.ns) {   // OutOfSamplesException before the first round
+    if (gtid == 0) { ts[0] = 1; ts[2] = 0; ts[3] = 1; }
+    return;
+  }
+  if (!meet(nullptr)) return;
+
+  // ---- round 0: every vertex samples its own sketch, an octet of lanes for two; the edges of `per`
+  //      passes are collected one per lane and unioned together ----
+  {
+    const uint32_t per = min(4u, max(1u, (span + 8 * gwarps - 1) / (8 * gwarps)));
+    for (uint32_t base = gwarp * 8 * per; base < span; base += gwarps * 8 * per) {
+      uint64_t mine = ~0ull;
+      bool failed = false;
+      for (uint32_t i = 0; i < per; i++) {
+        const GsBucket *col[2], *det[2];
+        bool active[2];
+        uint32_t code[2];
+        uint64_t idx[2];
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const uint32_t j = lane_id() + 32u * k;
-    if (j < w && (a[k] | gm[k])) {
-      atomicXor(reinterpret_cast<unsigned long long*>(&A.acc[(size_t)cur * A.W + j].alpha), (unsigned long long)a[k]);
-      atomicXor(reinterpret_cast<unsigned long long*>(&A.acc[(size_t)cur * A.W + j].gamma), (unsigned long long)gm[k]);
+        for (int u = 0; u < 2; u++) {
+          const uint32_t k = base + 8 * i + 4 * u + (lane >> 3);
+          active[u] = k < span;
+          const GsBucket* own = sk + (size_t)(k < span ? k : 0u) * T.nb;
+          col[u] = own + (size_t)T.round0_col * bkt;
+          det[u] = own + (T.nb - 1);
+        }
+        sample_octet2(col, det, bkt, T.csmix, active, code, idx);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          failed |= active[u] && code[u] == kFail;
+          const uint64_t e = active[u] && code[u] == kGood ? edge_of(idx[u]) : ~0ull;
+          const uint64_t x = __shfl_sync(0xffffffffu, e, (lane & 3u) * 8u);
+          if ((lane >> 2) == 2 * i + u) mine = x;
+        }
+      }
+      if (failed) s_mod = 1;
+      unite(mine);
     }
   }
-}
 
-// The accumulators a warp still holds at the end of the accumulate phase, flushed once per block:
-// warps of a block that hold the same component's row (every warp holds the largest component's)
-// combine them in shared memory, so one warp per block and component issues the global XORs instead
-// of every warp - the atomics on that row serialize in L2.  Called by every thread of the block.
-__device__ void block_flush(const BorArgs& A, uint32_t root, uint32_t w, const uint64_t* a, const uint64_t* gm,
-                            uint32_t* s_root, GsBucket* stage0) {
-  const uint32_t lane = lane_id(), wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  GsBucket* row = stage0 + (size_t)wib * kAccRun * A.W;
-  if (lane == 0) s_root[wib] = root;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const uint32_t j = lane + 32u * k;
-    if (j < w) row[j] = GsBucket{a[k], gm[k]};
-  }
-  __syncthreads();
-  if (root != 0xffffffffu) {
-    bool leader = true;
-    for (uint32_t o = 0; o < wib; o++) leader = leader && s_root[o] != root;
-    if (leader) {
-      uint64_t x[3] = {a[0], a[1], a[2]}, y[3] = {gm[0], gm[1], gm[2]};
-      for (uint32_t o = wib + 1; o < nw; o++) {
-        if (s_root[o] != root) continue;
-        const GsBucket* other = stage0 + (size_t)o * kAccRun * A.W;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          const uint32_t j = lane + 32u * k;
-          if (j < w) { x[k] ^= other[j].alpha; y[k] ^= other[j].gamma; }
-        }
+  uint32_t rounds = 0, oos = 0;
+  for (uint32_t round = 0;;) {
+    if (!meet(&ctr[round & 1].modified)) return;
+    if (!ld_volatile(&ctr[round & 1].modified)) break;
+    rounds = ++round;
+    oos = rounds >= T.ns;
+    BorCounters* const c = ctr + (round & 1);
+
+    // ---- compress, sizes, ranks, largest.  A block counts the members of every root among 1024 vertices
+    //      in shared memory and adds each count to the root's size once: atomics on the size of a giant
+    //      component's root queue in L2, one per warp took 170 us of a round at V = 10^6 ----
+    unsigned long long best = 0;
+    for (uint32_t base = block * kThreads; base < span; base += gthreads) {
+      for (uint32_t i = threadIdx.x; i < kTable; i += kThreads) {
+        s_key[i] = 0xffffffffu;
+        s_cnt[i] = 0;
       }
-      flush_acc(A, root, w, x, y);
-    }
-  }
-  __syncthreads();
-}
-
-// done flags of the tenants, copied from tstate into shared memory once per round
-__device__ __forceinline__ void snapshot_done(const BorArgs& A, uint32_t* s_done) {
-  for (uint32_t t = threadIdx.x; t < A.T; t += blockDim.x) s_done[t] = ld_volatile(&A.tstate[4 * t]);
-  __syncthreads();
-}
-
-// Dynamic shared memory: the tenants' done flags (T words, padded to 16 bytes), then one staging
-// area of kAccRun x W buckets per warp.
-// three blocks per SM, as shared memory allows: the bound keeps the registers at 78 (122 without it,
-// which left two blocks per SM), with no spills
-__global__ void __launch_bounds__(kThreads, 3) k_boruvka(const BorArgs A) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ uint32_t s_root[kWarps];
-  uint32_t* s_done = smem;
-  GsBucket* stage = reinterpret_cast<GsBucket*>(smem + ((A.T + 3u) & ~3u)) + (threadIdx.x >> 5) * kAccRun * A.W;
-  uint32_t* err = A.status;
-  uint32_t* nroots_p = A.status + 3;
-  uint32_t* acc_next = A.status + 12;  // accumulate work counter, zero at launch and after every round
-  uint32_t* bcount = A.status + 6;
-  uint32_t* bgen = A.status + 7;
-  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
-  const uint32_t gwarp = gtid >> 5, gwarps = gthreads >> 5, lane = lane_id();
-  const uint32_t limit = A.V + 64;
-  const uint32_t span = A.V - A.vlo;
-
-  for (uint32_t v = A.vlo + gtid; v < A.V; v += gthreads) A.parent[v] = v;
-  if (gtid == 0) *nroots_p = 0;
-  if (A.complement)
-    for (uint32_t t = gtid; t < A.T; t += gthreads) A.largest[t] = 0ull;
-  if (!grid_sync(bcount, bgen, err, A.wait_ns)) return;
-
-  for (uint32_t round = 0; round < A.max_rounds; round++) {
-    snapshot_done(A, s_done);
-    if (round > 0) {
-      // ---- sizes of the round's components (size[] was zeroed by the previous compress); the
-      //      first adder of each root appends it to the root list ----
-      for (uint32_t base = A.vlo + blockIdx.x * blockDim.x; base < A.V; base += gthreads) {
-        const uint32_t v = base + threadIdx.x;
-        uint32_t r = 0xffffffffu;
-        if (v < A.V) {
-          const uint32_t t = A.vtenant ? A.vtenant[v] : 0u;
-          if (!s_done[t]) r = __ldcg(&A.parent[v]);
-        }
-        const uint32_t peers = __match_any_sync(0xffffffffu, r);
-        bool fresh = false;
-        if (r != 0xffffffffu && lane == (uint32_t)(__ffs(peers) - 1))
-          fresh = atomicAdd(&A.size[r], (uint32_t)__popc(peers)) == 0u;
-        const uint32_t fm = __ballot_sync(0xffffffffu, fresh);
-        if (fm) {
-          uint32_t at = 0;
-          if (lane == (uint32_t)(__ffs(fm) - 1)) at = atomicAdd(nroots_p, (uint32_t)__popc(fm));
-          at = __shfl_sync(0xffffffffu, at, __ffs(fm) - 1);
-          if (fresh) A.roots[at + __popc(fm & ((1u << lane) - 1u))] = r;
-        }
+      __syncthreads();
+      const uint32_t v = vlo + base + threadIdx.x;
+      uint32_t r = 0xffffffffu;
+      if (v < vend) {
+        r = cached_root(A.parent, v, limit, err);
+        A.parent[v] = r;
       }
-      if (!grid_sync(bcount, bgen, err, A.wait_ns)) return;
-
-      // ---- complement: each tenant's largest component this round (ties to the smallest root) ----
-      if (A.complement) {
-        const uint32_t nr = ld_volatile(nroots_p);
-        if (A.T == 1) {
-          unsigned long long best = 0ull;
-          for (uint32_t k = gtid; k < nr; k += gthreads) {
-            const uint32_t r = __ldcg(&A.roots[k]);
-            const unsigned long long key = ((unsigned long long)__ldcg(&A.size[r]) << 32) | (0xffffffffu - r);
-            best = key > best ? key : best;
-          }
-          for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-            best = other > best ? other : best;
-          }
-          if (lane == 0 && best) atomicMax(A.largest, best);
-        } else {
-          for (uint32_t k = gtid; k < nr; k += gthreads) {
-            const uint32_t r = __ldcg(&A.roots[k]);
-            const uint32_t sz = __ldcg(&A.size[r]);
-            if (sz > 1u) atomicMax(A.largest + A.vtenant[r], ((unsigned long long)sz << 32) | (0xffffffffu - r));
-          }
-        }
-        if (!grid_sync(bcount, bgen, err, A.wait_ns)) return;
-      }
-
-      // ---- accumulate column r + the deterministic bucket per component ----
-      // Warps take runs of kAccGrab vertices from a shared counter (finished tenants' vertices cost
-      // almost nothing, so fixed slices would leave most warps idle at the barrier) and walk each
-      // run kAccRun at a time: the columns of the members are copied into shared memory with
-      // cp.async (all in flight together), then folded in vertex order into a register accumulator
-      // that is flushed with red.global.xor when the component changes.  A vertex whose root is
-      // another vertex is in a component of two or more, so only roots read their own size: no load
-      // hammers a giant component's root.
-      //
-      // Complement (sketch sets that XOR to zero, because every update reached both endpoints): the
-      // XOR of ALL of a graph's vertex sketches is zero, so its largest component's merged column
-      // equals the XOR of the columns of every vertex of the graph outside it.  The largest
-      // component's members are then skipped, and every other vertex - singletons included - is
-      // folded into its graph's largest-component row as well as its own.  A round reads the vertices
-      // outside the largest components instead of all of them.
-      {
-        uint32_t cur = 0xffffffffu, w = 0;
-        uint64_t a[3] = {0, 0, 0}, gm[3] = {0, 0, 0};
-        uint32_t ccur = 0xffffffffu, cw = 0;              // the largest-component row being folded
-        uint64_t ca[3] = {0, 0, 0}, cg[3] = {0, 0, 0};
-        // One graph with the complement: most vertices cost one parent load, so runs are assigned to
-        // warps in a fixed stride (measured 0.39 vs 0.52 ms per V=2^17 query against the counter).
-        // Otherwise warps take runs from the shared counter, because finished tenants' vertices cost
-        // almost nothing and fixed slices would leave warps idle (the 256-tenant query: 2.35 ms per
-        // query with the counter, 2.95 with the stride; reading the counter before the atomic, to keep
-        // warps that find the work gone off it, made it 3.05).
-        const bool strided = A.complement && A.T == 1;
-        uint32_t stride_next = gwarp * kAccRun;
-        const uint32_t grab = strided ? kAccRun : kAccGrab;   // vertices per taken piece of work
+      const uint32_t peers = __match_any_sync(0xffffffffu, r);
+      const uint32_t lead = __ffs(peers) - 1;
+      uint32_t h = 0, local = 0;
+      if (r != 0xffffffffu && lane == lead) {
+        h = __umulhi(r * 0x9E3779B1u, kTable);   // at most kThreads roots: half full
         for (;;) {
-          uint32_t g0 = 0;
-          if (strided) {
-            g0 = stride_next;
-            stride_next += gwarps * kAccRun;
-          } else {
-            if (lane == 0) g0 = atomicAdd(acc_next, grab);
-            g0 = __shfl_sync(0xffffffffu, g0, 0);
-          }
-          if (g0 >= span) break;
-          const uint32_t w1 = A.vlo + min(span, g0 + grab);
-        for (uint32_t start = A.vlo + g0; start < w1; start += kAccRun) {
-          const uint32_t n = min(kAccRun, w1 - start);
-          uint32_t rt = 0xffffffffu, tt = 0, cb = 0xffffffffu;
-          bool outside = false;   // folded into its graph's largest-component row cb (complement)
-          if (lane < n) {
-            const uint32_t v = start + lane;
-            tt = A.vtenant ? A.vtenant[v] : 0u;
-            if (!s_done[tt]) {
-              const uint32_t r = __ldcg(&A.parent[v]);
-              if (A.complement) cb = largest_root(A, tt);
-              if (cb != 0xffffffffu) {
-                outside = r != cb;
-                if (outside && (r != v || __ldcg(&A.size[v]) > 1u)) rt = r;
-              } else if (r != v || __ldcg(&A.size[v]) > 1u) {
-                rt = r;
-              }
-            }
-          }
-          const uint32_t own = __ballot_sync(0xffffffffu, rt != 0xffffffffu);
-          const uint32_t outm = __ballot_sync(0xffffffffu, outside);
-          const uint32_t live = own | outm;
-          for (uint32_t m = live; m;) {
-            const uint32_t i = __ffs(m) - 1;
-            m &= m - 1;
-            const GsBorTenant& T = tenant_of(A, __shfl_sync(0xffffffffu, tt, i));
-            const GsBucket* vb = A.sk + T.sk_off + (size_t)(start + i - T.vbase) * T.nb;
-            for (uint32_t j = lane; j <= T.bkt; j += 32)
-              cp_async16(stage + i * A.W + j, j < T.bkt ? vb + (size_t)round * T.bkt + j : vb + (T.nb - 1));
-          }
-          cp_async_wait_all();
-          __syncwarp();
-          for (uint32_t m = live; m;) {
-            const uint32_t i = __ffs(m) - 1;
-            m &= m - 1;
-            const uint32_t wi = tenant_of(A, __shfl_sync(0xffffffffu, tt, i)).bkt + 1;
-            if ((outm >> i) & 1u) {
-              const uint32_t ci = __shfl_sync(0xffffffffu, cb, i);
-              if (ci != ccur) {
-                if (ccur != 0xffffffffu) flush_acc(A, ccur, cw, ca, cg);
-                ccur = ci;
-                cw = wi;
+          const uint32_t k = atomicCAS(&s_key[h], 0xffffffffu, r);
+          if (k == 0xffffffffu || k == r) break;
+          h = (h + 1) & (kTable - 1);
+        }
+        local = atomicAdd(&s_cnt[h], (uint32_t)__popc(peers));
+      }
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < kTable; i += kThreads) {
+        const uint32_t root = s_key[i];
+        if (root == 0xffffffffu) continue;
+        const uint32_t n = s_cnt[i], old = atomicAdd(&A.size[root], n);
+        s_cnt[i] = old;
+        // the last block to add to a component sees its full size
+        const unsigned long long key = ((unsigned long long)(old + n) << 32) | (0xffffffffu - root);
+        best = key > best ? key : best;
+      }
+      __syncthreads();
+      if (r != 0xffffffffu && lane == lead) local += s_cnt[h];
+      local = __shfl_sync(0xffffffffu, local, lead);
+      if (r != 0xffffffffu) A.rank[v] = local + __popc(peers & ((1u << lane) - 1u));
+      __syncthreads();
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+      best = other > best ? other : best;
+    }
+    if (lane == 0 && best) atomicMax(&s_best, best);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (s_best) atomicMax(&c->largest, s_best);
+      s_best = 0;
+    }
+    if (!meet(nullptr)) return;
+    if (oos) break;   // the labels are compressed
+    const uint64_t top = ld_volatile64(&c->largest);
+    // the component whose column is the XOR of everything outside it, or ~0: none
+    const uint32_t comp = A.complement && (top >> 32) > 1ull ? 0xffffffffu - (uint32_t)top : 0xffffffffu;
+
+    // ---- allocate: member runs and tasks, one reservation per block; runs and tasks come in one order ----
+    {
+      const uint32_t share = (span + blocks - 1) / blocks;
+      const uint32_t v0 = vlo + min(span, block * share), v1 = vlo + min(span, block * share + share);
+      // only roots have a size; the first vertex's stays in its register for the second pass
+      const uint32_t first = v0 + threadIdx.x < v1 ? __ldcg(&A.size[v0 + threadIdx.x]) : 0u;
+      unsigned long long mine = 0, total;
+      for (uint32_t v = v0 + threadIdx.x; v < v1; v += kThreads) {
+        const uint32_t n = v == comp ? 0u : v == v0 + threadIdx.x ? first : __ldcg(&A.size[v]);
+        mine += ((unsigned long long)n << 32) | ((n + kPiece - 1) / kPiece);
+      }
+      unsigned long long at = block_scan<kWarps>(mine, s_sums, &total);
+      if (threadIdx.x == 0) s_base = total ? atomicAdd(&c->alloc, total) : 0ull;
+      __syncthreads();
+      at += s_base;
+      for (uint32_t vb = v0 + (threadIdx.x & ~31u); vb < v1; vb += kThreads) {
+        const uint32_t v = vb + lane;
+        const uint32_t size = v >= v1 ? 0u : v == v0 + threadIdx.x ? first : __ldcg(&A.size[v]);
+        const uint32_t n = v == comp ? 0u : size, pieces = (n + kPiece - 1) / kPiece;
+        const uint32_t start = (uint32_t)(at >> 32), task = (uint32_t)at;
+        if (n) A.off[v] = start;
+        if (pieces == 1) tasks[task] = make_uint4(v, start, n, 1u);
+        at += ((unsigned long long)n << 32) | pieces;
+        for (uint32_t m = __ballot_sync(0xffffffffu, pieces > 1); m; m &= m - 1) {
+          const uint32_t src = __ffs(m) - 1;   // a larger component's tasks are written by the warp
+          const uint32_t hn = __shfl_sync(0xffffffffu, n, src), hp = __shfl_sync(0xffffffffu, pieces, src);
+          const uint32_t h0 = __shfl_sync(0xffffffffu, start, src), ht = __shfl_sync(0xffffffffu, task, src);
+          for (uint32_t p = lane; p < hp; p += 32)
+            tasks[ht + p] = make_uint4(vb + src, h0 + p * kPiece, min(kPiece, hn - p * kPiece), hp);
+        }
+        const bool is_big = size && (v == comp || pieces > 1);
+        const uint32_t bm = __ballot_sync(0xffffffffu, is_big);
+        if (bm) {
+          uint32_t b = 0;
+          if (lane == 0) b = atomicAdd(&c->nbig, (uint32_t)__popc(bm));
+          b = __shfl_sync(0xffffffffu, b, 0);
+          if (is_big) big[b + __popc(bm & ((1u << lane) - 1u))] = v;
+        }
+      }
+    }
+    if (!meet(nullptr)) return;
+
+    // ---- place the members; clear the sizes and the other counter set for the next round ----
+    for (uint32_t v = vlo + gtid; v < vend; v += gthreads) {
+      const uint32_t r = __ldcg(&A.parent[v]);
+      if (r != comp) list[__ldcg(&A.off[r]) + __ldcg(&A.rank[v])] = v;
+      if (r == v) A.size[v] = 0;
+    }
+    if (gtid < sizeof(BorCounters) / sizeof(uint32_t))
+      reinterpret_cast<volatile uint32_t*>(ctr + ((round + 1) & 1))[gtid] = 0;
+    if (!meet(nullptr)) return;
+
+    // ---- gather: each warp a run of tasks, whose members are one run of the list.  The members' rows
+    //      stream through a ring in shared memory, kRing of them on their way at once ----
+    {
+      const uint32_t ntasks = (uint32_t)ld_volatile64(&c->alloc);
+      const uint32_t per = (ntasks + gwarps - 1) / gwarps;
+      const uint32_t t0 = min(ntasks, gwarp * per), t1 = min(ntasks, t0 + per);
+      GsBucket* const ring = s_ring + (size_t)(threadIdx.x >> 5) * kRing * R;
+      uint64_t ca[SLOTS] = {}, cb[SLOTS] = {};      // the run's share of the largest component's row
+      uint64_t ma[SLOTS] = {}, mb[SLOTS] = {};      // pieces of one larger component
+      uint32_t mroot = 0xffffffffu, held = 0;
+      uint64_t mine = ~0ull;
+      auto flush_pieces = [&]() {
+        if (mroot == 0xffffffffu) return;
 #pragma unroll
-                for (int k = 0; k < 3; k++) ca[k] = cg[k] = 0;
-              }
+        for (int k = 0; k < SLOTS; k++) {
+          const uint32_t j = lane + 32u * k;
+          if (j <= bkt && (ma[k] | mb[k])) xor_row(A.acc + (size_t)mroot * W, j, ma[k], mb[k]);
+          ma[k] = mb[k] = 0;
+        }
+        mroot = 0xffffffffu;
+      };
+      if (t0 < t1) {
+        const uint4 last = __ldcg(&tasks[t1 - 1]);
+        const uint32_t m0 = __ldcg(&tasks[t0].y), total = last.y + last.z - m0;
+        // lane l holds list entries l of the current and the next 32
+        uint32_t now = lane < total ? __ldcg(&list[m0 + lane]) : 0u;
+        uint32_t then = 32 + lane < total ? __ldcg(&list[m0 + 32 + lane]) : 0u;
+        uint32_t next = 0;   // the member whose row is asked for next
+        auto ask = [&]() {   // kGroup rows, one commit
 #pragma unroll
-              for (int k = 0; k < 3; k++) {
-                const uint32_t j = lane + 32u * k;
-                if (j < wi) {
-                  const GsBucket b = stage[i * A.W + j];
-                  ca[k] ^= b.alpha;
-                  cg[k] ^= b.gamma;
-                }
-              }
-            }
-            if (!((own >> i) & 1u)) continue;
-            const uint32_t root = __shfl_sync(0xffffffffu, rt, i);
-            if (root != cur) {
-              if (cur != 0xffffffffu) flush_acc(A, cur, w, a, gm);
-              cur = root;
-              w = wi;
+          for (uint32_t u = 0; u < kGroup; u++) {
+            const uint32_t v = __shfl_sync(0xffffffffu, now, (next + u) & 31u) - vlo;
+            if (next + u >= total) continue;
+            const GsBucket* vb = sk + (size_t)v * T.nb;
+            GsBucket* to = ring + ((next + u) % kRing) * R;
 #pragma unroll
-              for (int k = 0; k < 3; k++) a[k] = gm[k] = 0;
-            }
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
+            for (int k = 0; k < SLOTS; k++) {
               const uint32_t j = lane + 32u * k;
-              if (j < w) {
-                const GsBucket b = stage[i * A.W + j];
-                a[k] ^= b.alpha;
-                gm[k] ^= b.gamma;
-              }
+              if (j <= bkt) cp_async16(to + j, vb + (j < bkt ? round * bkt + j : T.nb - 1));
             }
           }
-          __syncwarp();
-        }
-        }
-        // the warps' last rows: combined per block (the largest component's row, or with the direct
-        // accumulation the giant component's, is held by nearly every warp)
-        block_flush(A, cur, w, a, gm, s_root, stage - (threadIdx.x >> 5) * kAccRun * A.W);
-        block_flush(A, ccur, cw, ca, cg, s_root, stage - (threadIdx.x >> 5) * kAccRun * A.W);
-      }
-      if (!grid_sync(bcount, bgen, err, A.wait_ns)) return;
-    }
-
-    // ---- sample every root into samp[root]: roots spread over the warps by list position ----
-    // The accumulator row of a sampled component is zeroed after reading, so every row is zero
-    // again when the round ends (and at the start of the next launch).
-    const uint32_t nroots = round == 0 ? span : ld_volatile(nroots_p);
-    if (round == 0 && A.T > 1) {
-      // every vertex samples its own sketch: one thread each (many sparse graphs)
-      for (uint32_t v = A.vlo + gtid; v < A.V; v += gthreads) {
-        const uint32_t t = A.vtenant ? A.vtenant[v] : 0u;
-        if (s_done[t]) continue;
-        const GsBorTenant& T = tenant_of(A, t);
-        const uint32_t col = T.round0_col;
-        if (col >= T.ns) {  // OutOfSamplesException
-          A.tstate[4 * t + 3] = 1u;
-          continue;
-        }
-        const GsBucket* own = A.sk + T.sk_off + (size_t)(v - T.vbase) * T.nb;
-        uint32_t code;
-        uint64_t idx;
-        sample_thread(own + (size_t)col * T.bkt, own + (T.nb - 1), T.bkt, T.csmix, &code, &idx);
-        uint64_t e = ~0ull;
-        if (code == kFail) {
-          A.tstate[4 * t + 1] = 1u;
-        } else if (code == kGood) {
-          const uint32_t s = (uint32_t)(idx >> 32), d = (uint32_t)idx;
-          if (s < T.V && d < T.V && s != d) e = ((uint64_t)(T.vbase + s) << 32) | (T.vbase + d);
-        }
-        A.samp[v] = e;
-      }
-    } else if (round == 0) {
-      // every vertex samples its own sketch: an octet of lanes each, four vertices per warp (one
-      // graph, whose high-degree vertices find their first good bucket deep in the column)
-      for (uint32_t base = A.vlo + gwarp * 4u; base < A.V; base += gwarps * 4u) {
-        const uint32_t v = base + (lane >> 3);
-        bool active = v < A.V;
-        uint32_t t = 0;
-        if (active) {
-          t = A.vtenant ? A.vtenant[v] : 0u;
-          active = !s_done[t];
-        }
-        const GsBorTenant& T = tenant_of(A, active ? t : 0u);
-        const uint32_t col = T.round0_col;
-        const bool oos = active && col >= T.ns;  // OutOfSamplesException
-        if (oos && (lane & 7u) == 0) A.tstate[4 * t + 3] = 1u;
-        const GsBucket* own = A.sk + T.sk_off + (size_t)((active ? v : T.vbase) - T.vbase) * T.nb;
-        uint32_t code;
-        uint64_t idx;
-        sample_octet(own + (size_t)(oos ? 0u : col) * T.bkt, own + (T.nb - 1), T.bkt, T.csmix, active && !oos, &code,
-                     &idx);
-        if (active && !oos && (lane & 7u) == 0) {
-          uint64_t e = ~0ull;
-          if (code == kFail) {
-            A.tstate[4 * t + 1] = 1u;
-          } else if (code == kGood) {
-            const uint32_t s = (uint32_t)(idx >> 32), d = (uint32_t)idx;
-            if (s < T.V && d < T.V && s != d) e = ((uint64_t)(T.vbase + s) << 32) | (T.vbase + d);
+          cp_async_commit();
+          next += kGroup;
+          if ((next & 31u) == 0) {
+            now = then;
+            then = next + 32 + lane < total ? __ldcg(&list[m0 + next + 32 + lane]) : 0u;
           }
-          A.samp[v] = e;
-        }
-      }
-    }
-    for (uint32_t k = gwarp; round > 0 && k < nroots; k += gwarps) {
-      const uint32_t v = round == 0 ? A.vlo + k : __ldcg(&A.roots[k]);
-      const uint32_t t = A.vtenant ? A.vtenant[v] : 0u;
-      if (s_done[t]) continue;
-      const uint32_t sz = round == 0 ? 1u : __ldcg(&A.size[v]);
-      const GsBorTenant& T = tenant_of(A, t);
-      const uint32_t col = round == 0 ? T.round0_col : round;
-      GsBucket* acc = A.acc + (size_t)v * A.W;
-      if (col >= T.ns) {  // OutOfSamplesException
-        if (lane == 0) A.tstate[4 * t + 3] = 1u;
-      } else {
-        const GsBucket* own = A.sk + T.sk_off + (size_t)(v - T.vbase) * T.nb;
-        uint32_t code;
-        uint64_t idx;
-        if (sz > 1) sample_warp(acc, acc + T.bkt, T.bkt, T.csmix, &code, &idx);
-        else sample_warp(own + (size_t)col * T.bkt, own + (T.nb - 1), T.bkt, T.csmix, &code, &idx);
-        if (lane == 0) {
-          uint64_t e = ~0ull;
-          if (code == kFail) {
-            A.tstate[4 * t + 1] = 1u;
-          } else if (code == kGood) {
-            const uint32_t s = (uint32_t)(idx >> 32), d = (uint32_t)idx;
-            if (s < T.V && d < T.V && s != d)  // anything else is a checksum collision
-              e = ((uint64_t)(T.vbase + s) << 32) | (T.vbase + d);
+        };
+        ask();
+        ask();
+        uint32_t done = 0;
+        uint4 batch = make_uint4(0, 0, 0, 0);
+        for (uint32_t tk = t0; tk < t1; tk++) {
+          if (((tk - t0) & 31u) == 0 && tk + lane < t1) batch = __ldcg(&tasks[tk + lane]);
+          const uint32_t root = __shfl_sync(0xffffffffu, batch.x, (tk - t0) & 31u);
+          const uint32_t n = __shfl_sync(0xffffffffu, batch.z, (tk - t0) & 31u);
+          const uint32_t pieces = __shfl_sync(0xffffffffu, batch.w, (tk - t0) & 31u);
+          uint64_t a[SLOTS] = {}, g[SLOTS] = {};
+#pragma unroll 1
+          for (uint32_t i = 0; i < n; i++) {
+            if (done % kGroup == 0) {        // the group before the last one asked for has landed
+              cp_async_wait<1>();
+              __syncwarp();
+            }
+            const GsBucket* row = ring + (done % kRing) * R;
+#pragma unroll
+            for (int k = 0; k < SLOTS; k++) {
+              const uint32_t j = lane + 32u * k;
+              if (j <= bkt) {
+                const GsBucket b = row[j];
+                a[k] ^= b.alpha;
+                g[k] ^= b.gamma;
+              }
+            }
+            if (++done % kGroup == 0) {      // its rows are read: the next group takes their place
+              __syncwarp();
+              ask();
+            }
           }
-          A.samp[v] = e;
+          if (comp != 0xffffffffu) {
+#pragma unroll
+            for (int k = 0; k < SLOTS; k++) { ca[k] ^= a[k]; cb[k] ^= g[k]; }
+          }
+          if (pieces > 1) {
+            if (root != mroot) {
+              flush_pieces();
+              mroot = root;
+            }
+#pragma unroll
+            for (int k = 0; k < SLOTS; k++) { ma[k] ^= a[k]; mb[k] ^= g[k]; }
+            continue;
+          }
+          // the whole component: sample it from the registers
+          uint64_t da = 0, dg = 0;
+          uint32_t good[SLOTS], det_good = 0;
+#pragma unroll
+          for (int k = 0; k < SLOTS; k++) {
+            const uint32_t j = lane + 32u * k;
+            if (bkt / 32u == (uint32_t)k) {
+              da = __shfl_sync(0xffffffffu, a[k], bkt & 31u);
+              dg = __shfl_sync(0xffffffffu, g[k], bkt & 31u);
+            }
+            good[k] = __ballot_sync(0xffffffffu, j <= bkt && is_good(GsBucket{a[k], g[k]}, T.csmix));
+            if (bkt / 32u == (uint32_t)k) det_good = (good[k] >> (bkt & 31u)) & 1u;
+          }
+          uint64_t e = ~0ull;
+          if ((da | dg) != 0ull) {
+            uint32_t at = 0xffffffffu;   // the first good depth, but the deterministic bucket before any
+#pragma unroll
+            for (int k = SLOTS - 1; k >= 0; k--)
+              if (good[k]) at = 32u * k + (__ffs(good[k]) - 1);
+            if (det_good) at = bkt;
+            if (at == 0xffffffffu) {
+              s_mod = 1;                 // FAIL
+            } else {
+              uint64_t idx = 0;
+#pragma unroll
+              for (int k = 0; k < SLOTS; k++)
+                if (at / 32u == (uint32_t)k) idx = __shfl_sync(0xffffffffu, a[k], at & 31u);
+              e = edge_of(idx);
+            }
+          }
+          if (lane == held) mine = e;
+          if (++held == 32) {
+            unite(mine);
+            __syncwarp();
+            mine = ~0ull;
+            held = 0;
+          }
+        }
+        if (held) unite(mine);
+        flush_pieces();
+      }
+      if (comp != 0xffffffffu) {
+        // one warp's row at a time would queue on the row's L2 lines: combined per block first
+        if (t0 < t1) {
+#pragma unroll
+          for (int k = 0; k < SLOTS; k++) {
+            const uint32_t j = lane + 32u * k;
+            if (j <= bkt && (ca[k] | cb[k])) {
+              atomicXor(&s_row[0][j], (uint32_t)ca[k]);
+              atomicXor(&s_row[1][j], (uint32_t)(ca[k] >> 32));
+              atomicXor(&s_row[2][j], (uint32_t)cb[k]);
+              atomicXor(&s_row[3][j], (uint32_t)(cb[k] >> 32));
+            }
+          }
+        }
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j <= bkt; j += kThreads) {
+          const uint64_t a = ((uint64_t)s_row[1][j] << 32) | s_row[0][j];
+          const uint64_t g = ((uint64_t)s_row[3][j] << 32) | s_row[2][j];
+          if (a | g) xor_row(A.acc + (size_t)comp * W, j, a, g);
+          s_row[0][j] = s_row[1][j] = s_row[2][j] = s_row[3][j] = 0;
         }
       }
-      if (sz > 1) {
-        __syncwarp();
-        for (uint32_t j = lane; j <= T.bkt; j += 32) acc[j] = GsBucket{0, 0};
-      }
     }
-    if (!grid_sync(bcount, bgen, err, A.wait_ns)) return;
+    if (!meet(nullptr)) return;
 
-    // ---- union the sampled edges: one thread per root, so many DSU walks are in flight ----
-    for (uint32_t k = gtid; k < nroots; k += gthreads) {
-      const uint32_t v = round == 0 ? A.vlo + k : __ldcg(&A.roots[k]);
-      const uint32_t t = A.vtenant ? A.vtenant[v] : 0u;
-      if (s_done[t]) continue;
-      const GsBorTenant& T = tenant_of(A, t);
-      if ((round == 0 ? T.round0_col : round) >= T.ns) continue;
-      const uint64_t e = __ldcg(&A.samp[v]);
-      if (e == ~0ull) continue;
-      const uint32_t gs = (uint32_t)(e >> 32), gd = (uint32_t)e;
-      if (dsu_union(A.parent, gs, gd, limit, err)) {
-        // read before writing: with one graph every successful union (2^17 in round 0 at V=2^17)
-        // would store to the same flag, and those stores queue on one L2 line
-        if (!ld_volatile(&A.tstate[4 * t + 1])) A.tstate[4 * t + 1] = 1u;
-        const uint32_t f = atomicAdd(&A.status[4], 1u);
-        if (f < A.forest_cap) {
-          A.forest[2 * f] = min(gs, gd);
-          A.forest[2 * f + 1] = max(gs, gd);
-        }
-      }
+    // ---- the largest component and those of several pieces: sampled from their rows ----
+    const uint32_t nbig = ld_volatile(&c->nbig);
+    for (uint32_t k = gwarp; k < nbig; k += gwarps) {
+      const uint32_t r = __ldcg(&big[k]);
+      GsBucket* row = A.acc + (size_t)r * W;
+      uint32_t code;
+      uint64_t idx;
+      sample_warp(row, row + bkt, bkt, T.csmix, &code, &idx);
+      if (code == kFail) s_mod = 1;
+      __syncwarp();
+      for (uint32_t j = lane; j <= bkt; j += 32) row[j] = GsBucket{0, 0};
+      unite(lane == 0 && code == kGood ? edge_of(idx) : ~0ull);
     }
-    if (!grid_sync(bcount, bgen, err, A.wait_ns)) return;
-
-    // ---- compress, clear the sizes and the root list for the next round, and per tenant stop
-    //      at the first unmodified round (the modified flags were final at the last barrier) ----
-    for (uint32_t v = A.vlo + gtid; v < A.V; v += gthreads) {
-      A.parent[v] = dsu_root(A.parent, v, limit, err);
-      A.size[v] = 0;
-    }
-    if (gtid == 0) {
-      *nroots_p = 0;
-      *acc_next = 0;
-    }
-    if (A.complement)
-      for (uint32_t t = gtid; t < A.T; t += gthreads) A.largest[t] = 0ull;
-    for (uint32_t t = gtid; t < A.T; t += gthreads) {
-      volatile uint32_t* ts = A.tstate + 4 * t;
-      if (ts[0]) continue;
-      if (ts[3]) {                     // ran out of samples
-        ts[0] = 1u;
-        atomicSub(&A.status[5], 1u);
-      } else if (ts[1]) {              // modified: the next round runs
-        ts[1] = 0u;
-        ts[2] = round + 1;
-        if (round + 1 >= tenant_of(A, t).ns) {
-          ts[3] = 1u;
-          ts[0] = 1u;
-          atomicSub(&A.status[5], 1u);
-        }
-      } else {
-        ts[0] = 1u;
-        atomicSub(&A.status[5], 1u);
-      }
-    }
-    if (!grid_sync(bcount, bgen, err, A.wait_ns)) return;
-    if (ld_volatile(&A.status[5]) == 0) return;
   }
+
+  if (gtid == 0) { ts[0] = 1; ts[2] = rounds; ts[3] = oos; }
+  // the first block's counters stay until every block has read them
+  if constexpr (CLUSTER) cg::this_cluster().sync();
+}
+
+// the edges of the hooked vertices, as (min, max) pairs in any order
+__global__ void __launch_bounds__(256) k_forest(const uint32_t* __restrict__ parent, const uint64_t* __restrict__ edge,
+                                                uint32_t V, uint32_t* __restrict__ count, uint2* __restrict__ forest) {
+  __shared__ uint32_t s_warp[8], s_at;
+  const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+  for (uint32_t base = blockIdx.x * 256; base < V; base += gridDim.x * 256) {
+    const uint32_t v = base + threadIdx.x;
+    const bool hooked = v < V && parent[v] != v;
+    const uint32_t m = __ballot_sync(0xffffffffu, hooked);
+    if (lane == 0) s_warp[w] = __popc(m);
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (uint32_t i = 0; i < 8; i++) {
+      if (i < w) before += s_warp[i];
+      all += s_warp[i];
+    }
+    if (threadIdx.x == 0) s_at = all ? atomicAdd(count, all) : 0u;
+    __syncthreads();
+    if (hooked) {
+      const uint64_t e = edge[v];
+      const uint32_t a = (uint32_t)(e >> 32), b = (uint32_t)e;
+      forest[s_at + before + __popc(m & ((1u << lane) - 1u))] = make_uint2(min(a, b), max(a, b));
+    }
+    __syncthreads();
+  }
+}
+
+size_t ring_bytes(int scope, uint32_t R) {
+  return (size_t)(threads_of(scope) / 32) * kRing * R * sizeof(GsBucket);
+}
+
+// Launches of more than 48 KB of dynamic shared memory, and clusters of more than 8 blocks, are opted into
+// per device and kernel; what was opted into is remembered per host thread.
+template <int SCOPE, int SLOTS>
+gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s) {
+  struct Opted { uint32_t R = 0, blocks = 0; int sms = 0; };
+  static thread_local Opted opted[64];
+  int dev = 0;
+  GS_CUDA_TRY(cudaGetDevice(&dev));
+  Opted& o = opted[dev & 63];
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.blockDim = dim3(threads_of(SCOPE));
+  cfg.dynamicSmemBytes = ring_bytes(SCOPE, L.R);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (o.R < L.R) {
+    GS_CUDA_TRY(cudaFuncSetAttribute(k_boruvka<SCOPE, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)cfg.dynamicSmemBytes));
+    GS_CUDA_TRY(cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev));
+    o.blocks = 8;
+    if (SCOPE != kGrid) {
+      // 16 blocks where the device can place them
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 16;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(16);
+      int n = 0;
+      if (cudaFuncSetAttribute(k_boruvka<SCOPE, SLOTS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&n, k_boruvka<SCOPE, SLOTS>, &cfg) == cudaSuccess && n > 0)
+        o.blocks = 16;
+      cudaGetLastError();
+    }
+    o.R = L.R;
+  }
+  if (SCOPE != kGrid) {
+    const uint32_t blocks = std::min(L.scope.blocks, o.blocks);
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(blocks * L.count);
+  } else {
+    // every block co-resident: cooperative through a launch attribute, so that the launch can also be
+    // captured into a CUDA graph
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.gridDim = dim3(o.sms);
+    GS_CUDA_TRY(cudaMemsetAsync(A.ctr, 0, kGsBorCounterWords * sizeof(uint32_t), s));
+  }
+  GS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_boruvka<SCOPE, SLOTS>, A));
+  return GS_OK;
+}
+
+template <int SLOTS>
+gs_status launch_scope(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s) {
+  if (!L.scope.blocks) return launch_boruvka<kGrid, SLOTS>(A, L, s);
+  return L.scope.wide ? launch_boruvka<kWide, SLOTS>(A, L, s) : launch_boruvka<kNarrow, SLOTS>(A, L, s);
 }
 
 }  // namespace
 
+static_assert((kGsBorCounterWords - 1) * sizeof(uint32_t) >= 2 * sizeof(BorCounters), "two counter sets and the barrier");
+
 gs_status gs_boruvka_launch(const GsBorLaunch& L, cudaStream_t s) {
   BorArgs A;
   A.sk = L.sk;
-  A.tenants = L.T > 1 ? L.tenants : nullptr;
+  A.tenants = L.tenants;
   A.t0 = L.t0;
-  A.vtenant = L.T > 1 ? L.vtenant : nullptr;
-  A.T = L.T;
-  A.V = L.V;
+  A.qlist = L.qlist;
+  A.tenant = L.tenant;
   A.W = L.W;
-  A.vlo = L.vlo;
-  A.max_rounds = L.max_rounds;
+  A.R = L.R;
   A.parent = L.parent;
   A.size = L.size;
+  const size_t n = L.vertices;
+  A.rank = L.members;
+  A.off = L.members + n;
+  A.list = L.members + 2 * n;
+  A.big = L.members + 3 * n;
+  A.tasks = L.tasks;
   A.acc = L.acc;
-  A.samp = L.samp;
-  A.roots = L.roots;
-  A.forest = L.forest;
-  A.forest_cap = L.forest_cap;
+  A.edge = L.edge;
   A.status = L.status;
   A.tstate = L.tstate;
+  A.ctr = reinterpret_cast<BorCounters*>(L.counters);
+  A.barrier = L.counters + kGsBorCounterWords - 1;
   A.wait_ns = L.wait_ns;
-  A.complement = (L.complement && L.largest) ? 1u : 0u;
-  A.largest = A.complement ? L.largest : nullptr;
-  int dev = 0;
-  GS_CUDA_TRY(cudaGetDevice(&dev));
-  const size_t smem = (size_t)((L.T + 3u) & ~3u) * sizeof(uint32_t) + (size_t)kWarps * kAccRun * L.W * sizeof(GsBucket);
-  // occupancy depends on the shared-memory size: cache it per (device, size)
-  struct Occ { size_t smem = 0; int blocks = 0; };
-  static thread_local Occ occ[64];  // per host thread: handles may be used from several threads at once
-  Occ& o = occ[dev < 64 ? dev : 63];
-  if (o.smem != smem) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(k_boruvka, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0, sms = 0;
-    GS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_boruvka, kThreads, smem));
-    GS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (per_sm < 1) {
-      gs_set_error("Boruvka kernel does not fit on an SM with " + std::to_string(smem) + " bytes of shared memory");
-      return GS_ERR_BAD_ARG;
-    }
-    o.smem = smem;
-    o.blocks = per_sm * sms;  // every block co-resident: the cooperative-launch limit
+  A.complement = L.complement;
+  if (L.R <= 32) return launch_scope<1>(A, L, s);
+  if (L.R <= 64) return launch_scope<2>(A, L, s);
+  gs_set_error("more than 63 buckets per column are not supported");
+  return GS_ERR_BAD_ARG;
+}
+
+gs_status gs_alloc_boruvka(gs_graph* g, uint64_t vertices, uint32_t width, bool forest) {
+  // one allocation, cut up by falling alignment
+  const uint64_t row = sizeof(uint4) + (forest ? 2 * sizeof(uint64_t) : 0) + 6 * sizeof(uint32_t);
+  GS_CUDA_TRY(cudaMalloc(&g->d_bor, vertices * row + kGsBorCounterWords * sizeof(uint32_t)));
+  uint8_t* p = static_cast<uint8_t*>(g->d_bor);
+  const auto take = [&](uint64_t bytes) { uint8_t* at = p; p += bytes; return at; };
+  g->d_tasks = reinterpret_cast<uint4*>(take(vertices * sizeof(uint4)));
+  g->d_bor_ctr = reinterpret_cast<uint32_t*>(take(kGsBorCounterWords * sizeof(uint32_t)));
+  if (forest) {
+    g->d_edge = reinterpret_cast<uint64_t*>(take(vertices * sizeof(uint64_t)));
+    g->d_forest = reinterpret_cast<uint32_t*>(take(vertices * 2 * sizeof(uint32_t)));
   }
-  // cooperative through a launch attribute, so the launch can also be captured into a CUDA graph
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(o.blocks);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  GS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_boruvka, A));
+  g->d_parent = reinterpret_cast<uint32_t*>(take(vertices * sizeof(uint32_t)));
+  g->d_size = reinterpret_cast<uint32_t*>(take(vertices * sizeof(uint32_t)));
+  g->d_members = reinterpret_cast<uint32_t*>(take(4 * vertices * sizeof(uint32_t)));
+  GS_CUDA_TRY(cudaMalloc(&g->d_acc, vertices * width * sizeof(GsBucket)));
+  return GS_OK;
+}
+
+gs_status gs_gather_forest(gs_graph* g, cudaStream_t s) {
+  if (!g->last_forest_edges) return GS_OK;
+  GS_CUDA_TRY(cudaMemsetAsync(g->d_bor_ctr, 0, sizeof(uint32_t), s));
+  const int grid = std::min<int>((int)((g->V + 255) / 256), g->num_sms * 8);
+  GsProfScope ps(g, GS_PROF_QUERY, s, 1);
+  k_forest<<<grid, 256, 0, s>>>(g->d_parent, g->d_edge, g->V, g->d_bor_ctr, reinterpret_cast<uint2*>(g->d_forest));
+  GS_CUDA_TRY(cudaGetLastError());
   return GS_OK;
 }
 
@@ -705,32 +894,28 @@ gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, c
   L.t0.ns = g->geom.num_samples;
   L.t0.round0_col = round0_col;
   L.t0.csmix = gs_seed_mix(g->seed);
-  L.T = 1;
-  L.V = V;
-  L.W = bkt + 1;
-  L.max_rounds = g->geom.num_samples;
+  // a handle with a wait limit of its own keeps the scope whose waits have one
+  if (g->wait_ns == kGsDefaultWaitNs) L.scope = gs_boruvka_scope(V, 1);
+  L.vertices = V;
+  L.W = L.R = bkt + 1;
   L.parent = g->d_parent;
   L.size = g->d_size;
   L.acc = g->d_acc;
-  L.samp = g->d_samp;
-  L.roots = g->d_res;
-  L.forest = g->d_forest;
-  L.forest_cap = V;
+  L.members = g->d_members;
+  L.tasks = g->d_tasks;
+  L.edge = g->d_edge;
   L.status = g->d_status;
   L.tstate = g->d_status + 8;
+  L.counters = g->d_bor_ctr;
   L.wait_ns = g->wait_ns;
   L.complement = g->sketches_symmetric ? 1u : 0u;
-  L.largest = reinterpret_cast<unsigned long long*>(g->d_status + 18);   // status words 18-19
 
   // the kernel expects all-zero accumulator rows and leaves them so when it runs to the end
   if (g->acc_dirty) GS_CUDA_TRY(cudaMemsetAsync(g->d_acc, 0, (size_t)V * (bkt + 1) * sizeof(GsBucket), s));
   g->acc_dirty = true;
-  // the ingest error bits not yet reported move to word 16 (read back with the query's words);
-  // status: everything else zero except the count of tenants still running
+  // the ingest error bits not yet reported move to word 16 (read back with the query's words)
   GS_CUDA_TRY(cudaMemcpyAsync(g->d_status + 16, g->d_status, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-  g->h_status[15] = 1;
   GS_CUDA_TRY(cudaMemsetAsync(g->d_status, 0, 16 * sizeof(uint32_t), s));
-  GS_CUDA_TRY(cudaMemcpyAsync(g->d_status + 5, g->h_status + 15, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   {
     GsProfScope ps(g, GS_PROF_QUERY, s, 1);
     GS_TRY(gs_boruvka_launch(L, s));
@@ -740,6 +925,21 @@ gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, c
   // calls queued after the query (a stale bit would fail the next synchronizing call)
   GS_CUDA_TRY(cudaMemsetAsync(g->d_status, 0, sizeof(uint32_t), s));
   return GS_OK;
+}
+
+// One graph: a cluster has 16 SMs and the hardware's barrier, the grid all of them and a barrier of about
+// 1.5 us; the two meet near 8192 vertices (us per query, cluster / grid: V = 1024 84 / 134, 4096 190 / 271,
+// 8192 225 / 234, 16384 295 / 195).  Several graphs: clusters side by side, smaller ones the more graphs
+// there are (256 graphs of up to 16384 vertices: 1.57 ms with 2 blocks each, 1.08 with 4, 1.54 with 8).
+GsBorScope gs_boruvka_scope(uint32_t V, uint32_t graphs) {
+  GsBorScope s;
+  if (graphs == 1) {
+    if (V <= 8192) s.blocks = 16;
+    return s;
+  }
+  s.blocks = graphs > 36 ? 4 : graphs > 18 ? 8 : 16;
+  s.wide = V > 4096 && graphs <= 18;
+  return s;
 }
 
 gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, const uint32_t* st) {

@@ -30,8 +30,7 @@ void gs_free_graph(gs_graph* g) {
   if (g->h_qlabels) cudaFreeHost(g->h_qlabels);
   if (g->ev_query) cudaEventDestroy(g->ev_query);
   cudaFree(g->d_status);
-  cudaFree(g->d_parent); cudaFree(g->d_size); cudaFree(g->d_res); cudaFree(g->d_samp); cudaFree(g->d_acc);
-  cudaFree(g->d_forest);
+  cudaFree(g->d_bor); cudaFree(g->d_res); cudaFree(g->d_acc);
   cudaFree(g->d_store);
   cudaFree(g->d_store_list);
   cudaFree(g->d_store_status);
@@ -185,12 +184,7 @@ gs_status gs_graph_create(const gs_graph_config* cfg, gs_graph** out) {
   GS_CUDA_TRY(cudaMalloc(&g->d_status, 32 * sizeof(uint32_t)));
   GS_CUDA_TRY(cudaMemsetAsync(g->d_status, 0, 32 * sizeof(uint32_t), g->stream));
   GS_CUDA_TRY(cudaMallocHost(&g->h_status, 32 * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_parent, (size_t)V * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_size, (size_t)V * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_res, (size_t)V * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_samp, (size_t)V * sizeof(uint64_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_acc, (size_t)V * (bkt + 1) * sizeof(GsBucket)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_forest, (size_t)2 * V * sizeof(uint32_t)));
+  GS_TRY(gs_alloc_boruvka(g.get(), V, bkt + 1, true));
   GS_CUDA_TRY(cudaStreamSynchronize(g->stream));
   *out = g.release();
   return GS_OK;
@@ -575,6 +569,8 @@ gs_status gs_spanning_forest(gs_graph* g, uint32_t level, uint32_t* edges, uint6
   GS_TRY(gs_connected_components(g, level, nullptr, nullptr, nullptr));
   GS_GUARD(g);
   if (g->last_answer_eager) GS_TRY(gs_eager_forest(g, g->stream));  // the eager forest, as the reference returns
+  else GS_TRY(gs_gather_forest(g, g->stream));
+  GS_CUDA_TRY(cudaStreamSynchronize(g->stream));
   *num_edges = g->last_forest_edges;
   GS_CUDA_TRY(cudaMemcpy(edges, g->d_forest, (size_t)2 * g->last_forest_edges * sizeof(uint32_t),
                          cudaMemcpyDeviceToHost));
@@ -600,6 +596,8 @@ gs_status gs_disjoint_spanning_forests(gs_graph* g, uint32_t level, uint32_t k, 
     // connected-components graph resets it before every query (CCSketchAlg::connected_components)
     const uint32_t col0 = (g->num_levels > 1 || g->num_subgraphs > 1) ? g->sample_cursor[level]++ : 0;
     st = gs_boruvka(g, level, col0, s);
+    if (st != GS_OK) break;
+    st = gs_gather_forest(g, s);
     if (st != GS_OK) break;
     const uint32_t ne = g->last_forest_edges;
     sizes[j] = ne;

@@ -230,6 +230,7 @@ gs_status gs_eager_rebuild(gs_graph* g, cudaStream_t s) {
   GS_CUDA_TRY(cudaMemsetAsync(g->d_eager_set, 0, ((size_t)g->eager_mask + 1) * sizeof(GsEagerSlot), s));
   GS_CUDA_TRY(cudaMemsetAsync(g->d_eager_status, 0, 4 * sizeof(uint32_t), s));
   if (g->last_forest_edges) {
+    GS_TRY(gs_gather_forest(g, s));
     k_eager_load_forest<<<grid_for_items(g, g->last_forest_edges), kEagerThreads, 0, s>>>(
         g->d_forest, g->last_forest_edges, g->d_eager_set, g->eager_mask, g->d_eager_status);
     GS_CUDA_TRY(cudaGetLastError());

@@ -157,11 +157,10 @@ struct gs_engine {
   GsBorTenant* d_bor = nullptr;  // [max_tenants + 1]
   uint32_t* d_vtenant = nullptr; // [max_vertices]
   uint32_t* d_tstate = nullptr;  // [(max_tenants + 1) * 4] Boruvka per-tenant state
-  unsigned long long* d_largest = nullptr;  // [max_tenants + 1] largest component of each tenant per round
   uint32_t* h_tstate = nullptr;  // pinned mirror
   uint32_t* d_qstatus = nullptr; // [16] Boruvka status words
   uint32_t* h_qstatus = nullptr; // pinned [16]
-  uint32_t* d_q = nullptr;       // [2 * (max_tenants + 1)] query list, then label offsets
+  uint32_t* d_q = nullptr;       // [3 * (max_tenants + 1)] query list, label offsets, query list by size
   uint32_t* h_q = nullptr;       // pinned mirror
   uint32_t* d_ncc = nullptr;     // [max_tenants + 1]
   // Slice tables (record offsets and tenants) of an ingest, two sets so that one ingest's tables
@@ -186,7 +185,7 @@ namespace {
 void free_engine(gs_engine* e) {
   if (!e) return;
   if (e->g) gs_free_graph(e->g);
-  cudaFree(e->d_ing); cudaFree(e->d_bor); cudaFree(e->d_vtenant); cudaFree(e->d_tstate); cudaFree(e->d_largest);
+  cudaFree(e->d_ing); cudaFree(e->d_bor); cudaFree(e->d_vtenant); cudaFree(e->d_tstate);
   cudaFree(e->d_qstatus); cudaFree(e->d_q); cudaFree(e->d_ncc);
   for (auto& tb : e->tabs) {
     cudaFree(tb.d_off); cudaFree(tb.d_ten);
@@ -298,18 +297,14 @@ gs_status copy_slices(const gs_engine::SliceTables& tb, uint32_t ns, cudaStream_
   return GS_OK;
 }
 
-// Queues one multi-tenant Boruvka launch and the read-back of its results into pinned memory.
+// Graphs too large for a cluster that a query still answers one after the other with the whole GPU.
+constexpr uint32_t kMaxGridQueries = 2;
+
+// Queues the multi-tenant Boruvka launch and the read-back of its results into pinned memory.
 // The pinned query tables must not be read by queued work any more.
 gs_status enqueue_query(gs_engine* e, const QueryPlan& qp, const uint32_t* tenants, uint32_t count, cudaStream_t s) {
   gs_graph* g = e->g;
   const uint32_t T1 = e->max_tenants + 1;
-  // every tenant done except the listed ones; the idle slot stays done
-  for (uint32_t t = 0; t < T1; t++) {
-    e->h_tstate[4 * t] = t < e->max_tenants && qp.seen[t] ? 0u : 1u;
-    e->h_tstate[4 * t + 1] = e->h_tstate[4 * t + 2] = e->h_tstate[4 * t + 3] = 0u;
-  }
-  std::memset(e->h_qstatus, 0, 16 * sizeof(uint32_t));
-  e->h_qstatus[5] = count;
   uint32_t off = 0;
   for (uint32_t i = 0; i < count; i++) {
     e->h_q[i] = tenants[i];
@@ -319,35 +314,47 @@ gs_status enqueue_query(gs_engine* e, const QueryPlan& qp, const uint32_t* tenan
   if (g->acc_dirty)
     GS_CUDA_TRY(cudaMemsetAsync(g->d_acc, 0, (size_t)e->max_vertices * e->W * sizeof(GsBucket), s));
   g->acc_dirty = true;
-  GS_CUDA_TRY(cudaMemcpyAsync(e->d_tstate, e->h_tstate, (size_t)T1 * 4 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  GS_CUDA_TRY(cudaMemcpyAsync(e->d_qstatus, e->h_qstatus, 16 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  GS_CUDA_TRY(cudaMemcpyAsync(e->d_q, e->h_q, (size_t)2 * T1 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  // one cluster per graph, the largest graphs first (the launch ends when the last cluster does); up to
+  // kMaxGridQueries graphs that would keep a cluster busy for longer get the whole GPU, one after the other
+  uint32_t* order = e->h_q + 2 * (size_t)T1;
+  std::copy(tenants, tenants + count, order);
+  std::stable_sort(order, order + count, [&](uint32_t a, uint32_t b) { return e->ten[a].V > e->ten[b].V; });
+  uint32_t large = 0;
+  while (large < count && e->ten[order[large]].V > (count == 1 ? 8192u : 65536u)) large++;
+  if (large > kMaxGridQueries) large = 0;
+  GS_CUDA_TRY(cudaMemsetAsync(e->d_qstatus, 0, 16 * sizeof(uint32_t), s));
+  GS_CUDA_TRY(cudaMemcpyAsync(e->d_q, e->h_q, (size_t)3 * T1 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   GS_CUDA_TRY(cudaMemsetAsync(e->d_ncc, 0, (size_t)count * sizeof(uint32_t), s));
 
   GsBorLaunch L;
   L.sk = g->d_sk;
   L.tenants = e->d_bor;
-  L.vtenant = e->d_vtenant;
-  L.T = T1;
-  L.vlo = qp.vlo;
-  L.V = qp.vhi;
+  L.vertices = e->max_vertices;
   L.W = e->W;
-  L.max_rounds = qp.max_rounds;
+  for (uint32_t i = 0; i < count; i++) L.R = std::max(L.R, e->ten[tenants[i]].geom.bkt_per_col + 1);
   L.parent = g->d_parent;
   L.size = g->d_size;
   L.acc = g->d_acc;
-  L.samp = g->d_samp;
-  L.roots = g->d_res;
-  L.forest = g->d_forest;
-  L.forest_cap = e->max_vertices;
+  L.members = g->d_members;
+  L.tasks = g->d_tasks;
   L.status = e->d_qstatus;
   L.tstate = e->d_tstate;
+  L.counters = g->d_bor_ctr;
   // tenants only take edge records, which reach both endpoints: every tenant's sketches XOR to zero
   L.complement = 1;
-  L.largest = e->d_largest;
   {
-    GsProfScope ps(g, GS_PROF_QUERY, s, 2);
-    GS_TRY(gs_boruvka_launch(L, s));
+    GsProfScope ps(g, GS_PROF_QUERY, s, large + (large < count) + 1);
+    for (uint32_t i = 0; i < large; i++) {
+      L.tenant = order[i];
+      GS_TRY(gs_boruvka_launch(L, s));
+    }
+    if (large < count) {
+      L.count = count - large;
+      L.qlist = e->d_q + 2 * (size_t)T1 + large;
+      L.scope = gs_boruvka_scope(e->ten[order[large]].V, L.count);
+      if (!L.scope.blocks) L.scope = GsBorScope{16, true};   // one graph left
+      GS_TRY(gs_boruvka_launch(L, s));
+    }
     const dim3 grid((unsigned)std::min<uint64_t>((qp.maxv + 255) / 256, 64), count);
     k_gather_labels<<<grid, 256, 0, s>>>(g->d_parent, e->d_q, e->d_q + T1, e->d_bor, g->d_res, e->d_ncc);
     GS_CUDA_TRY(cudaGetLastError());
@@ -471,16 +478,11 @@ gs_status gs_engine_create(const gs_engine_config* cfg, gs_engine** out) {
   GS_CUDA_TRY(cudaMemsetAsync(g->d_status, 0, 32 * sizeof(uint32_t), g->stream));
   GS_CUDA_TRY(cudaMallocHost(&g->h_status, 32 * sizeof(uint32_t)));
   const size_t V = e->max_vertices;
-  GS_CUDA_TRY(cudaMalloc(&g->d_parent, V * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_size, V * sizeof(uint32_t)));
+  GS_TRY(gs_alloc_boruvka(g, V, e->W, false));
   GS_CUDA_TRY(cudaMalloc(&g->d_res, V * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_samp, V * sizeof(uint64_t)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_acc, V * e->W * sizeof(GsBucket)));
-  GS_CUDA_TRY(cudaMalloc(&g->d_forest, 2 * V * sizeof(uint32_t)));
 
   GS_CUDA_TRY(cudaMalloc(&e->d_ing, (size_t)T1 * sizeof(GsIngTenant)));
   GS_CUDA_TRY(cudaMalloc(&e->d_bor, (size_t)T1 * sizeof(GsBorTenant)));
-  GS_CUDA_TRY(cudaMalloc(&e->d_largest, (size_t)T1 * sizeof(unsigned long long)));
   GS_CUDA_TRY(cudaMemsetAsync(e->d_ing, 0, (size_t)T1 * sizeof(GsIngTenant), g->stream));
   GS_CUDA_TRY(cudaMemsetAsync(e->d_bor, 0, (size_t)T1 * sizeof(GsBorTenant), g->stream));
   GS_CUDA_TRY(cudaMalloc(&e->d_vtenant, V * sizeof(uint32_t)));
@@ -490,8 +492,8 @@ gs_status gs_engine_create(const gs_engine_config* cfg, gs_engine** out) {
   GS_CUDA_TRY(cudaMallocHost(&e->h_tstate, (size_t)T1 * 4 * sizeof(uint32_t)));
   GS_CUDA_TRY(cudaMalloc(&e->d_qstatus, 32 * sizeof(uint32_t)));
   GS_CUDA_TRY(cudaMallocHost(&e->h_qstatus, 16 * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMalloc(&e->d_q, (size_t)2 * T1 * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMallocHost(&e->h_q, (size_t)2 * T1 * sizeof(uint32_t)));
+  GS_CUDA_TRY(cudaMalloc(&e->d_q, (size_t)3 * T1 * sizeof(uint32_t)));
+  GS_CUDA_TRY(cudaMallocHost(&e->h_q, (size_t)3 * T1 * sizeof(uint32_t)));
   GS_CUDA_TRY(cudaMalloc(&e->d_ncc, (size_t)T1 * sizeof(uint32_t)));
   for (auto& tb : e->tabs) GS_CUDA_TRY(cudaEventCreateWithFlags(&tb.ev_free, cudaEventDisableTiming));
   g->d_vtenant = e->d_vtenant;

@@ -113,13 +113,17 @@ struct gs_graph {
   cudaEvent_t ev_query = nullptr;  // recorded after the labels' read-back
 
   // ---- Boruvka scratch ----
+  void* d_bor = nullptr;         // the arrays below, up to d_acc
   uint32_t* d_parent = nullptr;  // [V]
   uint32_t* d_size = nullptr;    // [V]
-  uint32_t* d_res = nullptr;     // [V] sample result code
-  uint64_t* d_samp = nullptr;    // [V] sampled edge id
+  uint32_t* d_members = nullptr; // [4][V] member ranks, run offsets, member lists, large components
+  uint4* d_tasks = nullptr;      // [V] member runs to gather
+  uint32_t* d_bor_ctr = nullptr; // [kGsBorCounterWords]
+  uint64_t* d_edge = nullptr;    // [V] edge of every vertex that the last Boruvka run hooked
+  uint32_t* d_forest = nullptr;  // [2*(V-1)] forest edges of the last Boruvka run, once gathered
+  uint32_t* d_res = nullptr;     // [V] an engine's gathered labels
   GsBucket* d_acc = nullptr;     // [V][bkt_per_col+1] merged column + deterministic bucket
   bool acc_dirty = true;         // d_acc may hold non-zero rows (new, or a query ended early)
-  uint32_t* d_forest = nullptr;  // [2*(V-1)] forest edges of the last Boruvka run
   uint32_t last_forest_edges = 0;
   uint32_t last_rounds = 0;
   std::vector<uint32_t> sample_cursor;  // per level: round-0 column of the next k-forest
@@ -214,7 +218,7 @@ gs_status gs_ingest_device_batches(gs_graph* g, uint32_t level, const uint32_t* 
                                    const uint64_t* d_starts, const uint64_t* d_sizes,
                                    uint32_t nb, const uint32_t* d_dsts, cudaStream_t s,
                                    uint64_t max_records = 0);  // 0: read the record count back
-// Device Boruvka on one level; forest edges stay in g->d_forest.
+// Device Boruvka on one level; its forest stays in g->d_edge (gs_gather_forest).
 gs_status gs_boruvka(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s);
 // The same in two halves: the launch and the read-back of status words [0, 17) into pinned h_out
 // (word 16: ingest error bits queued before the query), queued on s without waiting; then, once
@@ -251,32 +255,49 @@ struct GsBorTenant {
   uint32_t round0_col;  // column sampled in round 0
 };
 
-struct GsBorLaunch {
-  const GsBucket* sk = nullptr;
-  const GsBorTenant* tenants = nullptr;  // device [T] when T > 1
-  GsBorTenant t0{};                      // the tenant when T == 1
-  const uint32_t* vtenant = nullptr;     // device [V] when T > 1
-  uint32_t T = 1, V = 0, W = 0, max_rounds = 0;
-  uint32_t vlo = 0;                      // vertices [vlo, V) take part
-  uint32_t* parent = nullptr;
-  uint32_t* size = nullptr;
-  GsBucket* acc = nullptr;
-  uint64_t* samp = nullptr;              // [V]
-  uint32_t* roots = nullptr;             // [V]
-  uint32_t* forest = nullptr;
-  uint32_t forest_cap = 0;
-  uint32_t* status = nullptr;            // 8 words: [0] errors [4] forest edges [5] running tenants [6,7] barrier
-  uint32_t* tstate = nullptr;            // [T][4]: done, modified, rounds, out of samples
-  uint64_t wait_ns = kGsDefaultWaitNs;   // grid-barrier wait limit
-  // Only when every graph's vertex sketches XOR to zero (every update reached both endpoints): each
-  // graph's largest component's merged column is taken as the XOR of the graph's vertices outside it,
-  // so the accumulate phase never reads the largest components' own members.  `largest` is device
-  // scratch of T 64-bit words.
-  uint32_t complement = 0;
-  unsigned long long* largest = nullptr;
+// Words of the counter sets of a grid-wide launch (two of them, then the barrier's arrivals).
+constexpr uint32_t kGsBorCounterWords = 32;
+
+// Where a graph's Boruvka rounds run: on a cluster of `blocks` blocks, or on the whole GPU (0).
+struct GsBorScope {
+  uint32_t blocks = 0;
+  bool wide = false;   // blocks of 1024 threads instead of 512
 };
 
-// All Boruvka rounds of every tenant in one cooperative launch (queued on s, no host sync).
+struct GsBorLaunch {
+  const GsBucket* sk = nullptr;
+  const GsBorTenant* tenants = nullptr;  // device table, or null: the one graph t0
+  GsBorTenant t0{};
+  GsBorScope scope;
+  uint32_t count = 1;                    // graphs (cluster scope)
+  const uint32_t* qlist = nullptr;       // device [count] tenants (cluster scope with a table)
+  uint32_t tenant = 0;                   // the tenant (grid scope with a table)
+  uint64_t vertices = 0;                 // length of the per-vertex arrays
+  uint32_t W = 0;                        // accumulator row width
+  uint32_t R = 0;                        // largest bkt_per_col + 1 of the launch's graphs
+  uint32_t* parent = nullptr;
+  uint32_t* size = nullptr;
+  GsBucket* acc = nullptr;               // [vertices][W], all zero
+  uint32_t* members = nullptr;           // [4][vertices]
+  uint4* tasks = nullptr;                // [vertices]
+  uint64_t* edge = nullptr;              // [vertices] edge of every vertex that a union hooked; may be null
+  uint32_t* status = nullptr;            // [0] errors [4] forest edges (with `edge`)
+  uint32_t* tstate = nullptr;            // [tenant][4]: done, -, rounds, out of samples
+  uint32_t* counters = nullptr;          // [kGsBorCounterWords] (grid scope)
+  uint64_t wait_ns = kGsDefaultWaitNs;   // grid-barrier wait limit
+  // Only when every graph's vertex sketches XOR to zero (every update reached both endpoints): the
+  // largest component's merged column is taken as the XOR of the vertices outside it.
+  uint32_t complement = 0;
+};
+
+// The scope of a query of `graphs` graphs of at most V vertices.
+GsBorScope gs_boruvka_scope(uint32_t V, uint32_t graphs);
+// The Boruvka scratch of a handle over `vertices` vertices with accumulator rows of `width` buckets.
+gs_status gs_alloc_boruvka(gs_graph* g, uint64_t vertices, uint32_t width, bool forest);
+// The last query's last_forest_edges forest edges into g->d_forest (queued on s).
+gs_status gs_gather_forest(gs_graph* g, cudaStream_t s);
+
+// All Boruvka rounds of the launch's graphs in one kernel (queued on s, no host sync).
 gs_status gs_boruvka_launch(const GsBorLaunch& L, cudaStream_t s);
 
 // Exact global min cut (host), gs_mincut.cpp.
