@@ -125,17 +125,21 @@ __device__ __forceinline__ uint32_t gs_depth_low(uint64_t x, uint32_t* h2_out) {
   return (uint32_t)__ffs((int)(l2 ^ __funnelshift_r(l2, h2, 28))) - 1u;
 }
 
-// min(ctz(final hash's low word), cap) for capbit = 1 << cap, cap < 32: the cap bit is OR-ed in by the
-// same three-input logic op as the xorshift, so the capped depth costs no instruction more than the
-// uncapped one.  A result of cap means "cap or deeper".
-__device__ __forceinline__ uint32_t gs_depth_capped(uint64_t x, uint32_t capbit) {
+// The final hash's low word with the cap bit 1 << cap (cap < 32) OR-ed in by the same three-input logic op
+// as the xorshift: its lowest set bit is min(depth, cap), and the cap costs no instruction.
+__device__ __forceinline__ uint32_t gs_low_capped(uint64_t x, uint32_t capbit) {
   uint64_t h = x * kGsMx2;
   uint32_t lo = (uint32_t)h, hi = (uint32_t)(h >> 32);
   lo ^= __umulhi(hi, 1u << 29) + 8u;
   h = ((uint64_t)hi << 32) | lo;
   h *= kGsMx2;
   const uint32_t l2 = (uint32_t)h, h2 = (uint32_t)(h >> 32);
-  return (uint32_t)__ffs((int)((l2 ^ __funnelshift_r(l2, h2, 28)) | capbit)) - 1u;
+  return (l2 ^ __funnelshift_r(l2, h2, 28)) | capbit;
+}
+
+// min(ctz(final hash's low word), cap) for capbit = 1 << cap; a result of cap means "cap or deeper"
+__device__ __forceinline__ uint32_t gs_depth_capped(uint64_t x, uint32_t capbit) {
+  return (uint32_t)__ffs((int)gs_low_capped(x, capbit)) - 1u;
 }
 
 __device__ __forceinline__ uint32_t gs_depth_finish(uint32_t d_low, uint32_t h2, uint32_t max_depth) {

@@ -108,6 +108,15 @@ __device__ uint2 block_exclusive_scan(uint2 x, uint2* total) {
   return res;
 }
 
+// Work of the sketch update, reset before the first kernel that adds to it: status[2] = work chunks listed,
+// status[3] = vertices of few records listed, status[13] = next of those, status[14] = next work chunk.
+__device__ __forceinline__ void reset_work(uint32_t* status) {
+  status[2] = 0;
+  status[3] = 0;
+  status[13] = 0;
+  status[14] = 0;
+}
+
 // ---- two-level counting sort of the records by virtual vertex ----
 //
 // Pass 1 partitions the records by the high bits of their key (key >> LB, at most kMaxBuckets
@@ -187,6 +196,7 @@ __global__ void __launch_bounds__(kScanThreads) k_part_scan(uint32_t* __restrict
     choff[H] = carry.y;
     status[1] = carry.x;
     status[5] = carry.y;
+    reset_work(status);
   }
 }
 
@@ -594,108 +604,148 @@ __global__ void k_scatter_batches(const uint32_t* __restrict__ srcs, const uint6
   }
 }
 
+// The lists that the sketch update works from.  A vertex of at most kFewRecords goes to `few`; any other is
+// cut into work chunks of at most `chunk` records, work[i] = {vertex, chunk of the vertex}.  Both are in any
+// order.
+constexpr uint32_t kFewRecords = 64;
+
+struct WorkLists {
+  uint32_t* few;
+  uint2* work;
+  uint32_t work_cap, chunk;
+  uint32_t* status;
+};
+
+// Lists the block's vertices (one a thread; n = 0: nothing to list), with one reservation per block.
+__device__ __forceinline__ void list_vertices(const WorkLists& L, uint32_t v, uint32_t n) {
+  __shared__ uint2 s_at;
+  const bool few = n > 0 && n <= kFewRecords;
+  const uint32_t nch = n > kFewRecords ? (n + L.chunk - 1) / L.chunk : 0u;
+  uint2 tot;
+  uint2 at = block_exclusive_scan(make_uint2(few ? 1u : 0u, nch), &tot);
+  if (threadIdx.x == 0) {
+    s_at.x = tot.x ? atomicAdd(&L.status[3], tot.x) : 0u;
+    s_at.y = tot.y ? atomicAdd(&L.status[2], tot.y) : 0u;
+  }
+  __syncthreads();
+  at = add2(at, s_at);
+  if (few) L.few[at.x] = v;
+  // a vertex of a few chunks writes its own entries; the warp writes a hub vertex's together
+  constexpr uint32_t kOwn = 8;
+  if (nch <= kOwn) {
+    for (uint32_t i = 0; i < nch; i++)
+      if (at.y + i < L.work_cap) L.work[at.y + i] = make_uint2(v, i);
+      else atomicOr(L.status, (uint32_t)GS_DEV_ERR_CAPACITY);
+  }
+  for (uint32_t m = __ballot_sync(0xffffffffu, nch > kOwn); m; m &= m - 1) {
+    const uint32_t src = __ffs(m) - 1;
+    const uint32_t w0 = __shfl_sync(0xffffffffu, at.y, src), wn = __shfl_sync(0xffffffffu, nch, src);
+    const uint32_t hv = __shfl_sync(0xffffffffu, v, src);
+    for (uint32_t i = lane_id(); i < wn; i += 32)
+      if (w0 + i < L.work_cap) L.work[w0 + i] = make_uint2(hv, i);
+      else atomicOr(L.status, (uint32_t)GS_DEV_ERR_CAPACITY);
+  }
+  __syncthreads();   // s_at and the scan's words may be used again
+}
+
+// Offsets of the directed batches' vertices: an exclusive scan of the counts over all vertices, in three
+// kernels.  (Edge records need none: pass 1 has placed every bucket, so k_vert_offsets scans inside them.)
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const uint32_t* __restrict__ cnt, uint32_t nv,
-                                                             uint32_t chunk, uint32_t* __restrict__ off,
-                                                             uint32_t* __restrict__ choff,
+                                                             uint32_t* __restrict__ off,
                                                              uint32_t* __restrict__ tile_sums) {
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanPer;
-  uint2 v[kScanPer];
+  uint32_t v[kScanPer];
   uint2 s = make_uint2(0, 0);
 #pragma unroll
   for (int k = 0; k < kScanPer; k++) {
     uint64_t i = base + k;
-    uint32_t c = i < nv ? cnt[i] : 0u;
-    v[k] = make_uint2(c, (c + chunk - 1) / chunk);
-    s = add2(s, v[k]);
+    v[k] = i < nv ? cnt[i] : 0u;
+    s.x += v[k];
   }
   uint2 tot;
-  uint2 ex = block_exclusive_scan(s, &tot);
+  uint32_t ex = block_exclusive_scan(s, &tot).x;
 #pragma unroll
   for (int k = 0; k < kScanPer; k++) {
     uint64_t i = base + k;
-    if (i < nv) { off[i] = ex.x; choff[i] = ex.y; }
-    ex = add2(ex, v[k]);
+    if (i < nv) off[i] = ex;
+    ex += v[k];
   }
-  if (threadIdx.x == 0) { tile_sums[2 * blockIdx.x] = tot.x; tile_sums[2 * blockIdx.x + 1] = tot.y; }
+  if (threadIdx.x == 0) tile_sums[blockIdx.x] = tot.x;
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_top(uint32_t* __restrict__ tile_sums, uint32_t tiles,
-                                                           uint32_t* __restrict__ off,
-                                                           uint32_t* __restrict__ choff, uint32_t nv,
                                                            uint32_t* __restrict__ status) {
-  uint2 carry = make_uint2(0, 0);
+  uint32_t carry = 0;
   for (uint32_t b0 = 0; b0 < tiles; b0 += kScanThreads) {
     uint32_t i = b0 + threadIdx.x;
-    uint2 x = i < tiles ? make_uint2(tile_sums[2 * i], tile_sums[2 * i + 1]) : make_uint2(0, 0);
     uint2 tot;
-    uint2 ex = block_exclusive_scan(x, &tot);
-    if (i < tiles) { tile_sums[2 * i] = ex.x + carry.x; tile_sums[2 * i + 1] = ex.y + carry.y; }
-    carry = add2(carry, tot);
+    const uint2 ex = block_exclusive_scan(make_uint2(i < tiles ? tile_sums[i] : 0u, 0u), &tot);
+    if (i < tiles) tile_sums[i] = ex.x + carry;
+    carry += tot.x;
   }
   if (threadIdx.x == 0) {
-    off[nv] = carry.x;
-    choff[nv] = carry.y;
-    status[1] = carry.x;
-    status[2] = carry.y;
-    status[14] = 0;  // next work chunk of the packed sketch update
+    status[1] = carry;
+    reset_work(status);
   }
 }
 
-// adds the tile prefixes and resets the counters to the record cursors used by the scatter; with an
-// owner table, also records the vertex of each of its work chunks below owner_cap, so the sketch
-// update finds a chunk's vertex with one load instead of a search over choff
-__global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t* __restrict__ off, uint32_t* __restrict__ choff,
-                                                           uint32_t* __restrict__ cursor,
+// adds the tile prefixes, turns the counts into the record cursors used by the scatter and lists the vertices
+__global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t* __restrict__ off, uint32_t* __restrict__ cursor,
                                                            const uint32_t* __restrict__ tile_sums, uint32_t nv,
-                                                           uint32_t chunk, uint32_t* __restrict__ owner,
-                                                           uint32_t owner_cap) {
-  const uint32_t t = blockIdx.x;
-  const uint32_t a = tile_sums[2 * t], b = tile_sums[2 * t + 1];
-  const uint64_t base = (uint64_t)t * kScanTile + (uint64_t)threadIdx.x * kScanPer;
-  const uint32_t lane = threadIdx.x & 31u;
+                                                           const WorkLists L) {
+  const uint32_t a = tile_sums[blockIdx.x];
+  const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanPer;
 #pragma unroll
   for (int k = 0; k < kScanPer; k++) {
     const uint64_t i = base + k;
-    uint32_t c0 = 0, n = 0;
+    uint32_t n = 0;
     if (i < nv) {
-      const uint32_t o = off[i] + a;
-      off[i] = o;
-      c0 = choff[i] + b;
-      choff[i] = c0;
-      if (owner) n = (cursor[i] + chunk - 1) / chunk;   // cursor still holds the count here
-      cursor[i] = o;
+      n = cursor[i];
+      cursor[i] = off[i] = off[i] + a;
     }
-    if (owner) {
-      // a vertex of a few chunks writes its own entries; the warp writes a hub vertex's together
-      constexpr uint32_t kOwnFew = 8;
-      if (n <= kOwnFew)
-        for (uint32_t c = c0; c < c0 + n && c < owner_cap; c++) owner[c] = (uint32_t)i;
-      for (uint32_t m = __ballot_sync(0xffffffffu, n > kOwnFew); m; m &= m - 1) {
-        const uint32_t src = __ffs(m) - 1;
-        const uint32_t hc0 = __shfl_sync(0xffffffffu, c0, src), hn = __shfl_sync(0xffffffffu, n, src);
-        const uint32_t hv = __shfl_sync(0xffffffffu, (uint32_t)i, src);
-        for (uint32_t c = hc0 + lane; c < hc0 + hn && c < owner_cap; c += 32) owner[c] = hv;
-      }
+    list_vertices(L, (uint32_t)i, n);
+  }
+}
+
+// Offsets of the vertices of one bucket (a block each): the bucket's first record plus an exclusive scan of
+// its vertices' counts, which become the cursors of the placement.  The vertices are listed for the update.
+__global__ void __launch_bounds__(kPartThreads) k_vert_offsets(const uint32_t* __restrict__ bkt, uint32_t H, uint32_t lb,
+                                                               uint32_t nv, uint32_t* __restrict__ off,
+                                                               uint32_t* __restrict__ cursor, const WorkLists L) {
+  const uint32_t d = blockIdx.x;
+  const uint64_t v0 = (uint64_t)d << lb, v1 = min((uint64_t)nv, v0 + ((uint64_t)1 << lb));
+  uint32_t run = bkt[H + d];
+  for (uint64_t b = v0; b < v1; b += kPartThreads) {
+    const uint64_t v = b + threadIdx.x;
+    const uint32_t n = v < v1 ? cursor[v] : 0u;
+    uint2 tot;
+    const uint32_t at = run + block_exclusive_scan(make_uint2(n, 0u), &tot).x;
+    if (v < v1) {
+      off[v] = at;
+      cursor[v] = at;
     }
+    run += tot.x;
+    list_vertices(L, (uint32_t)v, n);
   }
 }
 
 // ---- the sketch update ----
 
+// A vertex's records are nbr[off[v] .. end[v]).
 struct IngestArgs {
   const uint32_t* off;
-  const uint32_t* choff;
+  const uint32_t* end;
   const uint32_t* nbr;
   GsBucket* sk;
   const uint64_t* colmix;   // [C] column constants, [C] = checksum constant; per tenant: [T][kColStride]
-  const uint32_t* status;   // [2] = work chunks
+  uint32_t* status;         // error bits and the work counters (reset_work)
+  const uint32_t* few;
+  const uint2* work;
   uint32_t nv, V, C, bkt, nb, chunk;
   const uint32_t* vtenant;       // tenant of every vertex (tenant variant only)
   const GsIngTenant* tenants;    // geometry and arena offset of every tenant (tenant variant only)
   uint32_t warp_words;           // shared memory per warp in uint4 (packed variant only)
-  uint32_t* next_chunk;          // work-chunk counter, zero at launch (packed variant only)
-  const uint32_t* owner;         // vertex of every work chunk below owner_cap (may be null)
-  uint32_t owner_cap;
+  uint64_t seed;                 // k_ingest_direct without a constant table
 };
 
 // ---- packed lane layout (sketches of at most 24 columns) ----
@@ -736,19 +786,6 @@ GS_HD uint32_t pack_p1(uint32_t C) { return (C + 7u) & ~7u; }
 // uint4 words per warp: rows of the main lanes and of the spare slots, then the staged records
 GS_HD uint32_t pack_warp_words(uint32_t C) {
   return (uint32_t)kPackRowsAlloc * (pack_p1(C) + (pack_spare_lanes(C) ? kPackRounds * 8u : 0u)) + kRecWords;
-}
-
-__device__ __forceinline__ uint32_t chunk_owner(const IngestArgs& A, uint32_t ch, uint32_t lane) {
-  uint32_t lo = 0, hi = A.nv;
-  while (hi - lo > 1) {
-    const uint32_t step = (hi - lo + 31) / 32;
-    const uint32_t probe = lo + (lane + 1) * step;
-    const bool le = probe < hi && A.choff[probe] <= ch;
-    const uint32_t k = __popc(__ballot_sync(0xffffffffu, le));
-    lo = lo + k * step;
-    hi = min(hi, lo + step);
-  }
-  return lo;
 }
 
 __device__ __forceinline__ void xor_bucket_global(GsBucket* p, uint64_t a, uint64_t g) {
@@ -815,25 +852,18 @@ __global__ void __launch_bounds__(512) k_ingest(const IngestArgs A) {
     }
   }
 
+  // warps take work chunks from a counter; lane 0 fetches the next index while the current chunk runs
   const uint32_t total = A.status[2];
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-
-  // with a chunk counter, warps take work chunks from it (lane 0 fetches the next index while the
-  // current chunk runs); without one, a fixed stride
-  const bool dyn = A.next_chunk != nullptr;
   uint32_t nxt = 0;
-  if (dyn && lane == 0) nxt = atomicAdd(A.next_chunk, 1u);
-  for (uint32_t ch = dyn ? __shfl_sync(0xffffffffu, nxt, 0) : gw; ch < total;
-       ch = dyn ? __shfl_sync(0xffffffffu, nxt, 0) : ch + nw) {
-    if (dyn && lane == 0) nxt = atomicAdd(A.next_chunk, 1u);
-    const uint32_t vv = ch < A.owner_cap ? A.owner[ch] : chunk_owner(A, ch, lane);
-    const uint32_t c0 = A.choff[vv];
-    // a vertex of one chunk is this warp's alone: its merge is a plain read-modify-write (many small
-    // vertices, as an engine's tenants have, would saturate the L2 atomics)
-    const bool exclusive = (A.choff[vv + 1] - c0) == 1;
-    const uint32_t rb = A.off[vv] + (ch - c0) * A.chunk;
-    const uint32_t re = min(A.off[vv + 1], rb + A.chunk);
+  if (lane == 0) nxt = atomicAdd(&A.status[14], 1u);
+  for (uint32_t ch = __shfl_sync(0xffffffffu, nxt, 0); ch < total; ch = __shfl_sync(0xffffffffu, nxt, 0)) {
+    if (lane == 0) nxt = atomicAdd(&A.status[14], 1u);
+    const uint2 wk = A.work[ch];
+    const uint32_t vv = wk.x, first = A.off[vv], last = A.end[vv];
+    // a vertex of one chunk is this warp's alone: its merge is a plain read-modify-write
+    const bool exclusive = last - first <= A.chunk;
+    const uint32_t rb = first + wk.y * A.chunk;
+    const uint32_t re = min(last, rb + A.chunk);
     uint32_t v, vb = 0;  // vb: first engine vertex id of the tenant (neighbours are stored engine-wide)
     GsBucket* skv;
     if (TEN) {
@@ -1014,13 +1044,13 @@ __global__ void __launch_bounds__(kPackMaxThreads, 2) k_ingest_packed(const Inge
   // warps take work chunks from a counter, so no warp idles while others still have long chunks
   // left; lane 0 fetches the next index while the current chunk runs
   uint32_t nxt = 0;
-  if (lane == 0) nxt = atomicAdd(A.next_chunk, 1u);
+  if (lane == 0) nxt = atomicAdd(&A.status[14], 1u);
   for (uint32_t ch = __shfl_sync(0xffffffffu, nxt, 0); ch < total; ch = __shfl_sync(0xffffffffu, nxt, 0)) {
-    if (lane == 0) nxt = atomicAdd(A.next_chunk, 1u);
-    const uint32_t vv = ch < A.owner_cap ? A.owner[ch] : chunk_owner(A, ch, lane);
-    const uint32_t c0ff = A.choff[vv];
-    const uint32_t rb = A.off[vv] + (ch - c0ff) * A.chunk;
-    const uint32_t re = min(A.off[vv + 1], rb + A.chunk);
+    if (lane == 0) nxt = atomicAdd(&A.status[14], 1u);
+    const uint2 wk = A.work[ch];
+    const uint32_t vv = wk.x;
+    const uint32_t rb = A.off[vv] + wk.y * A.chunk;
+    const uint32_t re = min(A.end[vv], rb + A.chunk);
     uint32_t v, vb = 0;
     GsBucket* skv;
     if (TEN) {
@@ -1211,20 +1241,289 @@ __global__ void __launch_bounds__(kPackMaxThreads, 2) k_ingest_packed(const Inge
   }
 }
 
+// Sketch update of the vertices of few records.  A warp takes up to 32 listed vertices; lane = column, a
+// record's bucket {edge id, checksum} is XORed into the lane's shared-memory row of its depth (a discard row
+// takes what has no row, so the loop has no branch).  What costs in this regime is not the records but the
+// vertex, so rows hold edge ids instead of mixed keys (no inverse mix per bucket), a bit per depth says which
+// rows hold something, and only those are merged, four 16-byte loads of the sketch on their way at once, as
+// plain read-modify-writes: the vertex is this warp's alone.
+// Bound by instruction issue and the latency of the touched sectors together.  @FEW@
+constexpr uint32_t kFewStride = (kSlabDepth + 1) * 32;   // rows of one column group, with the discard row
+constexpr int few_threads(int cg) { return cg == 1 ? 256 : 128; }
+constexpr uint32_t few_warp_words(int cg) { return cg * kFewStride + 32 + 16; }   // uint4: rows, records, mixed keys
+
+__device__ __forceinline__ uint4 ld_bucket(const GsBucket* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
+__device__ __forceinline__ void st_bucket(GsBucket* p, const uint4& t) { __stcg(reinterpret_cast<uint4*>(p), t); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 t;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w) : "r"(a));
+  return t;
+}
+__device__ __forceinline__ uint64_t lds64(uint32_t a) {
+  uint64_t t;
+  asm volatile("ld.shared.u64 %0, [%1];" : "=l"(t) : "r"(a));
+  return t;
+}
+__device__ __forceinline__ void sts128(uint32_t a, const uint4& t) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(t.x), "r"(t.y), "r"(t.z), "r"(t.w) : "memory");
+}
+
+template <int CG, bool TEN>
+__global__ void __launch_bounds__(few_threads(CG), 3) k_ingest_few(const IngestArgs A) {
+  extern __shared__ uint4 smem[];
+  const uint32_t lane = lane_id();
+  uint4* const rows = smem + (size_t)(threadIdx.x >> 5) * few_warp_words(CG);
+  uint4* const rec = rows + CG * kFewStride;
+  uint64_t* const mixed = reinterpret_cast<uint64_t*>(rec + 32);
+  // 32-bit shared-window addresses: the lane's rows, the records, the mixed keys
+  const uint32_t ra = (uint32_t)__cvta_generic_to_shared(rows) + lane * 16u;
+  const uint32_t qa = (uint32_t)__cvta_generic_to_shared(rec), ma = (uint32_t)__cvta_generic_to_shared(mixed);
+
+  uint32_t C = A.C, bkt = A.bkt, nb = A.nb, cur_t = 0xffffffffu;
+  uint64_t csmix = 0, cm[CG];
+  auto set_columns = [&](const uint64_t* cmt) {
+    csmix = cmt[C];
+#pragma unroll
+    for (int g = 0; g < CG; g++) cm[g] = lane + 32u * g < C ? cmt[lane + 32u * g] : 0ull;
+  };
+  if (!TEN) set_columns(A.colmix);
+
+  // vertices a warp takes at once: as many as leave eight turns to every warp
+  const uint32_t total = A.status[3], warps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t grab = min(32u, max(1u, total / (8 * warps)));
+  uint32_t nxt = 0;
+  if (lane == 0) nxt = atomicAdd(&A.status[13], grab);
+  for (uint32_t at = __shfl_sync(0xffffffffu, nxt, 0); at < total; at = __shfl_sync(0xffffffffu, nxt, 0)) {
+    if (lane == 0) nxt = atomicAdd(&A.status[13], grab);
+    // lane l holds what is needed of the l-th vertex
+    const uint32_t have = min(grab, total - at);
+    const bool mine = lane < have;
+    const uint32_t myv = mine ? A.few[at + lane] : 0u;
+    const uint32_t first = mine ? A.off[myv] : 0u, count = mine ? A.end[myv] - first : 0u;
+    uint32_t myt = 0, myvb = 0, mylv = 0;
+    uint64_t mysk = 0;   // first bucket of the vertex's sketch
+    if (TEN) {
+      if (mine) {
+        myt = A.vtenant[myv];
+        const GsIngTenant T = A.tenants[myt];
+        myvb = T.vbase;
+        mylv = myv - myvb;
+        mysk = T.sk_off + (uint64_t)mylv * T.nb;
+      }
+    } else {
+      mylv = myv % A.V;
+      mysk = (uint64_t)myv * nb;
+    }
+
+    uint32_t rb = __shfl_sync(0xffffffffu, first, 0), n = __shfl_sync(0xffffffffu, count, 0);
+    uint32_t nu = lane < n ? A.nbr[rb + lane] : 0u;
+    for (uint32_t i = 0; i < have; i++) {
+      const uint32_t r0 = rb, cnt = n;
+      const uint32_t v = __shfl_sync(0xffffffffu, mylv, i), vb = TEN ? __shfl_sync(0xffffffffu, myvb, i) : 0u;
+      GsBucket* const skv = A.sk + __shfl_sync(0xffffffffu, mysk, i);
+      if (TEN) {
+        const uint32_t t = __shfl_sync(0xffffffffu, myt, i);
+        if (t != cur_t) {
+          cur_t = t;
+          const GsIngTenant T = A.tenants[t];
+          C = T.C;
+          bkt = T.bkt;
+          nb = T.nb;
+          set_columns(A.colmix + (size_t)t * kColStride);
+        }
+      }
+      uint32_t u = nu;
+      if (i + 1 < have) {   // the next vertex's neighbours are loaded under this one's work
+        rb = __shfl_sync(0xffffffffu, first, i + 1);
+        n = __shfl_sync(0xffffffffu, count, i + 1);
+        nu = lane < n ? A.nbr[rb + lane] : 0u;
+        // and its columns' first four depths, which most vertices touch, are asked into L2 (a hint: the tenant's
+        // geometry may be another; 3% of the kernel's time)
+        const GsBucket* col = A.sk + __shfl_sync(0xffffffffu, mysk, i + 1) + (size_t)lane * bkt;
+        if (lane < C) {
+          prefetch_l2(col);
+          prefetch_l2(col + 2);
+        }
+      }
+      // depths below cap are rows, row cap is the discard row; a geometry with more buckets per column than
+      // rows has deeper ones, which go straight to HBM (probability 2^-10 per column)
+      const uint32_t cap = min(bkt, (uint32_t)kSlabDepth), capbit = 1u << cap;
+#pragma unroll
+      for (int g = 0; g < CG; g++)
+        for (uint32_t d = 0; d < cap; d++) sts128(ra + (g * kFewStride + d * 32) * 16u, make_uint4(0, 0, 0, 0));
+      uint32_t held[CG];
+#pragma unroll
+      for (int g = 0; g < CG; g++) held[g] = 0;
+      uint32_t det[4] = {0, 0, 0, 0};
+
+      // XORs q into the row of its depth in column group g; the depth
+      auto update = [&](int g, uint64_t x, const uint4& q, bool live) {
+        const uint32_t f = live ? gs_low_capped(x, capbit) : capbit;
+        const uint32_t d = (uint32_t)__ffs((int)f) - 1u;
+        held[g] |= f & (0u - f);
+        const uint32_t a = ra + (g * kFewStride) * 16u + d * 512u;
+        uint4 t = lds128(a);
+        t.x ^= q.x; t.y ^= q.y; t.z ^= q.z; t.w ^= q.w;
+        sts128(a, t);
+        return d;
+      };
+      auto deep = [&](int g, uint64_t x, const uint4& q) {
+        const uint32_t dd = gs_depth_from_mixed(x, bkt);
+        if (lane + 32u * g < C && dd >= (uint32_t)kSlabDepth && dd < bkt)
+          xor_bucket_global(skv + (size_t)(lane + 32u * g) * bkt + dd, ((uint64_t)q.y << 32) | q.x,
+                            ((uint64_t)q.w << 32) | q.z);
+      };
+      for (uint32_t b = 0; b < cnt; b += 32) {
+        if (b) u = b + lane < cnt ? A.nbr[r0 + b + lane] : 0u;
+        const bool valid = b + lane < cnt;
+        const uint64_t id = gs_concat(v, u - vb);
+        const uint64_t E = gs_key_mix(id), cs = gs_hash_tail(E ^ csmix);
+        const uint4 q = make_uint4((uint32_t)id, (uint32_t)(id >> 32), (uint32_t)cs, (uint32_t)(cs >> 32));
+        if (valid) { det[0] ^= q.x; det[1] ^= q.y; det[2] ^= q.z; det[3] ^= q.w; }
+        sts128(qa + lane * 16u, q);
+        mixed[lane] = E;
+        __syncwarp();
+        const uint32_t c = min(32u, cnt - b);
+        for (uint32_t k = 0; k < c; k += 2) {
+          const bool two = k + 1 < c;
+          const uint64_t e0 = lds64(ma + k * 8u), e1 = lds64(ma + k * 8u + 8u);
+          const uint4 q0 = lds128(qa + k * 16u), q1 = lds128(qa + k * 16u + 16u);
+#pragma unroll
+          for (int g = 0; g < CG; g++) {
+            const uint32_t d0 = update(g, e0 ^ cm[g], q0, true);
+            const uint32_t d1 = update(g, e1 ^ cm[g], q1, two);
+            if (max(d0, d1) >= (uint32_t)kSlabDepth) {
+              if (d0 >= (uint32_t)kSlabDepth) deep(g, e0 ^ cm[g], q0);
+              if (two && d1 >= (uint32_t)kSlabDepth) deep(g, e1 ^ cm[g], q1);
+            }
+          }
+        }
+        __syncwarp();
+      }
+      // merge the held rows; the deterministic bucket's load goes with the first ones
+      uint4 td = make_uint4(0, 0, 0, 0);
+      if (lane == 0) td = ld_bucket(skv + (nb - 1));
+#pragma unroll
+      for (int g = 0; g < CG; g++) {
+        uint32_t h = lane + 32u * g < C ? held[g] & (capbit - 1u) : 0u;
+        GsBucket* col = skv + (size_t)(lane + 32u * g) * bkt;
+        while (h) {
+          uint4 t[4];
+          uint32_t d[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            d[k] = h ? __ffs(h) - 1 : 0xffffffffu;
+            h &= h - 1;
+            if (d[k] != 0xffffffffu) t[k] = ld_bucket(col + d[k]);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            if (d[k] == 0xffffffffu) continue;
+            const uint4 r = lds128(ra + (g * kFewStride + d[k] * 32) * 16u);
+            t[k].x ^= r.x; t[k].y ^= r.y; t[k].z ^= r.z; t[k].w ^= r.w;
+            st_bucket(col + d[k], t[k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) det[k] = __reduce_xor_sync(0xffffffffu, det[k]);
+      if (lane == 0) {
+        td.x ^= det[0]; td.y ^= det[1]; td.z ^= det[2]; td.w ^= det[3];
+        st_bucket(skv + (nb - 1), td);
+      }
+    }
+  }
+}
+
+// Sketch update of a small batch, without grouping it: a warp per edge record, a lane per bucket (column j,
+// or the deterministic bucket at j = C), both endpoints' buckets XORed in HBM.  The depths are hashed once
+// for both endpoints.
+template <int CG, bool TEN>
+__global__ void __launch_bounds__(256) k_ingest_direct(const uint2* __restrict__ pairs, uint32_t n, PairTag tag,
+                                                       const IngestArgs A) {
+  const uint32_t lane = lane_id();
+  uint32_t C = A.C, bkt = A.bkt, nb = A.nb, cur_t = 0xffffffffu;
+  uint64_t csmix = 0, cm[CG];
+  auto set_columns = [&](const uint64_t* cmt) {
+    csmix = cmt[C];
+#pragma unroll
+    for (int g = 0; g < CG; g++) cm[g] = lane + 32u * g < C ? cmt[lane + 32u * g] : 0ull;
+  };
+  if (!TEN) {
+    if (A.colmix) {
+      set_columns(A.colmix);
+    } else {   // no table: the constants from the seed
+      csmix = gs_seed_mix(A.seed);
+#pragma unroll
+      for (int g = 0; g < CG; g++) cm[g] = gs_seed_mix(A.seed + 5ull * (lane + 32u * g));
+    }
+  }
+  const uint32_t step = (gridDim.x * blockDim.x) >> 5;
+  uint32_t e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  uint2 next = e < n ? pairs[e] : make_uint2(0u, 0u);
+  for (; e < n; e += step) {
+    const uint2 p = next;
+    if (e + step < n) next = pairs[e + step];
+    int lo = 0, hi = -1;
+    if (!record_levels(tag, p.x, p.y, &lo, &hi, A.status)) continue;
+    uint32_t vb = 0;
+    GsBucket* sk = A.sk;
+    if (TEN) {
+      const uint32_t t = A.vtenant[p.x];
+      const GsIngTenant T = A.tenants[t];
+      if (t != cur_t) {
+        cur_t = t;
+        C = T.C;
+        bkt = T.bkt;
+        nb = T.nb;
+        set_columns(A.colmix + (size_t)t * kColStride);
+      }
+      vb = T.vbase;
+      sk += T.sk_off;
+    }
+    const uint32_t u = p.x - vb, v = p.y - vb;
+    const uint64_t id = gs_concat(u, v), E = gs_key_mix(id), cs = gs_hash_tail(E ^ csmix);
+    uint32_t at[CG];
+#pragma unroll
+    for (int g = 0; g < CG; g++) {
+      const uint32_t j = lane + 32u * g;
+      const uint32_t d = gs_depth_from_mixed(E ^ cm[g], bkt);
+      at[g] = j < C ? (d < bkt ? j * bkt + d : 0xffffffffu) : j == C ? nb - 1 : 0xffffffffu;
+    }
+    for (int l = lo; l <= hi; l++) {
+      GsBucket* const lvl = sk + (size_t)l * A.V * nb;
+#pragma unroll
+      for (int g = 0; g < CG; g++) {
+        if (at[g] == 0xffffffffu) continue;
+        xor_bucket_global(lvl + (size_t)u * nb + at[g], id, cs);
+        xor_bucket_global(lvl + (size_t)v * nb + at[g], id, cs);
+      }
+    }
+  }
+}
+
 size_t ingest_smem_bytes(int cg, int r, int warps) {
   return (size_t)warps * (size_t)(cg * (kSlabDepth - r) * kSlabPitch + 32) * sizeof(uint4);
 }
 
-template <int CG, int R, bool SMALL, bool TEN>
-gs_status launch_ingest(gs_graph* g, uint32_t nv, cudaStream_t s) {
+// What every kernel of an update reads: the records grouped by vertex, and the graph's (or the tenants')
+// sketches.
+IngestArgs ingest_args(const gs_graph* g, uint32_t nv) {
   IngestArgs A;
-  A.off = g->d_off; A.choff = g->d_choff; A.nbr = g->d_nbr; A.sk = g->d_sk; A.colmix = g->d_colmix;
-  A.status = g->d_status; A.nv = nv; A.V = g->V; A.C = g->geom.num_columns;
+  A.off = g->d_off; A.end = g->d_cnt; A.nbr = g->d_nbr; A.sk = g->d_sk; A.colmix = g->d_colmix;
+  A.status = g->d_status; A.few = g->d_few; A.work = g->d_work;
+  A.nv = nv; A.V = g->V; A.C = g->geom.num_columns;
   A.bkt = g->geom.bkt_per_col; A.nb = g->geom.num_buckets; A.chunk = g->tune.chunk;
+  A.vtenant = g->d_vtenant;
+  A.tenants = g->d_ten;
   A.warp_words = 0;
-  A.next_chunk = g->d_status + 14;
-  A.owner = g->d_owner;
-  A.owner_cap = (uint32_t)g->owner_cap;
+  A.seed = g->seed;
+  return A;
+}
+
+template <int CG, int R, bool SMALL, bool TEN>
+gs_status launch_ingest(gs_graph* g, const IngestArgs& A, cudaStream_t s) {
   const int warps = (int)g->tune.warps_per_block;
   const size_t smem = ingest_smem_bytes(CG, R, warps);
   // the opt-in shared-memory limit is a per-device function attribute; the persistent grid fills
@@ -1240,8 +1539,6 @@ gs_status launch_ingest(gs_graph* g, uint32_t nv, cudaStream_t s) {
     cc.warps = warps;
     cc.blocks = nb > 0 ? nb : 1;
   }
-  A.vtenant = TEN ? g->d_vtenant : nullptr;
-  A.tenants = TEN ? g->d_ten : nullptr;
   k_ingest<CG, R, SMALL, TEN><<<g->num_sms * cc.blocks, warps * 32, smem, s>>>(A);
   GS_CUDA_TRY(cudaGetLastError());
   return GS_OK;
@@ -1257,17 +1554,8 @@ uint32_t packed_warp_words(const gs_graph* g) {
 }
 
 template <bool TEN>
-gs_status launch_ingest_packed(gs_graph* g, uint32_t nv, cudaStream_t s) {
-  IngestArgs A;
-  A.off = g->d_off; A.choff = g->d_choff; A.nbr = g->d_nbr; A.sk = g->d_sk; A.colmix = g->d_colmix;
-  A.status = g->d_status; A.nv = nv; A.V = g->V; A.C = g->geom.num_columns;
-  A.bkt = g->geom.bkt_per_col; A.nb = g->geom.num_buckets; A.chunk = g->tune.chunk;
-  A.vtenant = TEN ? g->d_vtenant : nullptr;
-  A.tenants = TEN ? g->d_ten : nullptr;
+gs_status launch_ingest_packed(gs_graph* g, IngestArgs A, cudaStream_t s) {
   A.warp_words = packed_warp_words(g);
-  A.next_chunk = g->d_status + 14;
-  A.owner = g->d_owner;
-  A.owner_cap = (uint32_t)g->owner_cap;
   const int warps = std::min(kPackMaxThreads / 32, (int)g->tune.warps_per_block);
   const size_t smem = (size_t)warps * A.warp_words * sizeof(uint4);
   struct Cache { size_t smem = 0; int warps = 0; int blocks = 0; };
@@ -1286,21 +1574,52 @@ gs_status launch_ingest_packed(gs_graph* g, uint32_t nv, cudaStream_t s) {
   return GS_OK;
 }
 
+template <int CG, bool TEN>
+gs_status launch_ingest_few(const IngestArgs& A, int num_sms, cudaStream_t s) {
+  constexpr int warps = few_threads(CG) / 32;
+  const unsigned grid = std::min<uint32_t>((A.nv + warps - 1) / warps, (uint32_t)num_sms * 4);
+  constexpr size_t smem = warps * few_warp_words(CG) * sizeof(uint4);
+  static thread_local bool opted[64] = {};   // per host thread, device and instantiation
+  int dev = 0;
+  GS_CUDA_TRY(cudaGetDevice(&dev));
+  if (!opted[dev & 63]) {
+    GS_CUDA_TRY(cudaFuncSetAttribute(k_ingest_few<CG, TEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    opted[dev & 63] = true;
+  }
+  k_ingest_few<CG, TEN><<<grid, few_threads(CG), smem, s>>>(A);
+  GS_CUDA_TRY(cudaGetLastError());
+  return GS_OK;
+}
+
+template <bool TEN>
+gs_status launch_ingest_direct(const IngestArgs& A, uint32_t cols, const uint2* p, uint32_t n, const PairTag& t,
+                               int num_sms, cudaStream_t s) {
+  const unsigned grid = std::min<uint32_t>((n + 7) / 8, (uint32_t)num_sms * 8);
+  // a lane per bucket: the columns and the deterministic bucket
+  if (cols < 32) k_ingest_direct<1, TEN><<<grid, 256, 0, s>>>(p, n, t, A);
+  else if (cols < 64) k_ingest_direct<2, TEN><<<grid, 256, 0, s>>>(p, n, t, A);
+  else k_ingest_direct<3, TEN><<<grid, 256, 0, s>>>(p, n, t, A);
+  GS_CUDA_TRY(cudaGetLastError());
+  return GS_OK;
+}
+
 template <int CG, bool SMALL, bool TEN>
-gs_status launch_ingest_r(gs_graph* g, uint32_t nv, cudaStream_t s) {
+gs_status launch_ingest_r(gs_graph* g, const IngestArgs& A, cudaStream_t s) {
   switch (g->tune.reg_depth) {
     case 0:
-      if constexpr (CG == 1) return launch_ingest_packed<TEN>(g, nv, s);
-      else return launch_ingest<CG, 0, SMALL, TEN>(g, nv, s);
-    case 1: return launch_ingest<CG, 1, SMALL, TEN>(g, nv, s);
-    case 3: return launch_ingest<CG, 3, SMALL, TEN>(g, nv, s);
-    default: return launch_ingest<CG, 2, SMALL, TEN>(g, nv, s);
+      if constexpr (CG == 1) return launch_ingest_packed<TEN>(g, A, s);
+      else return launch_ingest<CG, 0, SMALL, TEN>(g, A, s);
+    case 1: return launch_ingest<CG, 1, SMALL, TEN>(g, A, s);
+    case 3: return launch_ingest<CG, 3, SMALL, TEN>(g, A, s);
+    default: return launch_ingest<CG, 2, SMALL, TEN>(g, A, s);
   }
 }
 
+// the vertices of few records, then the work chunks of the others
 template <int CG, bool TEN>
-gs_status launch_ingest_s(gs_graph* g, uint32_t nv, bool small, cudaStream_t s) {
-  return small ? launch_ingest_r<CG, true, TEN>(g, nv, s) : launch_ingest_r<CG, false, TEN>(g, nv, s);
+gs_status launch_update(gs_graph* g, const IngestArgs& A, bool small, cudaStream_t s) {
+  GS_TRY((launch_ingest_few<CG, TEN>(A, g->num_sms, s)));
+  return small ? launch_ingest_r<CG, true, TEN>(g, A, s) : launch_ingest_r<CG, false, TEN>(g, A, s);
 }
 
 template <bool COMPACT>
@@ -1343,13 +1662,13 @@ gs_status launch_vert_scatter_sorted(const uint2* part, const uint32_t* bkt, uin
 gs_status gs_ensure_ingest_scratch(gs_graph* g, uint64_t records) {
   const uint64_t nv = (uint64_t)g->num_levels * g->V;
   if (g->nv_cap < nv) {
-    cudaFree(g->d_cnt); cudaFree(g->d_off); cudaFree(g->d_choff); cudaFree(g->d_tile);
-    g->d_cnt = g->d_off = g->d_choff = g->d_tile = nullptr;
+    cudaFree(g->d_cnt); cudaFree(g->d_off); cudaFree(g->d_few); cudaFree(g->d_tile);
+    g->d_cnt = g->d_off = g->d_few = g->d_tile = nullptr;
     const uint64_t tiles = (nv + kScanTile - 1) / kScanTile + 1;
     GS_CUDA_TRY(cudaMalloc(&g->d_cnt, (nv + 1) * sizeof(uint32_t)));
     GS_CUDA_TRY(cudaMalloc(&g->d_off, (nv + 1) * sizeof(uint32_t)));
-    GS_CUDA_TRY(cudaMalloc(&g->d_choff, (nv + 1) * sizeof(uint32_t)));
-    GS_CUDA_TRY(cudaMalloc(&g->d_tile, 2 * tiles * sizeof(uint32_t)));
+    GS_CUDA_TRY(cudaMalloc(&g->d_few, nv * sizeof(uint32_t)));
+    GS_CUDA_TRY(cudaMalloc(&g->d_tile, tiles * sizeof(uint32_t)));
     g->nv_cap = nv;
   }
   if (g->nbr_cap < records) {
@@ -1416,18 +1735,20 @@ static gs_status ensure_chunkhist(gs_graph* g, uint64_t records, uint32_t** out)
   return GS_OK;
 }
 
-// The chunk-owner table: a chunk per vertex with records plus one per `chunk` records, the records
-// bounded by the neighbour scratch.  A smaller table is never wrong (the sketch update finds the
-// chunks past its end by search), so it is not grown while a stream is being captured.
-static gs_status ensure_owner_table(gs_graph* g) {
-  const uint64_t nv = (uint64_t)g->num_levels * g->V;
-  const uint64_t want = std::min<uint64_t>(nv + g->nbr_cap / std::max(1u, g->tune.chunk) + 1, 0xffffffffull);
-  if (g->owner_cap >= want || g->capturing) return GS_OK;
-  cudaFree(g->d_owner);
-  g->d_owner = nullptr;
-  g->owner_cap = 0;
-  GS_CUDA_TRY(cudaMalloc(&g->d_owner, want * sizeof(uint32_t)));
-  g->owner_cap = want;
+// work chunks of at most `records` records: each vertex cut into chunks has more than kFewRecords, and at
+// most one partial chunk
+static uint64_t work_chunks(uint64_t records, uint32_t chunk) {
+  return records / std::max(1u, chunk) + records / (kFewRecords + 1) + 1;
+}
+
+static gs_status ensure_work(gs_graph* g) {
+  const uint64_t want = std::min<uint64_t>(work_chunks(g->nbr_cap, g->tune.chunk), 0xffffffffull);
+  if (g->work_cap >= want) return GS_OK;
+  cudaFree(g->d_work);
+  g->d_work = nullptr;
+  g->work_cap = 0;
+  GS_CUDA_TRY(cudaMalloc(&g->d_work, want * sizeof(uint2)));
+  g->work_cap = want;
   return GS_OK;
 }
 
@@ -1438,35 +1759,125 @@ gs_status gs_reserve_ingest(gs_graph* g, uint64_t edges) {
   uint32_t* unused = nullptr;
   GS_TRY(ensure_blockhist(g, m, &unused));
   GS_TRY(ensure_chunkhist(g, 2 * m, &unused));
-  return ensure_owner_table(g);
+  return ensure_work(g);
 }
 
-static gs_status scan_counts(gs_graph* g, uint32_t nv, cudaStream_t s) {
+static WorkLists work_lists(const gs_graph* g) {
+  return WorkLists{g->d_few, g->d_work, (uint32_t)g->work_cap, g->tune.chunk, g->d_status};
+}
+
+// Scans the counts of directed batches of at most `records` records (0: unknown - then the count is read
+// back, because the neighbour scratch and the work list have to hold them).  *out: the bound or the count.
+static gs_status scan_counts(gs_graph* g, uint32_t nv, uint64_t records, uint64_t* out, cudaStream_t s) {
   const uint32_t tiles = (nv + kScanTile - 1) / kScanTile;
-  GS_TRY(ensure_owner_table(g));
-  k_scan_tiles<<<tiles, kScanThreads, 0, s>>>(g->d_cnt, nv, g->tune.chunk, g->d_off, g->d_choff, g->d_tile);
-  k_scan_top<<<1, kScanThreads, 0, s>>>(g->d_tile, tiles, g->d_off, g->d_choff, nv, g->d_status);
-  k_scan_add<<<tiles, kScanThreads, 0, s>>>(g->d_off, g->d_choff, g->d_cnt, g->d_tile, nv, g->tune.chunk, g->d_owner,
-                                            (uint32_t)g->owner_cap);
+  k_scan_tiles<<<tiles, kScanThreads, 0, s>>>(g->d_cnt, nv, g->d_off, g->d_tile);
+  k_scan_top<<<1, kScanThreads, 0, s>>>(g->d_tile, tiles, g->d_status);
   GS_CUDA_TRY(cudaGetLastError());
+  if (!records) {
+    GS_CUDA_TRY(cudaMemcpyAsync(g->h_status, g->d_status, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    GS_CUDA_TRY(cudaStreamSynchronize(s));
+    records = g->h_status[1];
+    if (records > g->nbr_cap) GS_TRY(gs_ensure_ingest_scratch(g, records));
+  }
+  GS_TRY(ensure_work(g));
+  k_scan_add<<<tiles, kScanThreads, 0, s>>>(g->d_off, g->d_cnt, g->d_tile, nv, work_lists(g));
+  GS_CUDA_TRY(cudaGetLastError());
+  *out = records;
   return GS_OK;
 }
 
-static gs_status ingest_chunks(gs_graph* g, uint32_t nv, cudaStream_t s) {
+// The sketch update of the grouped records.
+static gs_status ingest_grouped(gs_graph* g, uint32_t nv, cudaStream_t s) {
   const bool ten = g->d_ten != nullptr;
   const uint32_t cols = ten ? g->ten_max_cols : g->geom.num_columns;
   const bool small = (ten ? g->ten_min_bkt : g->geom.bkt_per_col) < (uint32_t)kSlabDepth;
-  if (cols <= 32) return ten ? launch_ingest_s<1, true>(g, nv, small, s) : launch_ingest_s<1, false>(g, nv, small, s);
-  if (cols <= 64) return ten ? launch_ingest_s<2, true>(g, nv, small, s) : launch_ingest_s<2, false>(g, nv, small, s);
+  const IngestArgs A = ingest_args(g, nv);
+  if (cols <= 32) return ten ? launch_update<1, true>(g, A, small, s) : launch_update<1, false>(g, A, small, s);
+  if (cols <= 64) return ten ? launch_update<2, true>(g, A, small, s) : launch_update<2, false>(g, A, small, s);
   gs_set_error("more than 64 sketch columns are not supported");
   return GS_ERR_BAD_ARG;
 }
+
+// Batches of at most this many edge records are not grouped by vertex.  Grouping costs about ten launches
+// and the smallest of its kernels' times (50 us) whatever the batch; a direct update costs four 64-bit
+// atomics per column.  us per batch of 2^13 / 2^16 / 2^18 records, grouped and direct: V = 8192 62 76 107 and
+// 9 31 111, V = 131072 71 150 246 and 8 113 460, V = 1000003 109 251 615 and 9 157 638.
+constexpr uint64_t kDirectEdges = 65536;
 
 static int grid_for(gs_graph* g, uint64_t work_items, int threads) {
   uint64_t want = (work_items + threads - 1) / threads;
   uint64_t cap = (uint64_t)g->num_sms * 8;
   if (want < 1) want = 1;
   return (int)std::min(want, cap);
+}
+
+// m edge records grouped by vertex, then the sketch update.
+static gs_status ingest_edges_grouped(gs_graph* g, const uint2* p, uint64_t m, const PairTag& t, bool tagged, uint32_t nv,
+                                      cudaStream_t s) {
+  const uint64_t bound = tagged ? std::max<uint64_t>(g->part_cap, 4 * m) : 2 * m;
+  GS_TRY(gs_ensure_ingest_scratch(g, tagged ? std::max<uint64_t>(g->nbr_cap, 4 * m) : 2 * m));
+  GS_TRY(ensure_partition_scratch(g, bound));
+  const uint32_t H = g->part_buckets, lb = g->part_lb;
+  const unsigned tiles = (unsigned)((m + kPartEdges - 1) / kPartEdges);
+  const int grid2 = g->num_sms * 4;
+  // per-block bucket counts handed from the count pass to the staged placement (untagged passes,
+  // while the table stays small: tiles x H words)
+  uint32_t* blockhist = nullptr;
+  if (!tagged) GS_TRY(ensure_blockhist(g, m, &blockhist));
+  {
+    GsProfScope ps(g, GS_PROF_BUCKET, s, 2);
+    GS_CUDA_TRY(cudaMemsetAsync(g->d_bkt, 0, (size_t)H * sizeof(uint32_t), s));
+    GS_CUDA_TRY(cudaMemsetAsync(g->d_cnt, 0, (size_t)(nv + 1) * sizeof(uint32_t), s));
+    k_part_count<<<tiles, kPartThreads, H * sizeof(uint32_t), s>>>(p, m, t, lb, H, g->d_bkt, g->d_status,
+                                                                   tagged ? nullptr : blockhist);
+    k_part_scan<<<1, kScanThreads, 0, s>>>(g->d_bkt, H, g->d_status);
+    GS_CUDA_TRY(cudaGetLastError());
+  }
+  if (tagged) {
+    // the record count depends on the tags: read it back and grow the scratch if needed
+    GS_CUDA_TRY(cudaMemcpyAsync(g->h_status, g->d_status, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    GS_CUDA_TRY(cudaStreamSynchronize(s));
+    const uint64_t recs = g->h_status[1];
+    if (recs > g->part_cap) GS_TRY(ensure_partition_scratch(g, recs + recs / 8));
+    if (recs > g->nbr_cap) GS_TRY(gs_ensure_ingest_scratch(g, recs + recs / 8));
+  }
+  {
+    GsProfScope ps(g, GS_PROF_BUCKET, s, 4);
+    // one-word records when a bucket-local key and a neighbour id fit together
+    const bool compact = !tagged && (uint64_t)g->V <= (1ull << (32u - lb));
+    if (tagged) {
+      k_part_scatter<<<tiles, kPartThreads, 2 * H * sizeof(uint32_t), s>>>(p, m, t, lb, H, g->d_bkt, g->d_part,
+                                                                           g->part_cap, g->d_status);
+    } else if (compact) {
+      GS_TRY(launch_part_scatter_staged<true>(p, m, t, lb, H, g->d_bkt, g->d_part, g->part_cap, g->d_status,
+                                              blockhist, s));
+    } else {
+      GS_TRY(launch_part_scatter_staged<false>(p, m, t, lb, H, g->d_bkt, g->d_part, g->part_cap, g->d_status,
+                                               blockhist, s));
+    }
+    const size_t vc_smem = (1u << lb) * sizeof(uint32_t), vs_smem = 2 * (1u << lb) * sizeof(uint32_t);
+    uint32_t* chunkhist = nullptr;
+    if (compact) {
+      GS_TRY(ensure_chunkhist(g, 2 * m, &chunkhist));
+      k_vert_count<true><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
+                                                             chunkhist);
+    } else {
+      k_vert_count<false><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
+                                                              nullptr);
+    }
+    GS_TRY(ensure_work(g));
+    k_vert_offsets<<<H, kPartThreads, 0, s>>>(g->d_bkt, H, lb, nv, g->d_off, g->d_cnt, work_lists(g));
+    if (compact) {
+      GS_TRY(launch_vert_scatter_sorted(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_nbr, g->nbr_cap, g->d_status,
+                                        chunkhist, g->num_sms * 3, s));
+    } else {
+      k_vert_scatter<false><<<grid2, kPartThreads, vs_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_nbr,
+                                                                 g->nbr_cap, g->d_status);
+    }
+    GS_CUDA_TRY(cudaGetLastError());
+  }
+  GsProfScope ps(g, GS_PROF_INGEST, s, 2);
+  return ingest_grouped(g, nv, s);
 }
 
 gs_status gs_ingest_device_pairs(gs_graph* g, const uint32_t* d_pairs, uint64_t n, int fixed_level,
@@ -1484,77 +1895,17 @@ gs_status gs_ingest_device_pairs(gs_graph* g, const uint32_t* d_pairs, uint64_t 
     const uint64_t m = std::min<uint64_t>(n - done, g->max_batch_edges);
     const uint2* p = reinterpret_cast<const uint2*>(d_pairs) + done;
     if (no_sketch) {
-      GS_TRY(gs_store_ingest(g, reinterpret_cast<const uint32_t*>(p), m, s));
-      GS_TRY(gs_store_maintain(g, s));
-      g->records_total += m;
-      done += m;
-      continue;
-    }
-    const uint64_t bound = tagged ? std::max<uint64_t>(g->part_cap, 4 * m) : 2 * m;
-    GS_TRY(gs_ensure_ingest_scratch(g, tagged ? std::max<uint64_t>(g->nbr_cap, 4 * m) : 2 * m));
-    GS_TRY(ensure_partition_scratch(g, bound));
-    const uint32_t H = g->part_buckets, lb = g->part_lb;
-    const unsigned tiles = (unsigned)((m + kPartEdges - 1) / kPartEdges);
-    const int grid2 = g->num_sms * 4;
-    // per-block bucket counts handed from the count pass to the staged placement (untagged passes,
-    // while the table stays small: tiles x H words)
-    uint32_t* blockhist = nullptr;
-    if (!tagged) GS_TRY(ensure_blockhist(g, m, &blockhist));
-    {
-      GsProfScope ps(g, GS_PROF_BUCKET, s, 2);
-      GS_CUDA_TRY(cudaMemsetAsync(g->d_bkt, 0, (size_t)H * sizeof(uint32_t), s));
-      GS_CUDA_TRY(cudaMemsetAsync(g->d_cnt, 0, (size_t)(nv + 1) * sizeof(uint32_t), s));
-      k_part_count<<<tiles, kPartThreads, H * sizeof(uint32_t), s>>>(p, m, t, lb, H, g->d_bkt, g->d_status,
-                                                                     tagged ? nullptr : blockhist);
-      k_part_scan<<<1, kScanThreads, 0, s>>>(g->d_bkt, H, g->d_status);
-      GS_CUDA_TRY(cudaGetLastError());
-    }
-    if (tagged) {
-      // the record count depends on the tags: read it back and grow the scratch if needed
-      GS_CUDA_TRY(cudaMemcpyAsync(g->h_status, g->d_status, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      GS_CUDA_TRY(cudaStreamSynchronize(s));
-      const uint64_t recs = g->h_status[1];
-      if (recs > g->part_cap) GS_TRY(ensure_partition_scratch(g, recs + recs / 8));
-      if (recs > g->nbr_cap) GS_TRY(gs_ensure_ingest_scratch(g, recs + recs / 8));
-    }
-    {
-      GsProfScope ps(g, GS_PROF_BUCKET, s, 6);
-      // one-word records when a bucket-local key and a neighbour id fit together
-      const bool compact = !tagged && (uint64_t)g->V <= (1ull << (32u - lb));
-      if (tagged) {
-        k_part_scatter<<<tiles, kPartThreads, 2 * H * sizeof(uint32_t), s>>>(p, m, t, lb, H, g->d_bkt, g->d_part,
-                                                                             g->part_cap, g->d_status);
-      } else if (compact) {
-        GS_TRY(launch_part_scatter_staged<true>(p, m, t, lb, H, g->d_bkt, g->d_part, g->part_cap, g->d_status,
-                                                blockhist, s));
-      } else {
-        GS_TRY(launch_part_scatter_staged<false>(p, m, t, lb, H, g->d_bkt, g->d_part, g->part_cap, g->d_status,
-                                                 blockhist, s));
-      }
-      const size_t vc_smem = (1u << lb) * sizeof(uint32_t), vs_smem = 2 * (1u << lb) * sizeof(uint32_t);
-      if (compact) {
-        uint32_t* chunkhist = nullptr;
-        GS_TRY(ensure_chunkhist(g, 2 * m, &chunkhist));
-        k_vert_count<true><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
-                                                               chunkhist);
-        GS_TRY(scan_counts(g, nv, s));
-        GS_TRY(launch_vert_scatter_sorted(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_nbr, g->nbr_cap, g->d_status,
-                                          chunkhist, g->num_sms * 3, s));
-      } else {
-        k_vert_count<false><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
-                                                                nullptr);
-        GS_TRY(scan_counts(g, nv, s));
-        k_vert_scatter<false><<<grid2, kPartThreads, vs_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_nbr,
-                                                                   g->nbr_cap, g->d_status);
-      }
-      GS_CUDA_TRY(cudaGetLastError());
-    }
-    {
+      // nothing to sketch
+    } else if (m <= kDirectEdges) {
       GsProfScope ps(g, GS_PROF_INGEST, s, 1);
-      GS_TRY(ingest_chunks(g, nv, s));
+      const IngestArgs A = ingest_args(g, nv);
+      if (g->d_ten) GS_TRY(launch_ingest_direct<true>(A, g->ten_max_cols, p, (uint32_t)m, t, g->num_sms, s));
+      else GS_TRY(launch_ingest_direct<false>(A, A.C, p, (uint32_t)m, t, g->num_sms, s));
+    } else {
+      GS_TRY(ingest_edges_grouped(g, p, m, t, tagged, nv, s));
     }
     if (fixed_level < 0) {
-      GS_TRY(gs_eager_ingest(g, reinterpret_cast<const uint32_t*>(p), m, s));
+      if (!no_sketch) GS_TRY(gs_eager_ingest(g, reinterpret_cast<const uint32_t*>(p), m, s));
       GS_TRY(gs_store_ingest(g, reinterpret_cast<const uint32_t*>(p), m, s));
       GS_TRY(gs_store_maintain(g, s));
     }
@@ -1573,20 +1924,12 @@ gs_status gs_ingest_device_batches(gs_graph* g, uint32_t level, const uint32_t* 
   const uint32_t nv = g->num_levels * g->V;
   GS_TRY(gs_ensure_ingest_scratch(g, std::max<uint64_t>(max_records, 1)));
   GS_CUDA_TRY(cudaMemsetAsync(g->d_cnt, 0, (size_t)(nv + 1) * sizeof(uint32_t), s));
+  uint64_t recs = 0;
   {
     GsProfScope ps(g, GS_PROF_BUCKET, s, 4);
     k_count_batches<<<grid_for(g, nbat, 256), 256, 0, s>>>(d_srcs, d_sizes, nbat, g->V, level, g->d_cnt, g->d_status);
     GS_CUDA_TRY(cudaGetLastError());
-    GS_TRY(scan_counts(g, nv, s));
-  }
-  // the record count sizes the neighbour scratch: a caller that knows a bound (the host path: the
-  // sum of the batch sizes) spares the read-back and its wait
-  uint64_t recs = max_records;
-  if (!max_records) {
-    GS_CUDA_TRY(cudaMemcpyAsync(g->h_status, g->d_status, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    GS_CUDA_TRY(cudaStreamSynchronize(s));
-    recs = g->h_status[1];
-    if (recs > g->nbr_cap) GS_TRY(gs_ensure_ingest_scratch(g, recs));
+    GS_TRY(scan_counts(g, nv, max_records, &recs, s));
   }
   {
     GsProfScope ps(g, GS_PROF_BUCKET, s, 1);
@@ -1595,68 +1938,18 @@ gs_status gs_ingest_device_batches(gs_graph* g, uint32_t level, const uint32_t* 
     GS_CUDA_TRY(cudaGetLastError());
   }
   g->records_total += recs;
-  GsProfScope ps(g, GS_PROF_INGEST, s, 1);
-  return ingest_chunks(g, nv, s);
+  GsProfScope ps(g, GS_PROF_INGEST, s, 2);
+  return ingest_grouped(g, nv, s);
 }
 
-// ---- ingest over caller-supplied scratch ----
+// ---- ingest into a caller's sketch buffer ----
 
-size_t gs_scratch_ingest_smem_bytes(const GsGeom& geom, uint32_t warps) {
-  return ingest_smem_bytes(geom.num_columns <= 32 ? 1 : 2, 1, (int)warps);
-}
-
-namespace {
-
-template <int CG, bool SMALL>
-gs_status launch_ingest_scratch(const GsScratchIngest& x, cudaStream_t s) {
-  IngestArgs A;
-  A.off = x.off; A.choff = x.choff; A.nbr = x.nbr; A.sk = x.sketches; A.colmix = x.colmix;
-  A.status = x.status; A.nv = x.geom.V; A.V = x.geom.V; A.C = x.geom.num_columns;
-  A.bkt = x.geom.bkt_per_col; A.nb = x.geom.num_buckets; A.chunk = x.chunk;
-  A.vtenant = nullptr;
-  A.tenants = nullptr;
-  A.warp_words = 0;
-  A.next_chunk = nullptr;
-  A.owner = nullptr;
-  A.owner_cap = 0;
-  const size_t smem = ingest_smem_bytes(CG, 1, (int)x.warps);
-  int nb = 0;
-  GS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ingest<CG, 1, SMALL, false>, (int)x.warps * 32, smem));
-  k_ingest<CG, 1, SMALL, false><<<x.num_sms * (nb > 0 ? nb : 1), x.warps * 32, smem, s>>>(A);
-  GS_CUDA_TRY(cudaGetLastError());
-  return GS_OK;
-}
-
-}  // namespace
-
-gs_status gs_ingest_pairs_on_scratch(const GsScratchIngest& x, cudaStream_t s) {
-  if (x.n == 0) return GS_OK;
-  const uint32_t nv = x.geom.V;
+gs_status gs_ingest_pairs_direct(const uint32_t* pairs, uint32_t n, const GsGeom& geom, GsBucket* sketches,
+                                 uint64_t seed, uint32_t* status, int num_sms, cudaStream_t s) {
+  IngestArgs A{};
+  A.sk = sketches; A.seed = seed; A.status = status;
+  A.nv = geom.V; A.V = geom.V; A.C = geom.num_columns; A.bkt = geom.bkt_per_col; A.nb = geom.num_buckets;
   PairTag t;
-  t.V = nv; t.num_levels = 1; t.L = 1; t.fixed_level = -1; t.cs_mix = 0;
-  const uint32_t H = x.part_buckets, lb = x.part_lb;
-  const unsigned tiles = (unsigned)((x.n + kPartEdges - 1) / kPartEdges);
-  const int grid2 = x.num_sms * 4;
-  // everything that must start at zero: error word and totals, bucket totals, vertex counts
-  GS_CUDA_TRY(cudaMemsetAsync(x.status, 0, 16 * sizeof(uint32_t), s));
-  GS_CUDA_TRY(cudaMemsetAsync(x.bkt, 0, (size_t)H * sizeof(uint32_t), s));
-  GS_CUDA_TRY(cudaMemsetAsync(x.cnt, 0, (size_t)(nv + 1) * sizeof(uint32_t), s));
-  const uint2* p = reinterpret_cast<const uint2*>(x.pairs);
-  k_part_count<<<tiles, kPartThreads, H * sizeof(uint32_t), s>>>(p, x.n, t, lb, H, x.bkt, x.status, nullptr);
-  k_part_scan<<<1, kScanThreads, 0, s>>>(x.bkt, H, x.status);
-  k_part_scatter<<<tiles, kPartThreads, 2 * H * sizeof(uint32_t), s>>>(p, x.n, t, lb, H, x.bkt, x.part,
-                                                                       x.records_cap, x.status);
-  k_vert_count<false><<<grid2, kPartThreads, (1u << lb) * sizeof(uint32_t), s>>>(x.part, x.bkt, H, lb, x.cnt, x.status,
-                                                                                nullptr);
-  const uint32_t stiles = (nv + kScanTile - 1) / kScanTile;
-  k_scan_tiles<<<stiles, kScanThreads, 0, s>>>(x.cnt, nv, x.chunk, x.off, x.choff, x.tile);
-  k_scan_top<<<1, kScanThreads, 0, s>>>(x.tile, stiles, x.off, x.choff, nv, x.status);
-  k_scan_add<<<stiles, kScanThreads, 0, s>>>(x.off, x.choff, x.cnt, x.tile, nv, x.chunk, nullptr, 0u);
-  k_vert_scatter<false><<<grid2, kPartThreads, 2 * (1u << lb) * sizeof(uint32_t), s>>>(x.part, x.bkt, H, lb, x.cnt, x.nbr,
-                                                                                x.records_cap, x.status);
-  GS_CUDA_TRY(cudaGetLastError());
-  const bool small = x.geom.bkt_per_col < (uint32_t)kSlabDepth;
-  if (x.geom.num_columns <= 32)
-    return small ? launch_ingest_scratch<1, true>(x, s) : launch_ingest_scratch<1, false>(x, s);
-  return small ? launch_ingest_scratch<2, true>(x, s) : launch_ingest_scratch<2, false>(x, s);
+  t.V = geom.V; t.num_levels = 1; t.L = 1; t.fixed_level = -1; t.cs_mix = 0;
+  return launch_ingest_direct<false>(A, A.C, reinterpret_cast<const uint2*>(pairs), n, t, num_sms, s);
 }

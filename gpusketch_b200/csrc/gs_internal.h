@@ -72,10 +72,9 @@ struct gs_graph {
 
   // ---- ingest scratch ----
   uint64_t nv_cap = 0;         // virtual vertices the per-vertex arrays hold (num_levels*V)
-  uint32_t* d_cnt = nullptr;   // [nv+1] records per virtual vertex, then cursors
-  uint32_t* d_off = nullptr;   // [nv+1] exclusive scan of d_cnt
-  uint32_t* d_choff = nullptr; // [nv+1] exclusive scan of d_nch
-  uint32_t* d_tile = nullptr;  // [2*tiles] per-tile sums for the scan
+  uint32_t* d_cnt = nullptr;   // [nv+1] records per virtual vertex, then cursors, then record ends
+  uint32_t* d_off = nullptr;   // [nv+1] first record of every virtual vertex
+  uint32_t* d_tile = nullptr;  // [tiles] per-tile sums for the scan
   uint32_t* d_nbr = nullptr;   // [nbr_cap] neighbour of each record, grouped by virtual vertex
   uint64_t nbr_cap = 0;
   uint2* d_part = nullptr;     // [part_cap] (key, neighbour) records partitioned by key >> part_lb
@@ -85,8 +84,9 @@ struct gs_graph {
   uint64_t blockhist_cap = 0;
   uint32_t* d_chunkhist = nullptr;  // [chunks][2^lb] vertex counts of every pass-2 chunk
   uint64_t chunkhist_cap = 0;
-  uint32_t* d_owner = nullptr;      // [work chunk] vertex owning it, for the chunks below owner_cap
-  uint64_t owner_cap = 0;
+  uint32_t* d_few = nullptr;        // [nv] vertices of few records
+  uint2* d_work = nullptr;          // [work_cap] work chunks {vertex, chunk of the vertex}
+  uint64_t work_cap = 0;
   uint32_t part_buckets = 0;   // H
   uint32_t part_lb = 9;        // low key bits resolved by the second pass
   uint32_t* d_pairs = nullptr; // staging for host-resident input pairs, 2 x [pairs_cap] u32 pairs
@@ -312,31 +312,7 @@ void gs_gen_rmat_host(uint32_t log2_v, double a, double b, double c, double dele
 
 GsTuning gs_tune_for(const GsGeom& geom, int num_sms);
 
-// Everything one ingest pass over single-level sketches needs, with every scratch buffer supplied by
-// the caller (the allocation-free entry point, gs_noalloc.cu).
-struct GsScratchIngest {
-  const uint32_t* pairs = nullptr;   // device, n interleaved pairs
-  uint64_t n = 0;
-  GsBucket* sketches = nullptr;      // device, [V][num_buckets]
-  GsGeom geom{};
-  const uint64_t* colmix = nullptr;  // device, num_columns + 1 constants
-  uint32_t* status = nullptr;        // device, 16 words
-  uint32_t* cnt = nullptr;           // device, V + 1
-  uint32_t* off = nullptr;           // device, V + 1
-  uint32_t* choff = nullptr;         // device, V + 1
-  uint32_t* tile = nullptr;          // device, 2 * (ceil(V / 4096) + 1)
-  uint32_t* bkt = nullptr;           // device, 4 * buckets + 2
-  uint2* part = nullptr;             // device, records_cap
-  uint32_t* nbr = nullptr;           // device, records_cap
-  uint64_t records_cap = 0;
-  uint32_t part_lb = 9;
-  uint32_t part_buckets = 0;
-  int num_sms = 148;
-  uint32_t chunk = 1024;
-  uint32_t warps = 4;
-};
-
-// Runs the bucketing passes and the sketch update on the buffers of `x` (no allocation).
-gs_status gs_ingest_pairs_on_scratch(const GsScratchIngest& x, cudaStream_t s);
-// Shared-memory bytes of one sketch-update block, for sizing checks by callers of the above.
-size_t gs_scratch_ingest_smem_bytes(const GsGeom& geom, uint32_t warps);
+// XORs n edge records into a caller's sketch buffer of one level, with no scratch; status[0] takes the error
+// bits (pointers device).
+gs_status gs_ingest_pairs_direct(const uint32_t* pairs, uint32_t n, const GsGeom& geom, GsBucket* sketches,
+                                 uint64_t seed, uint32_t* status, int num_sms, cudaStream_t s);

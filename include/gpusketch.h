@@ -319,10 +319,9 @@ gs_status gs_profile_read(gs_graph* g, gs_profile* out);
  * after start-up).  XORs n edge records (device pointer, interleaved uint32 pairs) into the caller's
  * device sketches of a connected-components graph, laid out [V][num_buckets] gs_bucket as
  * gs_geometry_for(num_vertices, sketches_factor) sizes them; the result equals gs_ingest_pairs on a
- * gs_graph with the same seed and factor.  Calls no allocator: all scratch is one static device array
- * of about 2.3 MB that every GPU loading the library holds until exit; each call looks up the array's
- * device address on the current device.  The array is shared by all calls and keeps the last call's
- * contents, so calls that overlap on the GPU race.  Rejects num_vertices outside
+ * gs_graph with the same seed and factor.  Calls no allocator and needs no scratch but one static device
+ * error word; each call looks up its device address on the current device.  The word is shared by all
+ * calls, so calls that overlap on the GPU can see one another's errors.  Rejects num_vertices outside
  * [2, GS_NOALLOC_MAX_VERTICES] and n > GS_NOALLOC_MAX_EDGES with GS_ERR_BAD_ARG before touching the
  * sketches.  Runs on `cuda_stream` (may be NULL) on the current device and is synchronous: it waits
  * for that stream to apply the update and check the device error word, so it must not be called while
