@@ -498,6 +498,7 @@ gs_status gs_engine_create(const gs_engine_config* cfg, gs_engine** out) {
   for (auto& tb : e->tabs) GS_CUDA_TRY(cudaEventCreateWithFlags(&tb.ev_free, cudaEventDisableTiming));
   g->d_vtenant = e->d_vtenant;
   g->d_ten = e->d_ing;
+  g->ten_max_vertices = e->max_tenant_vertices;
   refresh_bounds(e.get());
   // staging and bucketing scratch for a full batch are allocated now, so that serving allocates
   // nothing once it has started

@@ -109,10 +109,14 @@ __device__ uint2 block_exclusive_scan(uint2 x, uint2* total) {
 }
 
 // Work of the sketch update, reset before the first kernel that adds to it: status[2] = work chunks listed,
-// status[3] = vertices of few records listed, status[13] = next of those, status[14] = next work chunk.
+// status[3] = vertices of few records listed, status[13] = next of those, status[14] = next work chunk;
+// status[20] = parity items listed, status[21] = next of those, status[22] = shared parity bitmaps in use.
 __device__ __forceinline__ void reset_work(uint32_t* status) {
   status[2] = 0;
   status[3] = 0;
+  status[20] = 0;
+  status[21] = 0;
+  status[22] = 0;
   status[13] = 0;
   status[14] = 0;
 }
@@ -132,13 +136,44 @@ constexpr int kVertUnroll = 8;        // records a pass-2 thread loads before it
 constexpr uint64_t kMaxBlockHistWords = 1ull << 24;  // per-block bucket counts kept between pass-1 kernels (64 MB)
 constexpr uint64_t kMaxChunkHistWords = 1ull << 25;  // per-chunk vertex counts kept between pass-2 kernels (128 MB)
 
+// ---- does the batch toggle edges more than once? ----
+//
+// Two toggles of an edge cancel, so a vertex's records need only be sketched where a neighbour occurs an odd
+// number of times (k_parity).  Whether that is worth a pass over the records is estimated from a sample of the
+// batch's EDGES: those whose hash falls into one of 2^shift classes (about kSampleEdges of them, every
+// occurrence of a sampled edge) toggle a bit of a kSampleBits bitmap, and the bits set at the end count the
+// sampled edges that survive.
+constexpr uint32_t kSampleBits = 1u << 20, kSampleWords = kSampleBits / 32;
+constexpr uint64_t kSampleEdges = 65536;
+
+struct Sample {
+  uint32_t* bits;      // [kSampleWords], zero at the start of a pass
+  uint32_t* counts;    // [0] records of sampled edges [1] bits set (zero at the start of a pass)
+  uint32_t mask;       // 2^shift - 1
+};
+
+__device__ __forceinline__ uint32_t edge_hash(uint32_t u, uint32_t v) {
+  uint32_t h = min(u, v) * 0x9E3779B1u + max(u, v) * 0x85EBCA77u;
+  h ^= h >> 15;
+  return h * 0x2C1B3C6Du;
+}
+
+// Whether at least a tenth of the sampled records cancels.  m distinct edges in B bits leave
+// B (1 - exp(-2m/B)) / 2 bits set, expanded here to second order in m/B.
+__device__ __forceinline__ bool toggles_cancel(const uint32_t* counts) {
+  const float m = (float)counts[0], x = m / (float)kSampleBits;
+  return m >= 1024.0f && (float)counts[1] < 0.9f * m * (1.0f - x + 0.6667f * x * x);
+}
+
 // blockhist (may be null): the block's own histogram is also stored at [blockIdx.x * H], so that the
-// staged placement of the same block need not count its edges again
+// staged placement of the same block need not count its edges again.  sample.bits null: no sample.
 __global__ void __launch_bounds__(kPartThreads) k_part_count(const uint2* __restrict__ pairs, uint64_t n, PairTag t,
                                                              uint32_t lb, uint32_t H, uint32_t* __restrict__ tot,
                                                              uint32_t* __restrict__ status,
-                                                             uint32_t* __restrict__ blockhist) {
+                                                             uint32_t* __restrict__ blockhist, const Sample sample) {
   extern __shared__ uint32_t hist[];
+  __shared__ uint32_t s_sampled;
+  if (threadIdx.x == 0) s_sampled = 0;
   for (uint32_t i = threadIdx.x; i < H; i += blockDim.x) hist[i] = 0;
   __syncthreads();
   const uint64_t e0 = (uint64_t)blockIdx.x * kPartEdges;
@@ -157,6 +192,13 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(const uint2* __rest
       const uint2 p = ps[j];
       int lo = 0, hi = -1;
       if (!record_levels(t, p.x, p.y, &lo, &hi, status)) continue;
+      if (sample.bits) {
+        const uint32_t h = edge_hash(p.x, p.y);
+        if ((h & sample.mask) == 0) {
+          atomicXor(&sample.bits[h >> 17], 1u << ((h >> 12) & 31u));
+          atomicAdd(&s_sampled, 1u);
+        }
+      }
       for (int g = lo; g <= hi; g++) {
         atomicAdd(&hist[((uint32_t)g * t.V + p.x) >> lb], 1u);
         atomicAdd(&hist[((uint32_t)g * t.V + p.y) >> lb], 1u);
@@ -164,6 +206,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_count(const uint2* __rest
     }
   }
   __syncthreads();
+  if (threadIdx.x == 0 && s_sampled) atomicAdd(&sample.counts[0], s_sampled);
   for (uint32_t d = threadIdx.x; d < H; d += blockDim.x) {
     if (hist[d]) atomicAdd(&tot[d], hist[d]);
     if (blockhist) blockhist[(size_t)blockIdx.x * H + d] = hist[d];
@@ -375,9 +418,16 @@ template <bool COMPACT>
 __global__ void __launch_bounds__(kPartThreads) k_vert_count(const uint2* __restrict__ part, const uint32_t* __restrict__ bkt,
                                                              uint32_t H, uint32_t lb, uint32_t* __restrict__ cnt,
                                                              const uint32_t* __restrict__ status,
-                                                             uint32_t* __restrict__ chunkhist) {
+                                                             uint32_t* __restrict__ chunkhist, const Sample sample) {
   extern __shared__ uint32_t hist[];
   __shared__ uint32_t s_d;
+  if (sample.bits) {
+    uint32_t set = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kSampleWords; i += gridDim.x * blockDim.x)
+      set += __popc(sample.bits[i]);
+    set = __reduce_add_sync(0xffffffffu, set);
+    if (lane_id() == 0 && set) atomicAdd(&sample.counts[1], set);
+  }
   const uint32_t* off = bkt + H;
   const uint32_t* choff = bkt + 3 * H + 1;
   const uint32_t nk = 1u << lb, mask = nk - 1;
@@ -605,24 +655,29 @@ __global__ void k_scatter_batches(const uint32_t* __restrict__ srcs, const uint6
 }
 
 // The lists that the sketch update works from.  A vertex of at most kFewRecords goes to `few`; any other is
-// cut into work chunks of at most `chunk` records, work[i] = {vertex, chunk of the vertex}.  Both are in any
-// order.
+// cut into work chunks of at most `chunk` records, work[i] = {vertex, chunk of the vertex}.  When toggles
+// cancel, a vertex of more than kParityMin records is first cut into parity items of at most kParityRecords,
+// and listed by k_parity with the records that are left.  All lists are in any order.
 constexpr uint32_t kFewRecords = 64;
+constexpr uint32_t kParityMin = 1024, kParityRecords = 65536;
 
 struct WorkLists {
   uint32_t* few;
   uint2* work;
   uint32_t work_cap, chunk;
   uint32_t* status;
+  uint4* parity;           // {vertex, item of the vertex, items, shared bitmap}; null: no parity pass
+  uint32_t parity_cap, shared_cap;
 };
 
 // Lists the block's vertices (one a thread; n = 0: nothing to list), with one reservation per block.
-__device__ __forceinline__ void list_vertices(const WorkLists& L, uint32_t v, uint32_t n) {
+__device__ __forceinline__ void list_vertices(const WorkLists& L, uint32_t v, uint32_t n, bool parity) {
   __shared__ uint2 s_at;
   const bool few = n > 0 && n <= kFewRecords;
-  const uint32_t nch = n > kFewRecords ? (n + L.chunk - 1) / L.chunk : 0u;
+  parity = parity && n > kParityMin;
+  const uint32_t nch = few ? 0u : (n + L.chunk - 1) / L.chunk;
   uint2 tot;
-  uint2 at = block_exclusive_scan(make_uint2(few ? 1u : 0u, nch), &tot);
+  uint2 at = block_exclusive_scan(make_uint2(few ? 1u : 0u, parity ? 0u : nch), &tot);
   if (threadIdx.x == 0) {
     s_at.x = tot.x ? atomicAdd(&L.status[3], tot.x) : 0u;
     s_at.y = tot.y ? atomicAdd(&L.status[2], tot.y) : 0u;
@@ -630,20 +685,27 @@ __device__ __forceinline__ void list_vertices(const WorkLists& L, uint32_t v, ui
   __syncthreads();
   at = add2(at, s_at);
   if (few) L.few[at.x] = v;
-  // a vertex of a few chunks writes its own entries; the warp writes a hub vertex's together
-  constexpr uint32_t kOwn = 8;
-  if (nch <= kOwn) {
-    for (uint32_t i = 0; i < nch; i++)
-      if (at.y + i < L.work_cap) L.work[at.y + i] = make_uint2(v, i);
+  const auto put = [&](uint32_t i, uint32_t vertex, uint32_t part) {
+    if (i < L.work_cap) L.work[i] = make_uint2(vertex, part);
+    else atomicOr(L.status, (uint32_t)GS_DEV_ERR_CAPACITY);
+  };
+  if (parity) {
+    // vertices of several items share a bitmap in memory
+    const uint32_t items = (n + kParityRecords - 1) / kParityRecords;
+    const uint32_t shared = items > 1 ? atomicAdd(&L.status[22], 1u) : 0u, i0 = atomicAdd(&L.status[20], items);
+    for (uint32_t i = 0; i < items; i++)
+      if (i0 + i < L.parity_cap && shared < L.shared_cap) L.parity[i0 + i] = make_uint4(v, i, items, shared);
       else atomicOr(L.status, (uint32_t)GS_DEV_ERR_CAPACITY);
   }
-  for (uint32_t m = __ballot_sync(0xffffffffu, nch > kOwn); m; m &= m - 1) {
+  // a vertex of a few chunks writes its own entries; the warp writes a hub vertex's together
+  constexpr uint32_t kOwn = 8;
+  if (!parity && nch <= kOwn)
+    for (uint32_t i = 0; i < nch; i++) put(at.y + i, v, i);
+  for (uint32_t m = __ballot_sync(0xffffffffu, !parity && nch > kOwn); m; m &= m - 1) {
     const uint32_t src = __ffs(m) - 1;
     const uint32_t w0 = __shfl_sync(0xffffffffu, at.y, src), wn = __shfl_sync(0xffffffffu, nch, src);
     const uint32_t hv = __shfl_sync(0xffffffffu, v, src);
-    for (uint32_t i = lane_id(); i < wn; i += 32)
-      if (w0 + i < L.work_cap) L.work[w0 + i] = make_uint2(hv, i);
-      else atomicOr(L.status, (uint32_t)GS_DEV_ERR_CAPACITY);
+    for (uint32_t i = lane_id(); i < wn; i += 32) put(w0 + i, hv, i);
   }
   __syncthreads();   // s_at and the scan's words may be used again
 }
@@ -703,7 +765,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t* __restrict_
       n = cursor[i];
       cursor[i] = off[i] = off[i] + a;
     }
-    list_vertices(L, (uint32_t)i, n);
+    list_vertices(L, (uint32_t)i, n, false);
   }
 }
 
@@ -711,7 +773,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t* __restrict_
 // its vertices' counts, which become the cursors of the placement.  The vertices are listed for the update.
 __global__ void __launch_bounds__(kPartThreads) k_vert_offsets(const uint32_t* __restrict__ bkt, uint32_t H, uint32_t lb,
                                                                uint32_t nv, uint32_t* __restrict__ off,
-                                                               uint32_t* __restrict__ cursor, const WorkLists L) {
+                                                               uint32_t* __restrict__ cursor, const WorkLists L,
+                                                               const Sample sample) {
+  const bool parity = sample.bits && toggles_cancel(sample.counts);
   const uint32_t d = blockIdx.x;
   const uint64_t v0 = (uint64_t)d << lb, v1 = min((uint64_t)nv, v0 + ((uint64_t)1 << lb));
   uint32_t run = bkt[H + d];
@@ -725,7 +789,165 @@ __global__ void __launch_bounds__(kPartThreads) k_vert_offsets(const uint32_t* _
       cursor[v] = at;
     }
     run += tot.x;
-    list_vertices(L, (uint32_t)v, n);
+    list_vertices(L, (uint32_t)v, n, parity);
+  }
+}
+
+// ---- parity: toggles that cancel ----
+//
+// A block takes an item (up to kParityRecords records of one vertex) and toggles a bit per record in a
+// shared-memory bitmap over the neighbour ids.  Small items then walk their records again: the first of the
+// records whose bit is set keeps its place (and clears the bit), so the records that are left move to the
+// front of the vertex's run and the bitmap is clean again.  Large items (more records than the bitmap has
+// words, twice over) list the bitmap's set bits instead.  The items of a vertex that has several XOR their
+// bitmaps into one in memory, and the last of them lists that one.
+// Bound by the shared-memory atomics and one read of the records.  R-MAT of 2^27 edge records, V = 2^17:
+// @PARITY@
+constexpr uint32_t kParityThreads = 256;
+constexpr uint32_t kParityTile = kParityThreads * 8;
+constexpr uint32_t kParityMaxVertices = 1u << 18;   // 32 KB of bitmap: six blocks per SM
+
+// words of a bitmap over V ids: rows of 32 words
+GS_HD uint32_t parity_words(uint32_t V) { return (V + 1023u) / 1024u * 32u; }
+
+// Place of id u: row u >> 10, bit (u >> 5) & 31, and a word of the row that mixes every bit group of u:
+// skewed streams name ids whose bits are all zero most often, and would crowd into one bank.
+__device__ __forceinline__ uint32_t parity_fold(uint32_t rest) { return (rest ^ (rest >> 5) ^ (rest >> 10)) & 31u; }
+__device__ __forceinline__ uint2 parity_place(uint32_t u) {
+  const uint32_t rest = u >> 5;
+  return make_uint2((rest >> 5) * 32u + ((u & 31u) ^ parity_fold(rest)), 1u << (rest & 31u));
+}
+__device__ __forceinline__ uint32_t parity_id(uint32_t word, uint32_t bit) {
+  const uint32_t rest = (word >> 5) * 32u + bit;
+  return rest * 32u + ((word & 31u) ^ parity_fold(rest));
+}
+
+struct ParityArgs {
+  const uint32_t* off;
+  uint32_t* end;
+  uint32_t* nbr;
+  WorkLists lists;
+  uint32_t words;                // of one bitmap
+  uint32_t* shared;              // [shared_cap][words + 1] bitmaps in memory and their finished items, zero
+                                 // between passes
+  const uint32_t* vtenant;
+  const GsIngTenant* tenants;    // null: ids start at 0
+};
+
+__global__ void __launch_bounds__(kParityThreads) k_parity(const ParityArgs A) {
+  extern __shared__ uint32_t bm[];
+  __shared__ uint32_t s_item, s_kept, s_last, s_at;
+  const uint32_t lane = lane_id();
+  const uint32_t total = A.lists.status[20];
+  for (uint32_t i = threadIdx.x; i < A.words; i += kParityThreads) bm[i] = 0;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_item = atomicAdd(&A.lists.status[21], 1u);
+      s_kept = 0;
+    }
+    __syncthreads();
+    if (s_item >= total) return;
+    const uint4 it = A.lists.parity[s_item];
+    const uint32_t v = it.x, first = A.off[v], last = A.end[v];
+    const uint32_t r0 = first + it.y * kParityRecords, r1 = min(last, r0 + kParityRecords), n = r1 - r0;
+    const uint32_t vb = A.tenants ? A.tenants[A.vtenant[v]].vbase : 0u;
+    uint32_t u[8];
+    for (uint32_t b = r0; b < r1; b += kParityTile) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const uint32_t i = b + k * kParityThreads + threadIdx.x;
+        u[k] = i < r1 ? A.nbr[i] : 0xffffffffu;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (u[k] != 0xffffffffu) {
+          const uint2 w = parity_place(u[k] - vb);
+          atomicXor(&bm[w.x], w.y);
+        }
+    }
+    __syncthreads();
+    bool list = true;   // this block lists what is left of the vertex
+    if (it.z == 1 && n <= 2 * A.words) {
+      // walk the records again; the last tile (the only one of a short item) is still in registers
+      for (uint32_t b = r0; b < r1; b += kParityTile) {
+        if (n > kParityTile) {
+#pragma unroll
+          for (int k = 0; k < 8; k++) {
+            const uint32_t i = b + k * kParityThreads + threadIdx.x;
+            u[k] = i < r1 ? A.nbr[i] : 0xffffffffu;
+          }
+          __syncthreads();   // the tile is read before its places (or earlier ones) are written
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          bool keep = false;
+          if (u[k] != 0xffffffffu) {
+            const uint2 w = parity_place(u[k] - vb);
+            keep = atomicAnd(&bm[w.x], ~w.y) & w.y;
+          }
+          const uint32_t m = __ballot_sync(0xffffffffu, keep);
+          if (!m) continue;
+          uint32_t at = 0;
+          if (lane == 0) at = atomicAdd(&s_kept, (uint32_t)__popc(m));
+          at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+          if (keep) A.nbr[first + at] = u[k];
+        }
+        __syncthreads();
+      }
+    } else {
+      uint32_t* src = bm;
+      if (it.z > 1) {
+        uint32_t* const g = A.shared + (size_t)it.w * (A.words + 1);
+        for (uint32_t i = threadIdx.x; i < A.words; i += kParityThreads) {
+          if (bm[i]) atomicXor(&g[i], bm[i]);
+          bm[i] = 0;
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(&g[A.words], 1u) == it.z - 1;
+        __syncthreads();
+        list = s_last;
+        src = g;
+      }
+      if (list) {
+        __threadfence();
+        for (uint32_t b = 0; b < A.words; b += kParityThreads) {
+          const uint32_t i = b + threadIdx.x;
+          uint32_t x = 0;
+          if (i < A.words) {
+            x = it.z > 1 ? __ldcg(&src[i]) : src[i];
+            if (x) src[i] = 0;
+          }
+          const uint32_t c = __popc(x);
+          uint32_t inc = c;
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (uint32_t)o) inc += y;
+          }
+          uint32_t at = 0;
+          if (lane == 31 && inc) at = atomicAdd(&s_kept, inc);
+          at = first + __shfl_sync(0xffffffffu, at, 31) + inc - c;
+          for (; x; x &= x - 1) A.nbr[at++] = vb + parity_id(i, __ffs(x) - 1);
+        }
+        if (it.z > 1 && threadIdx.x == 0) src[A.words] = 0;
+        __syncthreads();
+      }
+    }
+    if (list) {
+      const uint32_t kept = s_kept;
+      const uint32_t nch = kept > kFewRecords ? (kept + A.lists.chunk - 1) / A.lists.chunk : 0u;
+      if (threadIdx.x == 0) {
+        A.end[v] = first + kept;
+        if (nch) s_at = atomicAdd(&A.lists.status[2], nch);
+        else if (kept) A.lists.few[atomicAdd(&A.lists.status[3], 1u)] = v;
+      }
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < nch; i += kParityThreads) {
+        if (s_at + i < A.lists.work_cap) A.lists.work[s_at + i] = make_uint2(v, i);
+        else atomicOr(A.lists.status, (uint32_t)GS_DEV_ERR_CAPACITY);
+      }
+    }
   }
 }
 
@@ -1689,7 +1911,9 @@ static gs_status ensure_partition_scratch(gs_graph* g, uint64_t records) {
     while ((nv >> lb) >= (uint64_t)kMaxBuckets) lb++;
     g->part_lb = lb;
     g->part_buckets = (uint32_t)((nv + (1ull << lb) - 1) >> lb);
-    GS_CUDA_TRY(cudaMalloc(&g->d_bkt, (4 * (size_t)g->part_buckets + 2) * sizeof(uint32_t)));
+    // the sample's bitmap and counts come first: one memset clears them and the bucket totals
+    GS_CUDA_TRY(cudaMalloc(&g->d_sample, (kSampleWords + 4 + 4 * (size_t)g->part_buckets + 2) * sizeof(uint32_t)));
+    g->d_bkt = g->d_sample + kSampleWords + 4;
   }
   if (g->part_cap < records) {
     cudaFree(g->d_part);
@@ -1735,22 +1959,50 @@ static gs_status ensure_chunkhist(gs_graph* g, uint64_t records, uint32_t** out)
   return GS_OK;
 }
 
-// work chunks of at most `records` records: each vertex cut into chunks has more than kFewRecords, and at
-// most one partial chunk
-static uint64_t work_chunks(uint64_t records, uint32_t chunk) {
-  return records / std::max(1u, chunk) + records / (kFewRecords + 1) + 1;
+// entries of a list that cuts vertices of more than `least` records into pieces of `per`: at most one partial
+// piece per vertex
+static uint64_t list_entries(const gs_graph* g, uint64_t records, uint32_t per, uint32_t least) {
+  const uint64_t nv = (uint64_t)g->num_levels * g->V;
+  return std::min<uint64_t>(records / std::max(1u, per) + std::min(records / (least + 1), nv) + 1, 0xffffffffull);
 }
 
-static gs_status ensure_work(gs_graph* g) {
-  const uint64_t want = std::min<uint64_t>(work_chunks(g->nbr_cap, g->tune.chunk), 0xffffffffull);
-  if (g->work_cap >= want) return GS_OK;
-  cudaFree(g->d_work);
-  g->d_work = nullptr;
-  g->work_cap = 0;
-  GS_CUDA_TRY(cudaMalloc(&g->d_work, want * sizeof(uint2)));
-  g->work_cap = want;
+// ids a vertex's neighbours can have, counted from its graph's first
+static uint32_t neighbour_ids(const gs_graph* g) { return g->d_ten ? g->ten_max_vertices : g->V; }
+
+// The update's work list, and with `parity` what the parity pass needs.
+static gs_status ensure_work(gs_graph* g, bool parity, cudaStream_t s) {
+  const uint64_t want = list_entries(g, g->nbr_cap, g->tune.chunk, kFewRecords);
+  if (g->work_cap < want) {
+    cudaFree(g->d_work);
+    g->d_work = nullptr;
+    g->work_cap = 0;
+    GS_CUDA_TRY(cudaMalloc(&g->d_work, want * sizeof(uint2)));
+    g->work_cap = want;
+  }
+  if (!parity) return GS_OK;
+  const uint64_t items = list_entries(g, g->nbr_cap, kParityRecords, kParityMin);
+  const uint64_t shared = g->nbr_cap / kParityRecords + 1, words = parity_words(neighbour_ids(g)) + 1;
+  if (g->parity_cap < items) {
+    cudaFree(g->d_parity);
+    g->d_parity = nullptr;
+    g->parity_cap = 0;
+    GS_CUDA_TRY(cudaMalloc(&g->d_parity, items * sizeof(uint4)));
+    g->parity_cap = items;
+  }
+  if (g->parity_shared_cap < shared) {
+    cudaFree(g->d_parity_shared);
+    g->d_parity_shared = nullptr;
+    g->parity_shared_cap = 0;
+    GS_CUDA_TRY(cudaMalloc(&g->d_parity_shared, shared * words * sizeof(uint32_t)));
+    GS_CUDA_TRY(cudaMemsetAsync(g->d_parity_shared, 0, shared * words * sizeof(uint32_t), s));
+    g->parity_shared_cap = shared;
+  }
   return GS_OK;
 }
+
+// The bitmaps of the parity pass have to fit next to one another on an SM; above, vertices with enough
+// records to repeat a neighbour are rare.
+static bool parity_possible(const gs_graph* g) { return neighbour_ids(g) <= kParityMaxVertices; }
 
 gs_status gs_reserve_ingest(gs_graph* g, uint64_t edges) {
   const uint64_t m = std::min<uint64_t>(edges, g->max_batch_edges);
@@ -1759,11 +2011,12 @@ gs_status gs_reserve_ingest(gs_graph* g, uint64_t edges) {
   uint32_t* unused = nullptr;
   GS_TRY(ensure_blockhist(g, m, &unused));
   GS_TRY(ensure_chunkhist(g, 2 * m, &unused));
-  return ensure_work(g);
+  return ensure_work(g, parity_possible(g), g->stream);
 }
 
 static WorkLists work_lists(const gs_graph* g) {
-  return WorkLists{g->d_few, g->d_work, (uint32_t)g->work_cap, g->tune.chunk, g->d_status};
+  return WorkLists{g->d_few, g->d_work, (uint32_t)g->work_cap, g->tune.chunk, g->d_status,
+                   g->d_parity, (uint32_t)g->parity_cap, (uint32_t)g->parity_shared_cap};
 }
 
 // Scans the counts of directed batches of at most `records` records (0: unknown - then the count is read
@@ -1779,10 +2032,26 @@ static gs_status scan_counts(gs_graph* g, uint32_t nv, uint64_t records, uint64_
     records = g->h_status[1];
     if (records > g->nbr_cap) GS_TRY(gs_ensure_ingest_scratch(g, records));
   }
-  GS_TRY(ensure_work(g));
+  GS_TRY(ensure_work(g, false, s));
   k_scan_add<<<tiles, kScanThreads, 0, s>>>(g->d_off, g->d_cnt, g->d_tile, nv, work_lists(g));
   GS_CUDA_TRY(cudaGetLastError());
   *out = records;
+  return GS_OK;
+}
+
+// Drops the records that cancel from the vertices listed for it (none unless the sample says so).
+static gs_status launch_parity(gs_graph* g, cudaStream_t s) {
+  ParityArgs A;
+  A.off = g->d_off; A.end = g->d_cnt; A.nbr = g->d_nbr;
+  A.lists = work_lists(g);
+  A.words = parity_words(neighbour_ids(g));
+  A.shared = g->d_parity_shared;
+  A.vtenant = g->d_vtenant;
+  A.tenants = g->d_ten;
+  const size_t smem = A.words * sizeof(uint32_t);
+  const int per_sm = (int)std::min<size_t>(8, (200u << 10) / smem);
+  k_parity<<<g->num_sms * per_sm, kParityThreads, smem, s>>>(A);
+  GS_CUDA_TRY(cudaGetLastError());
   return GS_OK;
 }
 
@@ -1824,12 +2093,18 @@ static gs_status ingest_edges_grouped(gs_graph* g, const uint2* p, uint64_t m, c
   // while the table stays small: tiles x H words)
   uint32_t* blockhist = nullptr;
   if (!tagged) GS_TRY(ensure_blockhist(g, m, &blockhist));
+  Sample sample{};
+  if (parity_possible(g)) {
+    sample.bits = g->d_sample;
+    sample.counts = g->d_sample + kSampleWords;
+    while ((m >> __builtin_popcount(sample.mask)) > kSampleEdges && sample.mask < 0xfffu) sample.mask = 2 * sample.mask + 1;
+  }
   {
     GsProfScope ps(g, GS_PROF_BUCKET, s, 2);
-    GS_CUDA_TRY(cudaMemsetAsync(g->d_bkt, 0, (size_t)H * sizeof(uint32_t), s));
+    GS_CUDA_TRY(cudaMemsetAsync(g->d_sample, 0, (kSampleWords + 4 + (size_t)H) * sizeof(uint32_t), s));
     GS_CUDA_TRY(cudaMemsetAsync(g->d_cnt, 0, (size_t)(nv + 1) * sizeof(uint32_t), s));
     k_part_count<<<tiles, kPartThreads, H * sizeof(uint32_t), s>>>(p, m, t, lb, H, g->d_bkt, g->d_status,
-                                                                   tagged ? nullptr : blockhist);
+                                                                   tagged ? nullptr : blockhist, sample);
     k_part_scan<<<1, kScanThreads, 0, s>>>(g->d_bkt, H, g->d_status);
     GS_CUDA_TRY(cudaGetLastError());
   }
@@ -1842,7 +2117,7 @@ static gs_status ingest_edges_grouped(gs_graph* g, const uint2* p, uint64_t m, c
     if (recs > g->nbr_cap) GS_TRY(gs_ensure_ingest_scratch(g, recs + recs / 8));
   }
   {
-    GsProfScope ps(g, GS_PROF_BUCKET, s, 4);
+    GsProfScope ps(g, GS_PROF_BUCKET, s, sample.bits ? 5 : 4);
     // one-word records when a bucket-local key and a neighbour id fit together
     const bool compact = !tagged && (uint64_t)g->V <= (1ull << (32u - lb));
     if (tagged) {
@@ -1860,13 +2135,13 @@ static gs_status ingest_edges_grouped(gs_graph* g, const uint2* p, uint64_t m, c
     if (compact) {
       GS_TRY(ensure_chunkhist(g, 2 * m, &chunkhist));
       k_vert_count<true><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
-                                                             chunkhist);
+                                                             chunkhist, sample);
     } else {
       k_vert_count<false><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
-                                                              nullptr);
+                                                              nullptr, sample);
     }
-    GS_TRY(ensure_work(g));
-    k_vert_offsets<<<H, kPartThreads, 0, s>>>(g->d_bkt, H, lb, nv, g->d_off, g->d_cnt, work_lists(g));
+    GS_TRY(ensure_work(g, parity_possible(g), s));
+    k_vert_offsets<<<H, kPartThreads, 0, s>>>(g->d_bkt, H, lb, nv, g->d_off, g->d_cnt, work_lists(g), sample);
     if (compact) {
       GS_TRY(launch_vert_scatter_sorted(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_nbr, g->nbr_cap, g->d_status,
                                         chunkhist, g->num_sms * 3, s));
@@ -1875,6 +2150,7 @@ static gs_status ingest_edges_grouped(gs_graph* g, const uint2* p, uint64_t m, c
                                                                  g->nbr_cap, g->d_status);
     }
     GS_CUDA_TRY(cudaGetLastError());
+    if (sample.bits) GS_TRY(launch_parity(g, s));
   }
   GsProfScope ps(g, GS_PROF_INGEST, s, 2);
   return ingest_grouped(g, nv, s);

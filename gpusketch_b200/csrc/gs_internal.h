@@ -69,6 +69,7 @@ struct gs_graph {
   const GsIngTenant* d_ten = nullptr;   // tenant geometry table; d_colmix then holds kColStride per tenant
   uint32_t ten_max_cols = 0;            // most columns of any live tenant
   uint32_t ten_min_bkt = 0;             // fewest buckets per column of any live tenant
+  uint32_t ten_max_vertices = 0;        // most vertices a tenant can have
 
   // ---- ingest scratch ----
   uint64_t nv_cap = 0;         // virtual vertices the per-vertex arrays hold (num_levels*V)
@@ -87,6 +88,11 @@ struct gs_graph {
   uint32_t* d_few = nullptr;        // [nv] vertices of few records
   uint2* d_work = nullptr;          // [work_cap] work chunks {vertex, chunk of the vertex}
   uint64_t work_cap = 0;
+  uint4* d_parity = nullptr;        // [parity_cap] parity items
+  uint64_t parity_cap = 0;
+  uint32_t* d_parity_shared = nullptr;  // bitmaps of vertices of several items, zero between passes
+  uint64_t parity_shared_cap = 0;
+  uint32_t* d_sample = nullptr;     // bitmap and counts of the sampled edges; d_bkt follows
   uint32_t part_buckets = 0;   // H
   uint32_t part_lb = 9;        // low key bits resolved by the second pass
   uint32_t* d_pairs = nullptr; // staging for host-resident input pairs, 2 x [pairs_cap] u32 pairs

@@ -84,3 +84,63 @@ def test_tagged_levels(restatement, n):
     flat = sk.tobytes()
     step = len(flat) // levels
     assert got == [flat[l * step:(l + 1) * step] for l in range(levels)]
+
+
+def _repeated(V, hubs, n, seed, share=0.5):
+    """n records of which `share` repeat an earlier one: vertex i < len(hubs) has about hubs[i] records."""
+    r = np.random.default_rng(seed)
+    parts = [np.stack([np.full(c, i), r.integers(len(hubs), V, c)], 1) for i, c in enumerate(hubs)]
+    fresh = np.concatenate(parts + [r.integers(0, V, size=(max(0, int(n * (1 - share)) - sum(hubs)), 2))]).astype(np.uint32)
+    again = fresh[r.integers(0, len(fresh), max(0, n - len(fresh)))][:, ::-1]
+    p = np.concatenate([fresh, again])
+    return np.ascontiguousarray(p[r.permutation(len(p))])
+
+
+@pytest.mark.parametrize("V,hubs,n", [
+    (50, [], 2_000_000),                              # every vertex several items
+    (100, [], 300_000),                               # bitmap listed by words
+    (5000, [1023, 1024, 1025, 2048, 2049, 4000], DIRECT + 5000),   # limits of the pass, of a tile
+    (200_003, [9000, 12000, 30000, 70000], 400_000),  # several tiles, by words, two items of one vertex
+    (1 << 18, [5000], DIRECT + 3), ((1 << 18) + 1, [5000], DIRECT + 3)])   # largest bitmap; none
+def test_toggles_that_cancel(restatement, V, hubs, n):
+    pairs = _repeated(V, hubs, n, V + n)
+    with gs.GraphSketch(V, 0xC0FFEE) as g:
+        for _ in range(2 if V <= 5000 else 1):        # a second pass starts from what the first one left
+            g.clear()
+            g.ingest_pairs(pairs)
+            g.synchronize()
+            if V <= 5000:
+                sk = restatement.new_sketches(V)
+                restatement.ingest(sk, V, 0xC0FFEE, pairs)
+                assert g.download().tobytes() == sk.tobytes()
+            else:
+                # by linearity: the same records in batches that are not grouped give the same sketches
+                with gs.GraphSketch(V, 0xC0FFEE) as h:
+                    for i in range(0, len(pairs), DIRECT):
+                        h.ingest_pairs(pairs[i:i + DIRECT])
+                    h.synchronize()
+                    for lo in range(0, V, 60000):
+                        c = min(60000, V - lo)
+                        assert g.download(first=lo, count=c).tobytes() == h.download(first=lo, count=c).tobytes()
+
+
+def test_toggles_that_cancel_in_tenants_and_levels(restatement):
+    sizes = [40, 3000, 700]
+    with SketchEngine(sum(tenant_bytes(V) for V in sizes) + (1 << 20), 3, sum(sizes), 3700) as e:
+        ids = [e.add_tenant(V, 9 + i) for i, V in enumerate(sizes)]
+        recs = [_repeated(V, [2500] if V == 3000 else [], 90_000, 31 + i, 0.6) for i, V in enumerate(sizes)]
+        e.ingest_batches(list(zip(ids, recs)))
+        e.synchronize()
+        for i, V in enumerate(sizes):
+            sk = restatement.new_sketches(V)
+            restatement.ingest(sk, V, 9 + i, recs[i])
+            assert e.download(ids[i]).tobytes() == sk.tobytes()
+    V, levels, L, seed = 60, 3, 9, 0xABC
+    pairs = _repeated(V, [], 200_000, 8)
+    with gs.GraphSketch(V, seed, num_levels=levels, num_subgraphs=L) as g:
+        g.ingest_pairs(pairs)
+        g.synchronize()
+        got = b"".join(g.download(level=l).tobytes() for l in range(levels))
+    sk = restatement.new_sketches(V, 1.0, levels)
+    restatement.ingest_levels(sk, V, levels, L, seed, pairs)
+    assert got == sk.tobytes()
