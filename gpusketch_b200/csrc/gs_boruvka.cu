@@ -234,6 +234,8 @@ struct BorArgs {
   GsBucket* acc;               // [vertex][W]
   uint64_t* edge;              // per hooked vertex: the edge that joined its component to another; may be null
   uint32_t* status;            // [0] error bits [4] forest edges (with `edge`)
+  uint32_t* out;               // one graph: result words in page-locked host memory (gs_boruvka_enqueue); or null
+  uint32_t* labels;            // one graph: [V] its labels in page-locked host memory, may be null
   uint32_t* tstate;            // [tenant][4]: done, -, rounds, out of samples
   BorCounters* ctr;            // grid scope: [2], zero at launch
   uint32_t* barrier;           // grid scope: arrivals, zero at launch
@@ -387,15 +389,18 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
     A.parent[v] = v;
     A.size[v] = 0;
   }
-  if (T.round0_col >= T.ns) {   // OutOfSamplesException before the first round
-    if (gtid == 0) { ts[0] = 1; ts[2] = 0; ts[3] = 1; }
-    return;
+  // with `out` the launch owns the status words: the error bits of earlier ingest calls move to word 16
+  if (A.out && gtid == 0) {
+    A.status[16] = A.status[0];
+    A.status[17] = 0;
+    for (int i = 0; i < 16; i++) A.status[i] = 0;
   }
   if (!meet(nullptr)) return;
+  uint32_t rounds = 0, oos = T.round0_col >= T.ns;   // OutOfSamplesException before the first round
 
   // ---- round 0: every vertex samples its own sketch, an octet of lanes for two; the edges of `per`
   //      passes are collected one per lane and unioned together ----
-  {
+  if (!oos) {
     const uint32_t per = min(4u, max(1u, (span + 8 * gwarps - 1) / (8 * gwarps)));
     for (uint32_t base = gwarp * 8 * per; base < span; base += gwarps * 8 * per) {
       uint64_t mine = ~0ull;
@@ -427,8 +432,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
     }
   }
 
-  uint32_t rounds = 0, oos = 0;
-  for (uint32_t round = 0;;) {
+  for (uint32_t round = 0; !oos || round;) {
     if (!meet(&ctr[round & 1].modified)) return;
     if (!ld_volatile(&ctr[round & 1].modified)) break;
     rounds = ++round;
@@ -721,6 +725,22 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
   }
 
   if (gtid == 0) { ts[0] = 1; ts[2] = rounds; ts[3] = oos; }
+  if (A.out) {
+    // the answer goes to the host from here: no read-back is queued behind the kernel, and no clearing
+    uint32_t count = 0;
+    for (uint32_t v = vlo + gtid; v < vend; v += gthreads) {
+      const uint32_t r = __ldcg(&A.parent[v]);
+      if (A.labels) A.labels[v] = r;
+      count += r == v;
+    }
+    count = __reduce_add_sync(0xffffffffu, count);
+    if (lane == 0 && count) atomicAdd(&A.status[17], count);
+    if (!meet(nullptr)) return;
+    if (gtid == 0) {
+      for (int i = 0; i < 18; i++) A.out[i] = ld_volatile(&A.status[i]);
+      A.status[0] = 0;   // read with this answer: the calls queued behind it start clean
+    }
+  }
   // the first block's counters stay until every block has read them
   if constexpr (CLUSTER) cg::this_cluster().sync();
 }
@@ -839,6 +859,8 @@ gs_status gs_boruvka_launch(const GsBorLaunch& L, cudaStream_t s) {
   A.acc = L.acc;
   A.edge = L.edge;
   A.status = L.status;
+  A.out = L.out;
+  A.labels = L.labels;
   A.tstate = L.tstate;
   A.ctr = reinterpret_cast<BorCounters*>(L.counters);
   A.barrier = L.counters + kGsBorCounterWords - 1;
@@ -879,7 +901,8 @@ gs_status gs_gather_forest(gs_graph* g, cudaStream_t s) {
   return GS_OK;
 }
 
-gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s, uint32_t* h_out) {
+gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s, uint32_t* h_out,
+                             uint32_t* h_labels) {
   const uint32_t V = g->V, nb = g->geom.num_buckets, bkt = g->geom.bkt_per_col;
   g->labels_valid = false;
   g->last_forest_edges = 0;
@@ -913,18 +936,12 @@ gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, c
   // the kernel expects all-zero accumulator rows and leaves them so when it runs to the end
   if (g->acc_dirty) GS_CUDA_TRY(cudaMemsetAsync(g->d_acc, 0, (size_t)V * (bkt + 1) * sizeof(GsBucket), s));
   g->acc_dirty = true;
-  // the ingest error bits not yet reported move to word 16 (read back with the query's words)
-  GS_CUDA_TRY(cudaMemcpyAsync(g->d_status + 16, g->d_status, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-  GS_CUDA_TRY(cudaMemsetAsync(g->d_status, 0, 16 * sizeof(uint32_t), s));
-  {
-    GsProfScope ps(g, GS_PROF_QUERY, s, 1);
-    GS_TRY(gs_boruvka_launch(L, s));
-  }
-  GS_CUDA_TRY(cudaMemcpyAsync(h_out, g->d_status, 17 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  // the query's error bits are read back with its words: the error word starts clean for the ingest
-  // calls queued after the query (a stale bit would fail the next synchronizing call)
-  GS_CUDA_TRY(cudaMemsetAsync(g->d_status, 0, sizeof(uint32_t), s));
-  return GS_OK;
+  // the kernel writes the words when it ends; one that gave up waiting does not
+  h_out[0] = GS_DEV_ERR_TIMEOUT;
+  L.out = h_out;
+  L.labels = h_labels;
+  GsProfScope ps(g, GS_PROF_QUERY, s, 1);
+  return gs_boruvka_launch(L, s);
 }
 
 // One graph: a cluster has 16 SMs and the hardware's barrier, the grid all of them and a barrier of about
@@ -942,7 +959,22 @@ GsBorScope gs_boruvka_scope(uint32_t V, uint32_t graphs) {
   return s;
 }
 
-gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, const uint32_t* st) {
+gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, uint32_t* st) {
+  if (st[0] & GS_DEV_ERR_TIMEOUT) {
+    // the words are still on the device
+    GS_CUDA_TRY(cudaMemcpy(st, g->d_status, 18 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    GS_CUDA_TRY(cudaMemset(g->d_status, 0, sizeof(uint32_t)));
+    st[0] |= GS_DEV_ERR_TIMEOUT;
+  }
+  // records skipped by the ingest calls before the query are reported first
+  if (st[16]) {
+    if (st[16] & GS_DEV_ERR_VERTEX_RANGE) {
+      gs_set_error("an edge record named a vertex id >= num_vertices; those records were skipped");
+      return GS_ERR_BAD_ARG;
+    }
+    gs_set_error("device consistency check failed (bits " + std::to_string(st[16]) + ")");
+    return GS_ERR_INTERNAL;
+  }
   if (st[0] & GS_DEV_ERR_TIMEOUT) {
     gs_set_error("a grid barrier of the Boruvka kernel gave up waiting");
     return GS_ERR_TIMEOUT;
@@ -958,13 +990,14 @@ gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, const uint32_t* st) {
   }
   g->last_rounds = st[8 + 2];
   g->last_forest_edges = st[4] < g->V ? st[4] : g->V - 1;
+  g->last_components = st[17];
   g->labels_valid = true;
   g->labels_level = level;
   return GS_OK;
 }
 
-gs_status gs_boruvka(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s) {
-  GS_TRY(gs_boruvka_enqueue(g, level, round0_col, s, g->h_status));
+gs_status gs_boruvka(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s, uint32_t* h_labels) {
+  GS_TRY(gs_boruvka_enqueue(g, level, round0_col, s, g->h_status, h_labels));
   GS_CUDA_TRY(cudaStreamSynchronize(s));
   return gs_boruvka_finish(g, level, g->h_status);
 }

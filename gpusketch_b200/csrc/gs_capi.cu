@@ -73,6 +73,19 @@ gs_status check_status(gs_graph* g, cudaStream_t s) {
   return GS_OK;
 }
 
+// Labels of graphs of at most this many vertices are written into page-locked memory by the query's kernel
+// and copied to the caller from there; larger ones are read back with a copy (at 10^6 vertices the extra
+// host copy costs more than the launch that it saves).
+constexpr uint32_t kKernelLabels = 1u << 16;
+
+gs_status ensure_query_buffers(gs_graph* g) {
+  if (g->h_qlabels) return GS_OK;
+  if (!g->h_qstatus) GS_CUDA_TRY(cudaMallocHost(&g->h_qstatus, 32 * sizeof(uint32_t)));
+  if (!g->ev_query) GS_CUDA_TRY(cudaEventCreateWithFlags(&g->ev_query, cudaEventDisableTiming));
+  GS_CUDA_TRY(cudaMallocHost(&g->h_qlabels, (size_t)g->V * sizeof(uint32_t)));
+  return GS_OK;
+}
+
 // work queued on a caller stream s must finish before the handle's own stream touches the sketches
 gs_status order_after(gs_graph* g, cudaStream_t s) {
   if (s == g->stream) return GS_OK;
@@ -244,6 +257,11 @@ uint64_t gs_desired_updates_per_batch(const gs_graph* g) {
 
 namespace {
 
+// Host batches of at most this many records are read by the kernels where they lie in the page-locked ring
+// (us per call of 100 records: 27 with the copy, 12 without; the eager DSU's and the exact tier's passes read
+// them again).
+constexpr uint64_t kZeroCopyPairs = 1024;
+
 // Host input moves through the staging slots: slice k is copied on the copy stream into device slot
 // k % 2 (from the caller's memory when it is page-locked, else through the pinned ring) while the
 // ingest of slice k - 1 runs.  With `wait_copies`, the call returns once every copy has landed (the
@@ -252,6 +270,19 @@ namespace {
 // the device, so copies of this call can run ahead of queries queued before it.
 gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cudaStream_t s, bool wait_copies) {
   GS_TRY(gs_ensure_pair_staging(g, n));
+  if (n <= kZeroCopyPairs) {
+    // a few records: copied into the ring by the host and read from there by the update's kernel, instead of
+    // a copy on another stream and the two events and the wait that tie it to this one
+    const int slot = (int)(g->zero_copy_next++ & 1);
+    GS_CUDA_TRY(cudaEventSynchronize(g->ev_done[slot]));
+    GS_CUDA_TRY(cudaEventSynchronize(g->ev_copy[slot]));
+    uint32_t* h = static_cast<uint32_t*>(g->h_pin) + (size_t)slot * g->pairs_cap * 2;
+    std::memcpy(h, pairs, (size_t)n * 2 * sizeof(uint32_t));
+    GS_TRY(gs_ingest_device_pairs(g, h, n, -1, s));
+    GS_CUDA_TRY(cudaEventRecord(g->ev_done[slot], s));
+    GS_CUDA_TRY(cudaEventRecord(g->ev_copy[slot], s));   // who waits for either may write the slot
+    return order_after(g, s);
+  }
   cudaPointerAttributes attr{};
   const bool pinned = cudaPointerGetAttributes(&attr, pairs) == cudaSuccess && attr.type == cudaMemoryTypeHost;
   cudaGetLastError();
@@ -454,29 +485,38 @@ gs_status gs_connected_components(gs_graph* g, uint32_t level, uint32_t* labels,
   if (g->query_pending) { gs_set_error("a queued query is pending: collect it with gs_query_wait first"); return GS_ERR_BAD_ARG; }
   GS_GUARD(g);
   cudaStream_t s = g->stream;
-  GS_TRY(check_status(g, s));
   bool cached = false;
-  if (level == 0) GS_TRY(gs_eager_state(g, s, &cached));
+  if (level == 0 && g->eager_on) {
+    GS_TRY(check_status(g, s));
+    GS_TRY(gs_eager_state(g, s, &cached));
+  }
+  const uint32_t V = g->V;
+  bool have_labels = false;   // already in h_qlabels
   if (cached) {
     GS_TRY(gs_eager_answer(g, s));   // CCSketchAlg::connected_components with shared_dsu_valid
   } else {
-    GS_TRY(gs_boruvka(g, level, 0, s));
+    have_labels = labels && V <= kKernelLabels;
+    if (have_labels) GS_TRY(ensure_query_buffers(g));
+    GS_TRY(gs_boruvka(g, level, 0, s, have_labels ? g->h_qlabels : nullptr));
     g->last_answer_eager = false;
     if (level == 0) GS_TRY(gs_eager_rebuild(g, s));
   }
   if (rounds) *rounds = g->last_rounds;
-  if (labels || num_cc) {
+  if (have_labels) {
+    std::memcpy(labels, g->h_qlabels, (size_t)V * sizeof(uint32_t));
+  } else if (labels || (num_cc && cached)) {
     std::vector<uint32_t> tmp;
     uint32_t* dst = labels;
-    if (!dst) { tmp.resize(g->V); dst = tmp.data(); }
-    GS_CUDA_TRY(cudaMemcpyAsync(dst, g->d_parent, (size_t)g->V * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (!dst) { tmp.resize(V); dst = tmp.data(); }
+    GS_CUDA_TRY(cudaMemcpyAsync(dst, g->d_parent, (size_t)V * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     GS_CUDA_TRY(cudaStreamSynchronize(s));
-    if (num_cc) {
+    if (num_cc && cached) {
       uint32_t c = 0;
-      for (uint32_t v = 0; v < g->V; v++) c += dst[v] == v;
+      for (uint32_t v = 0; v < V; v++) c += dst[v] == v;
       *num_cc = c;
     }
   }
+  if (num_cc && !cached) *num_cc = g->last_components;
   return GS_OK;
 }
 
@@ -486,11 +526,7 @@ gs_status gs_connected_components_async(gs_graph* g, uint32_t level) {
   if (g->query_pending) { gs_set_error("a queued query is pending: collect it with gs_query_wait first"); return GS_ERR_BAD_ARG; }
   GS_GUARD(g);
   cudaStream_t s = g->stream;
-  if (!g->h_qlabels) {
-    GS_CUDA_TRY(cudaMallocHost(&g->h_qstatus, 32 * sizeof(uint32_t)));
-    GS_CUDA_TRY(cudaMallocHost(&g->h_qlabels, (size_t)g->V * sizeof(uint32_t)));
-    GS_CUDA_TRY(cudaEventCreateWithFlags(&g->ev_query, cudaEventDisableTiming));
-  }
+  GS_TRY(ensure_query_buffers(g));
   g->query_level = level;
   g->query_changes = g->changes;
   g->query_done = false;
@@ -505,8 +541,10 @@ gs_status gs_connected_components_async(gs_graph* g, uint32_t level) {
     g->query_pending = true;
     return GS_OK;
   }
-  GS_TRY(gs_boruvka_enqueue(g, level, 0, s, g->h_qstatus));
-  GS_CUDA_TRY(cudaMemcpyAsync(g->h_qlabels, g->d_parent, (size_t)g->V * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  const bool kernel_labels = g->V <= kKernelLabels;
+  GS_TRY(gs_boruvka_enqueue(g, level, 0, s, g->h_qstatus, kernel_labels ? g->h_qlabels : nullptr));
+  if (!kernel_labels)
+    GS_CUDA_TRY(cudaMemcpyAsync(g->h_qlabels, g->d_parent, (size_t)g->V * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   GS_CUDA_TRY(cudaEventRecord(g->ev_query, s));
   g->query_pending = true;
   return GS_OK;
@@ -526,30 +564,14 @@ gs_status gs_query_wait(gs_graph* g, uint32_t* labels, uint32_t* num_cc, uint32_
     return GS_OK;
   }
   GS_CUDA_TRY(cudaEventSynchronize(g->ev_query));
-  const uint32_t* st = g->h_qstatus;
-  if (st[16] & GS_DEV_ERR_VERTEX_RANGE) {
-    // as gs_connected_components, which reports records skipped by earlier ingest calls first
-    gs_set_error("an edge record named a vertex id >= num_vertices; those records were skipped");
-    g->acc_dirty = true;
-    return GS_ERR_BAD_ARG;
-  }
-  if (st[16]) {
-    gs_set_error("device consistency check failed (bits " + std::to_string(st[16]) + ")");
-    g->acc_dirty = true;
-    return GS_ERR_INTERNAL;
-  }
-  GS_TRY(gs_boruvka_finish(g, g->query_level, st));
+  GS_TRY(gs_boruvka_finish(g, g->query_level, g->h_qstatus));
   g->last_answer_eager = false;
   // the partition stays valid for point queries only while no later call has changed the sketches
   g->labels_valid = g->changes == g->query_changes;
   if (g->query_level == 0 && g->eager_on) GS_TRY(gs_eager_rebuild(g, g->stream));
   if (rounds) *rounds = g->last_rounds;
   if (labels) std::memcpy(labels, g->h_qlabels, (size_t)V * sizeof(uint32_t));
-  if (num_cc) {
-    uint32_t c = 0;
-    for (uint32_t v = 0; v < V; v++) c += g->h_qlabels[v] == v;
-    *num_cc = c;
-  }
+  if (num_cc) *num_cc = g->last_components;
   return GS_OK;
 }
 

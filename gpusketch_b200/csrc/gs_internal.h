@@ -100,6 +100,7 @@ struct gs_graph {
   void* h_pin = nullptr;       // 2 pinned staging buffers of pairs_cap pairs
   uint2* d_file_pairs = nullptr; // decoded records of one stream-file slice (gs_ingest_stream_file)
   cudaStream_t copy_stream = nullptr;               // H2D of host input slices
+  uint64_t zero_copy_next = 0;                      // ring slot of the next small host batch
   cudaEvent_t ev_copy[2] = {nullptr, nullptr};      // slice copied into d_pairs[slot]
   cudaEvent_t ev_done[2] = {nullptr, nullptr};      // slice in d_pairs[slot] consumed
   uint32_t* d_status = nullptr;  // [0] error bits [1] records [2] chunks [3] modified [4] forest [5] part chunks
@@ -115,7 +116,7 @@ struct gs_graph {
   gs_status query_status = GS_OK;  // answer already known at submission (eager DSU, or an error)
   bool query_done = false;
   uint32_t* h_qstatus = nullptr;   // pinned, 32 words: the query's status words
-  uint32_t* h_qlabels = nullptr;   // pinned, V labels
+  uint32_t* h_qlabels = nullptr;   // pinned, V labels (also of synchronous queries of small graphs)
   cudaEvent_t ev_query = nullptr;  // recorded after the labels' read-back
 
   // ---- Boruvka scratch ----
@@ -132,6 +133,7 @@ struct gs_graph {
   bool acc_dirty = true;         // d_acc may hold non-zero rows (new, or a query ended early)
   uint32_t last_forest_edges = 0;
   uint32_t last_rounds = 0;
+  uint32_t last_components = 0;
   std::vector<uint32_t> sample_cursor;  // per level: round-0 column of the next k-forest
   bool labels_valid = false;     // d_parent holds the partition of the last query
   uint32_t labels_level = 0;
@@ -224,13 +226,15 @@ gs_status gs_ingest_device_batches(gs_graph* g, uint32_t level, const uint32_t* 
                                    const uint64_t* d_starts, const uint64_t* d_sizes,
                                    uint32_t nb, const uint32_t* d_dsts, cudaStream_t s,
                                    uint64_t max_records = 0);  // 0: read the record count back
-// Device Boruvka on one level; its forest stays in g->d_edge (gs_gather_forest).
-gs_status gs_boruvka(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s);
-// The same in two halves: the launch and the read-back of status words [0, 17) into pinned h_out
-// (word 16: ingest error bits queued before the query), queued on s without waiting; then, once
-// that work is done, the interpretation of those words.
-gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s, uint32_t* h_out);
-gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, const uint32_t* st);
+// Device Boruvka on one level; its forest stays in g->d_edge (gs_gather_forest).  h_labels (page-locked host
+// memory, may be null): the kernel also writes the labels there.
+gs_status gs_boruvka(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s, uint32_t* h_labels = nullptr);
+// The same in two halves: the launch, whose kernel writes 18 result words to page-locked h_out (0 error bits,
+// 4 forest edges, 8-11 the graph's state, 16 error bits of the ingest calls before the query, 17 components),
+// queued on s without waiting; then, once that work is done, the interpretation of those words.
+gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, cudaStream_t s, uint32_t* h_out,
+                             uint32_t* h_labels);
+gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, uint32_t* st);
 
 // Eager DSU (gs_eager.cu).
 gs_status gs_eager_enable(gs_graph* g, bool on, cudaStream_t s);
@@ -289,6 +293,8 @@ struct GsBorLaunch {
   uint64_t* edge = nullptr;              // [vertices] edge of every vertex that a union hooked; may be null
   uint32_t* status = nullptr;            // [0] errors [4] forest edges (with `edge`)
   uint32_t* tstate = nullptr;            // [tenant][4]: done, -, rounds, out of samples
+  uint32_t* out = nullptr;               // one graph: page-locked host memory for the result words, and
+  uint32_t* labels = nullptr;            // for the labels; may be null
   uint32_t* counters = nullptr;          // [kGsBorCounterWords] (grid scope)
   uint64_t wait_ns = kGsDefaultWaitNs;   // grid-barrier wait limit
   // Only when every graph's vertex sketches XOR to zero (every update reached both endpoints): the
