@@ -60,9 +60,8 @@ namespace {
 
 constexpr uint32_t kGood = 0, kZero = 1, kFail = 2;
 // Threads of a block.  Grid scope: one block per SM, so that the barrier has few arrivals.  Narrow
-// clusters: two blocks per SM, because a small graph's block mostly waits and another's fills in (256 graphs
-// of up to 16384 vertices: 1.08 ms against 1.23 with wide ones).  Wide clusters: few graphs, whose largest
-// one sets the time (8 graphs of up to 65536: 0.53 against 0.61 ms).
+// clusters (many graphs): two blocks per SM, because a small graph's block mostly waits and another's fills
+// in (256 graphs of up to 16384 vertices: 1.08 ms against 1.23 with wide ones).  Wide clusters: few graphs.
 enum Scope { kGrid = 0, kNarrow = 1, kWide = 2 };
 constexpr uint32_t threads_of(int scope) { return scope == kNarrow ? 512u : 1024u; }
 constexpr uint32_t kPiece = 16;                  // members of a component that one warp gathers
@@ -282,6 +281,86 @@ __device__ __forceinline__ void xor_row(GsBucket* row, uint32_t j, uint64_t a, u
   atomicXor(reinterpret_cast<unsigned long long*>(&row[j].gamma), (unsigned long long)g);
 }
 
+// What the kernels know of the graph that a thread works on.
+struct Graph {
+  uint32_t vlo, span;
+  uint32_t* parent;
+  uint64_t* edge;
+  uint32_t* err;
+};
+
+// the edge of a sample, or ~0: anything but a pair of distinct vertices is a checksum collision
+__device__ __forceinline__ uint64_t edge_of(const Graph& G, uint64_t idx) {
+  const uint32_t s = (uint32_t)(idx >> 32), d = (uint32_t)idx;
+  return s < G.span && d < G.span && s != d ? ((uint64_t)(G.vlo + s) << 32) | (G.vlo + d) : ~0ull;
+}
+
+// Every lane unions its edge (~0: none), so that up to 32 overlap.  A vertex is hooked once at most: its edge
+// is kept at its place, and the hooked vertices' edges are the forest.
+__device__ __forceinline__ void unite(const Graph& G, uint64_t e, uint32_t* s_hooked) {
+  if (e == ~0ull) return;
+  const uint32_t hooked = cached_union(G.parent, (uint32_t)(e >> 32), (uint32_t)e, G.span + 64, G.err);
+  if (hooked == 0xffffffffu) return;
+  atomicAdd(s_hooked, 1u);
+  if (G.edge) G.edge[hooked] = e;
+}
+
+// Round 0: every vertex samples its own sketch, an octet of lanes for two; the edges of `per` passes are
+// collected one per lane and unioned together.
+__device__ __forceinline__ void round_zero(const Graph& G, const GsBucket* sk, const GsBorTenant& T, uint32_t gwarp,
+                                           uint32_t gwarps, uint32_t* s_mod, uint32_t* s_hooked) {
+  const uint32_t lane = lane_id(), span = G.span;
+  const uint32_t per = min(4u, max(1u, (span + 8 * gwarps - 1) / (8 * gwarps)));
+  for (uint32_t base = gwarp * 8 * per; base < span; base += gwarps * 8 * per) {
+    uint64_t mine = ~0ull;
+    bool failed = false;
+    for (uint32_t i = 0; i < per; i++) {
+      const GsBucket *col[2], *det[2];
+      bool active[2];
+      uint32_t code[2];
+      uint64_t idx[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const uint32_t k = base + 8 * i + 4 * u + (lane >> 3);
+        active[u] = k < span;
+        const GsBucket* own = sk + (size_t)(k < span ? k : 0u) * T.nb;
+        col[u] = own + (size_t)T.round0_col * T.bkt;
+        det[u] = own + (T.nb - 1);
+      }
+      sample_octet2(col, det, T.bkt, T.csmix, active, code, idx);
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        failed |= active[u] && code[u] == kFail;
+        const uint64_t e = active[u] && code[u] == kGood ? edge_of(G, idx[u]) : ~0ull;
+        const uint64_t x = __shfl_sync(0xffffffffu, e, (lane & 3u) * 8u);
+        if ((lane >> 2) == 2 * i + u) mine = x;
+      }
+    }
+    if (failed) *s_mod = 1;
+    unite(G, mine, s_hooked);
+  }
+}
+
+// The answer of a query of one graph, written to the host from the kernel: no read-back is queued behind it,
+// and no clearing.  `meet` is the graph's barrier.
+template <typename Meet>
+__device__ __forceinline__ void write_answer(const BorArgs& A, const Graph& G, uint32_t gtid, uint32_t gthreads,
+                                             Meet&& meet) {
+  uint32_t count = 0;
+  for (uint32_t v = G.vlo + gtid; v < G.vlo + G.span; v += gthreads) {
+    const uint32_t r = __ldcg(&G.parent[v]);
+    if (A.labels) A.labels[v] = r;
+    count += r == v;
+  }
+  count = __reduce_add_sync(0xffffffffu, count);
+  if (lane_id() == 0 && count) atomicAdd(&A.status[17], count);
+  if (!meet(nullptr)) return;
+  if (gtid == 0) {
+    for (int i = 0; i < 18; i++) A.out[i] = ld_volatile(&A.status[i]);
+    A.status[0] = 0;   // read with this answer: the calls queued behind it start clean
+  }
+}
+
 // exclusive scan over the block (every thread calls it), and the block's total
 template <uint32_t kWarps>
 __device__ __forceinline__ unsigned long long block_scan(unsigned long long x, unsigned long long* s_sums,
@@ -366,20 +445,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       return grid_barrier(A.barrier, barriers, err, A.wait_ns);
     }
   };
-  // the edge of a sample, or ~0: anything but a pair of distinct vertices is a checksum collision
-  auto edge_of = [&](uint64_t idx) -> uint64_t {
-    const uint32_t s = (uint32_t)(idx >> 32), d = (uint32_t)idx;
-    return s < span && d < span && s != d ? ((uint64_t)(vlo + s) << 32) | (vlo + d) : ~0ull;
-  };
-  // every lane unions its edge (~0: none), so that up to 32 overlap.  A vertex is hooked once at most: its
-  // edge is kept at its place, and the hooked vertices' edges are the forest.
-  auto unite = [&](uint64_t e) {
-    if (e == ~0ull) return;
-    const uint32_t hooked = cached_union(A.parent, (uint32_t)(e >> 32), (uint32_t)e, limit, err);
-    if (hooked == 0xffffffffu) return;
-    atomicAdd(&s_hooked, 1u);
-    if (A.edge) A.edge[hooked] = e;
-  };
+  const Graph G{vlo, span, A.parent, A.edge, err};
 
   if (threadIdx.x == 0) { s_mod = 0; s_hooked = 0; s_best = 0; }
   if (CLUSTER && threadIdx.x < 2 * sizeof(BorCounters) / sizeof(uint32_t))
@@ -398,39 +464,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
   if (!meet(nullptr)) return;
   uint32_t rounds = 0, oos = T.round0_col >= T.ns;   // OutOfSamplesException before the first round
 
-  // ---- round 0: every vertex samples its own sketch, an octet of lanes for two; the edges of `per`
-  //      passes are collected one per lane and unioned together ----
-  if (!oos) {
-    const uint32_t per = min(4u, max(1u, (span + 8 * gwarps - 1) / (8 * gwarps)));
-    for (uint32_t base = gwarp * 8 * per; base < span; base += gwarps * 8 * per) {
-      uint64_t mine = ~0ull;
-      bool failed = false;
-      for (uint32_t i = 0; i < per; i++) {
-        const GsBucket *col[2], *det[2];
-        bool active[2];
-        uint32_t code[2];
-        uint64_t idx[2];
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const uint32_t k = base + 8 * i + 4 * u + (lane >> 3);
-          active[u] = k < span;
-          const GsBucket* own = sk + (size_t)(k < span ? k : 0u) * T.nb;
-          col[u] = own + (size_t)T.round0_col * bkt;
-          det[u] = own + (T.nb - 1);
-        }
-        sample_octet2(col, det, bkt, T.csmix, active, code, idx);
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          failed |= active[u] && code[u] == kFail;
-          const uint64_t e = active[u] && code[u] == kGood ? edge_of(idx[u]) : ~0ull;
-          const uint64_t x = __shfl_sync(0xffffffffu, e, (lane & 3u) * 8u);
-          if ((lane >> 2) == 2 * i + u) mine = x;
-        }
-      }
-      if (failed) s_mod = 1;
-      unite(mine);
-    }
-  }
+  if (!oos) round_zero(G, sk, T, gwarp, gwarps, &s_mod, &s_hooked);
 
   for (uint32_t round = 0; !oos || round;) {
     if (!meet(&ctr[round & 1].modified)) return;
@@ -670,18 +704,18 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
 #pragma unroll
               for (int k = 0; k < SLOTS; k++)
                 if (at / 32u == (uint32_t)k) idx = __shfl_sync(0xffffffffu, a[k], at & 31u);
-              e = edge_of(idx);
+              e = edge_of(G, idx);
             }
           }
           if (lane == held) mine = e;
           if (++held == 32) {
-            unite(mine);
+            unite(G, mine, &s_hooked);
             __syncwarp();
             mine = ~0ull;
             held = 0;
           }
         }
-        if (held) unite(mine);
+        if (held) unite(G, mine, &s_hooked);
         flush_pieces();
       }
       if (comp != 0xffffffffu) {
@@ -720,29 +754,191 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       if (code == kFail) s_mod = 1;
       __syncwarp();
       for (uint32_t j = lane; j <= bkt; j += 32) row[j] = GsBucket{0, 0};
-      unite(lane == 0 && code == kGood ? edge_of(idx) : ~0ull);
+      unite(G, lane == 0 && code == kGood ? edge_of(G, idx) : ~0ull, &s_hooked);
     }
   }
 
   if (gtid == 0) { ts[0] = 1; ts[2] = rounds; ts[3] = oos; }
-  if (A.out) {
-    // the answer goes to the host from here: no read-back is queued behind the kernel, and no clearing
-    uint32_t count = 0;
-    for (uint32_t v = vlo + gtid; v < vend; v += gthreads) {
-      const uint32_t r = __ldcg(&A.parent[v]);
-      if (A.labels) A.labels[v] = r;
-      count += r == v;
-    }
-    count = __reduce_add_sync(0xffffffffu, count);
-    if (lane == 0 && count) atomicAdd(&A.status[17], count);
-    if (!meet(nullptr)) return;
-    if (gtid == 0) {
-      for (int i = 0; i < 18; i++) A.out[i] = ld_volatile(&A.status[i]);
-      A.status[0] = 0;   // read with this answer: the calls queued behind it start clean
-    }
-  }
+  if (A.out) write_answer(A, G, gtid, gthreads, meet);
   // the first block's counters stay until every block has read them
   if constexpr (CLUSTER) cg::this_cluster().sync();
+}
+
+// One graph on a cluster, few graphs in the launch: a round in two phases.
+//   accumulate  a warp takes consecutive vertices, walks to their roots (compressing the parents) and XORs their
+//               column r and deterministic bucket into the root's accumulator row - in registers while the root
+//               stays the same, then by atomics; the warps' last rows are combined per block
+//   sample      an octet of lanes per vertex: a root samples its row, zeroes it and unions the sampled edge
+// Atomics on rows in L2 are fast (200 per ns) as long as the rows fit there, so nothing is listed, sized or
+// complemented: what a small graph's round costs is the chain of phases and their latency, not the bytes.
+// Measured (us per query call, against the member lists of k_boruvka on the same cluster): V = 1000 117 -> 80,
+// 4096 127 -> 109, 16384 341 -> 285; 8 graphs of up to 65536 vertices 620 -> 418.
+template <int SLOTS>
+__global__ void __launch_bounds__(threads_of(kWide), 1) k_boruvka_flat(const BorArgs A) {
+  constexpr uint32_t kThreads = threads_of(kWide), kWarps = kThreads / 32;
+  extern __shared__ __align__(16) GsBucket s_rows[];   // [kWarps][R] the warps' last rows
+  __shared__ uint32_t s_flag[2];                       // the first block's: some sample failed or union succeeded
+  __shared__ uint32_t s_root[kWarps], s_mod, s_hooked;
+  const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
+  cg::cluster_group cl = cg::this_cluster();
+  const uint32_t block = cl.block_rank(), blocks = cl.num_blocks();
+  volatile uint32_t* const flag = cl.map_shared_rank(s_flag, 0);
+  const uint32_t t = A.qlist ? A.qlist[blockIdx.x / blocks] : 0u;
+  const GsBorTenant T = A.tenants ? A.tenants[t] : A.t0;
+  const uint32_t vlo = T.vbase, span = T.V, vend = T.vbase + T.V;
+  const uint32_t bkt = T.bkt, W = A.W, R = A.R;
+  const uint32_t gtid = block * kThreads + threadIdx.x, gthreads = blocks * kThreads;
+  const uint32_t gwarp = gtid >> 5, gwarps = gthreads >> 5;
+  const uint32_t limit = span + 64;
+  const GsBucket* const sk = A.sk + T.sk_off;
+  uint32_t* const ts = A.tstate + 4 * t;
+  const Graph G{vlo, span, A.parent, A.edge, A.status};
+
+  auto meet = [&](volatile uint32_t* f) -> bool {
+    if (f) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        if (s_mod | s_hooked) *f = 1u;
+        if (s_hooked && A.edge) atomicAdd(&A.status[4], s_hooked);
+        s_mod = 0;
+        s_hooked = 0;
+      }
+    }
+    cg::this_cluster().sync();
+    return true;
+  };
+
+  if (threadIdx.x == 0) { s_mod = 0; s_hooked = 0; s_flag[0] = 0; s_flag[1] = 0; }
+  for (uint32_t v = vlo + gtid; v < vend; v += gthreads) A.parent[v] = v;
+  if (A.out && gtid == 0) {   // as in k_boruvka
+    A.status[16] = A.status[0];
+    A.status[17] = 0;
+    for (int i = 0; i < 16; i++) A.status[i] = 0;
+  }
+  meet(nullptr);
+  uint32_t rounds = 0, oos = T.round0_col >= T.ns;
+  if (!oos) round_zero(G, sk, T, gwarp, gwarps, &s_mod, &s_hooked);
+
+  for (uint32_t round = 0; !oos || round;) {
+    meet(flag + (round & 1));
+    if (!flag[round & 1]) break;
+    rounds = ++round;
+    oos = rounds >= T.ns;
+
+    // ---- accumulate ----
+    {
+      constexpr uint32_t kTake = 4;
+      const uint32_t take = min(kTake, max(1u, (span + gwarps - 1) / gwarps));
+      uint32_t cur = 0xffffffffu;
+      uint64_t a[SLOTS] = {}, g[SLOTS] = {};
+      for (uint32_t base = gwarp * take; base < span; base += gwarps * take) {
+        const uint32_t n = min(take, span - base);
+        uint32_t r = 0;
+        if (lane < n) {
+          const uint32_t v = vlo + base + lane;
+          r = cached_root(A.parent, v, limit, A.status);
+          A.parent[v] = r;
+          A.size[v] = r == v;   // the roots that sample: a union of the sample phase may hook one before its turn
+        }
+        if (oos) continue;   // only the labels are still wanted
+        GsBucket b[kTake][SLOTS];
+#pragma unroll
+        for (uint32_t u = 0; u < kTake; u++) {
+          const GsBucket* vb = sk + (size_t)(base + u) * T.nb;
+#pragma unroll
+          for (int k = 0; k < SLOTS; k++) {
+            const uint32_t j = lane + 32u * k;
+            b[u][k] = u < n && j <= bkt ? ld_bucket_cg(vb + (j < bkt ? round * bkt + j : T.nb - 1)) : GsBucket{0, 0};
+          }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kTake; u++) {
+          if (u >= n) break;
+          const uint32_t root = __shfl_sync(0xffffffffu, r, u);
+          if (root != cur) {
+            if (cur != 0xffffffffu) {
+#pragma unroll
+              for (int k = 0; k < SLOTS; k++)
+                if (lane + 32u * k <= bkt && (a[k] | g[k])) xor_row(A.acc + (size_t)cur * W, lane + 32u * k, a[k], g[k]);
+            }
+            cur = root;
+#pragma unroll
+            for (int k = 0; k < SLOTS; k++) a[k] = g[k] = 0;
+          }
+#pragma unroll
+          for (int k = 0; k < SLOTS; k++) { a[k] ^= b[u][k].alpha; g[k] ^= b[u][k].gamma; }
+        }
+      }
+      // the last rows: most warps hold the largest component's, and its atomics would queue
+      if (lane == 0) s_root[wib] = cur;
+#pragma unroll
+      for (int k = 0; k < SLOTS; k++)
+        if (lane + 32u * k <= bkt) s_rows[wib * R + lane + 32u * k] = GsBucket{a[k], g[k]};
+      __syncthreads();
+      const uint32_t same = __ballot_sync(0xffffffffu, s_root[lane] == cur);
+      if (cur != 0xffffffffu && wib == (uint32_t)(__ffs(same) - 1)) {
+        for (uint32_t m = same & (same - 1); m; m &= m - 1) {
+          const GsBucket* other = s_rows + (__ffs(m) - 1) * R;
+#pragma unroll
+          for (int k = 0; k < SLOTS; k++)
+            if (lane + 32u * k <= bkt) { a[k] ^= other[lane + 32u * k].alpha; g[k] ^= other[lane + 32u * k].gamma; }
+        }
+#pragma unroll
+        for (int k = 0; k < SLOTS; k++)
+          if (lane + 32u * k <= bkt && (a[k] | g[k])) xor_row(A.acc + (size_t)cur * W, lane + 32u * k, a[k], g[k]);
+      }
+    }
+    meet(nullptr);
+    if (threadIdx.x == 0 && block == 0) flag[(round + 1) & 1] = 0;   // everyone read it before this barrier
+    if (oos) break;
+
+    // ---- sample ----
+    for (uint32_t base = gwarp * 4; base < span; base += gwarps * 4) {
+      const uint32_t sub = lane & 7u, oct = lane >> 3;
+      const uint32_t v = vlo + base + oct;
+      const bool root = base + oct < span && __ldcg(&A.size[v]) != 0;
+      if (!__any_sync(0xffffffffu, root)) continue;
+      GsBucket* const row = A.acc + (size_t)(root ? v : vlo) * W;
+      const GsBucket det = root ? ld_bucket_cg(row + bkt) : GsBucket{0, 0};
+      bool decided = !root;
+      uint32_t code = kFail;
+      uint64_t idx = 0;
+      for (uint32_t j0 = 0; j0 < bkt; j0 += 32) {   // four depths a lane on their way at once
+        GsBucket b[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t j = j0 + 8 * k + sub;
+          b[k] = !decided && j < bkt ? ld_bucket_cg(row + j) : GsBucket{0, 0};
+        }
+        if (j0 == 0 && root) {
+          if (det.alpha == 0 && det.gamma == 0) { code = kZero; decided = true; }
+          else if (is_good(det, T.csmix)) { code = kGood; idx = det.alpha; decided = true; }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t j = j0 + 8 * k + sub;
+          const uint32_t m = __ballot_sync(0xffffffffu, !decided && j < bkt && is_good(b[k], T.csmix));
+          const uint32_t mine = (m >> (8u * oct)) & 0xffu;
+          const uint64_t x = __shfl_sync(0xffffffffu, b[k].alpha, mine ? 8u * oct + (uint32_t)(__ffs(mine) - 1) : lane);
+          if (!decided && mine) { code = kGood; idx = x; decided = true; }
+        }
+        if (__all_sync(0xffffffffu, decided)) break;
+      }
+      __syncwarp();
+      if (root) {
+        for (uint32_t j = sub; j <= bkt; j += 8) row[j] = GsBucket{0, 0};
+        if (sub == 0) {
+          if (code == kFail) s_mod = 1;
+          if (code == kGood) unite(G, edge_of(G, idx), &s_hooked);
+        }
+      }
+      __syncwarp();
+    }
+  }
+
+  if (gtid == 0) { ts[0] = 1; ts[2] = rounds; ts[3] = oos; }
+  if (A.out) write_answer(A, G, gtid, gthreads, meet);
+  cg::this_cluster().sync();   // the first block's flags stay until every block has read them
 }
 
 // the edges of the hooked vertices, as (min, max) pairs in any order
@@ -772,8 +968,14 @@ __global__ void __launch_bounds__(256) k_forest(const uint32_t* __restrict__ par
   }
 }
 
-size_t ring_bytes(int scope, uint32_t R) {
-  return (size_t)(threads_of(scope) / 32) * kRing * R * sizeof(GsBucket);
+template <int SCOPE, int SLOTS>
+constexpr auto kernel_of() {
+  if constexpr (SCOPE == kWide) return k_boruvka_flat<SLOTS>;
+  else return k_boruvka<SCOPE, SLOTS>;
+}
+
+size_t dynamic_bytes(int scope, uint32_t R) {
+  return (size_t)(threads_of(scope) / 32) * (scope == kWide ? 1 : kRing) * R * sizeof(GsBucket);
 }
 
 // Launches of more than 48 KB of dynamic shared memory, and clusters of more than 8 blocks, are opted into
@@ -782,19 +984,19 @@ template <int SCOPE, int SLOTS>
 gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s) {
   struct Opted { uint32_t R = 0, blocks = 0; int sms = 0; };
   static thread_local Opted opted[64];
+  constexpr auto kernel = kernel_of<SCOPE, SLOTS>();
   int dev = 0;
   GS_CUDA_TRY(cudaGetDevice(&dev));
   Opted& o = opted[dev & 63];
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cfg.blockDim = dim3(threads_of(SCOPE));
-  cfg.dynamicSmemBytes = ring_bytes(SCOPE, L.R);
+  cfg.dynamicSmemBytes = dynamic_bytes(SCOPE, L.R);
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (o.R < L.R) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(k_boruvka<SCOPE, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)cfg.dynamicSmemBytes));
+    GS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
     GS_CUDA_TRY(cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev));
     o.blocks = 8;
     if (SCOPE != kGrid) {
@@ -804,8 +1006,8 @@ gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s)
       attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
       cfg.gridDim = dim3(16);
       int n = 0;
-      if (cudaFuncSetAttribute(k_boruvka<SCOPE, SLOTS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-          cudaOccupancyMaxActiveClusters(&n, k_boruvka<SCOPE, SLOTS>, &cfg) == cudaSuccess && n > 0)
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0)
         o.blocks = 16;
       cudaGetLastError();
     }
@@ -825,7 +1027,7 @@ gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s)
     cfg.gridDim = dim3(o.sms);
     GS_CUDA_TRY(cudaMemsetAsync(A.ctr, 0, kGsBorCounterWords * sizeof(uint32_t), s));
   }
-  GS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_boruvka<SCOPE, SLOTS>, A));
+  GS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A));
   return GS_OK;
 }
 
@@ -945,18 +1147,14 @@ gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, c
 }
 
 // One graph: a cluster has 16 SMs and the hardware's barrier, the grid all of them and a barrier of about
-// 1.5 us; the two meet near 8192 vertices (us per query, cluster / grid: V = 1024 84 / 134, 4096 190 / 271,
-// 8192 225 / 234, 16384 295 / 195).  Several graphs: clusters side by side, smaller ones the more graphs
-// there are (256 graphs of up to 16384 vertices: 1.57 ms with 2 blocks each, 1.08 with 4, 1.54 with 8).
+// 1.5 us; the two meet above 8192 vertices (us per query call, cluster / grid: V = 1024 88 / 178, 4096
+// 109 / 165, 8192 184 / 220, 16384 285 / 207).  Several graphs: clusters side by side.  Up to 18 graphs get
+// wide ones (8 graphs of up to 65536 vertices: 0.42 ms against 0.62 with narrow ones); of more, the rows
+// fall out of L2, so members are listed, on smaller clusters (256 graphs of up to 16384 vertices, narrow:
+// 1.57 ms with 2 blocks each, 1.08 with 4, 1.54 with 8; wide: 2.1 at best).
 GsBorScope gs_boruvka_scope(uint32_t V, uint32_t graphs) {
-  GsBorScope s;
-  if (graphs == 1) {
-    if (V <= 8192) s.blocks = 16;
-    return s;
-  }
-  s.blocks = graphs > 36 ? 4 : graphs > 18 ? 8 : 16;
-  s.wide = V > 4096 && graphs <= 18;
-  return s;
+  if (graphs == 1) return V <= 8192 ? GsBorScope{16, true} : GsBorScope{};
+  return graphs <= 18 ? GsBorScope{16, true} : GsBorScope{graphs > 36 ? 4u : 8u, false};
 }
 
 gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, uint32_t* st) {
