@@ -16,8 +16,9 @@
 // phases, in one of two scopes:
 //   cluster   one thread-block cluster per graph: the barrier is the hardware's, and any number of
 //             graphs share a launch without waiting for one another;
-//   grid      one graph over the whole GPU (cooperative launch); the barrier is a counter in
-//             global memory, and every wait on it is bounded and reports GS_DEV_ERR_TIMEOUT.
+//   grid      one graph, or the large ones of several, over the whole GPU (cooperative launch); the
+//             barrier is a counter in global memory, and every wait on it is bounded and reports
+//             GS_DEV_ERR_TIMEOUT.
 //
 // A round after round 0 (barriers between the phases):
 //   compress  parent[v] = root(v); in the same pass every component's size, every vertex's rank in
@@ -38,6 +39,10 @@
 // the columns of every vertex outside it.  The largest component's members are then never listed or
 // read, and every gathered piece is folded into the largest component's row as well.
 //
+// Closed components (the same sketch sets): a component whose deterministic bucket is zero has no edge out,
+// its merged columns are zero, and no other component can sample an edge into it; its vertices are marked
+// and cost a load per round from then on (isolated vertices are most of a sparse R-MAT graph).
+//
 // Bound: latency.  A round is a chain of about a dozen dependent loads and five barriers, whatever the
 // graph's size, until the graph is large enough for the member columns' bytes to matter.
 // Measured (one query, us): V = 1024 199 -> 84, 16384 345 -> 195, 100003 835 -> 400, 131072 (R-MAT) 1062 ->
@@ -50,6 +55,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "gs_dsu.cuh"
 #include "gs_internal.h"
@@ -59,11 +65,12 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr uint32_t kGood = 0, kZero = 1, kFail = 2;
+constexpr uint32_t kClosed = 0xffffffffu;         // rank of a vertex whose component has no edge out
 // Threads of a block.  Grid scope: one block per SM, so that the barrier has few arrivals.  Narrow
 // clusters (many graphs): two blocks per SM, because a small graph's block mostly waits and another's fills
 // in (256 graphs of up to 16384 vertices: 1.08 ms against 1.23 with wide ones).  Wide clusters: few graphs.
 enum Scope { kGrid = 0, kNarrow = 1, kWide = 2 };
-constexpr uint32_t threads_of(int scope) { return scope == kNarrow ? 512u : 1024u; }
+constexpr uint32_t threads_of(int scope, bool many = false) { return scope == kNarrow ? 512u : many ? 768u : 1024u; }
 constexpr uint32_t kPiece = 16;                  // members of a component that one warp gathers
 constexpr uint32_t kGroup = 4;                   // member rows a warp asks for together
 constexpr uint32_t kRing = 2 * kGroup;           // member rows a warp has room for
@@ -110,16 +117,19 @@ __device__ __forceinline__ void sample_warp(const GsBucket* col, const GsBucket*
 // sketch: eight vertices per warp).  Lane k of the octet checks depths k, k+8, ...; a vertex's answer is
 // the lowest good depth among the octet's lanes.  The deterministic buckets and the first eight depths of
 // both vertices are loaded together: most vertices are decided by them, and a pass is one DRAM latency.
-// Every lane of the warp runs the same passes (bkt is the graph's) and reaches every full-warp collective.
-__device__ __forceinline__ void sample_octet2(const GsBucket* const col[2], const GsBucket* const det[2], uint32_t bkt,
-                                              uint64_t csmix, const bool active[2], uint32_t code[2], uint64_t idx[2]) {
+// The octets of a warp may belong to graphs of different bkt, so the pass count is the warp's largest: every
+// lane runs the same passes and reaches every full-warp collective.
+__device__ __forceinline__ void sample_octet2(const GsBucket* const col[2], const GsBucket* const det[2],
+                                              const uint32_t bkt[2], const uint64_t csmix[2], const bool active[2],
+                                              uint32_t code[2], uint64_t idx[2]) {
   const uint32_t lane = lane_id(), sub = lane & 7u, oct = lane >> 3;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, max(bkt[0], bkt[1]));
   GsBucket d[2], b[2];
   bool decided[2];
 #pragma unroll
   for (int u = 0; u < 2; u++) {
     d[u] = active[u] ? ld_bucket_cg(det[u]) : GsBucket{0, 0};
-    b[u] = active[u] && sub < bkt ? ld_bucket_cg(col[u] + sub) : GsBucket{0, 0};
+    b[u] = active[u] && sub < bkt[u] ? ld_bucket_cg(col[u] + sub) : GsBucket{0, 0};
   }
 #pragma unroll
   for (int u = 0; u < 2; u++) {
@@ -128,20 +138,20 @@ __device__ __forceinline__ void sample_octet2(const GsBucket* const col[2], cons
     decided[u] = !active[u];
     if (active[u]) {
       if (d[u].alpha == 0 && d[u].gamma == 0) { code[u] = kZero; decided[u] = true; }
-      else if (is_good(d[u], csmix)) { code[u] = kGood; idx[u] = d[u].alpha; decided[u] = true; }
+      else if (is_good(d[u], csmix[u])) { code[u] = kGood; idx[u] = d[u].alpha; decided[u] = true; }
     }
   }
-  for (uint32_t j0 = 0; j0 < bkt; j0 += 8) {
+  for (uint32_t j0 = 0; j0 < most; j0 += 8) {
     if (__all_sync(0xffffffffu, decided[0] && decided[1])) break;
     const uint32_t j = j0 + sub;
     if (j0 > 0) {
 #pragma unroll
       for (int u = 0; u < 2; u++)
-        if (!decided[u] && j < bkt) b[u] = ld_bucket_cg(col[u] + j);
+        if (!decided[u] && j < bkt[u]) b[u] = ld_bucket_cg(col[u] + j);
     }
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      const uint32_t m = __ballot_sync(0xffffffffu, !decided[u] && j < bkt && is_good(b[u], csmix));
+      const uint32_t m = __ballot_sync(0xffffffffu, !decided[u] && j < bkt[u] && is_good(b[u], csmix[u]));
       const uint32_t mine = (m >> (8u * oct)) & 0xffu;
       const uint64_t a = __shfl_sync(0xffffffffu, b[u].alpha, mine ? 8u * oct + (uint32_t)(__ffs(mine) - 1) : lane);
       if (!decided[u] && mine) {
@@ -221,6 +231,11 @@ struct BorArgs {
   GsBorTenant t0;
   const uint32_t* qlist;       // cluster scope with a table: the tenant of every cluster
   uint32_t tenant;             // grid scope with a table: the tenant
+  uint32_t T1;                 // grid scope over several graphs: entries of the tables, else 0
+  const uint32_t* vtenant;     //   tenant of every vertex
+  uint32_t vlo, vhi;           //   the graphs' vertices lie in [vlo, vhi)
+  uint32_t* tmod;              //   [2][T1] the round was modified, zero at launch
+  unsigned long long* tlargest;  // [2][T1] (size << 32) | ~root of the largest component, zero at launch
   uint32_t W;                  // accumulator row width, >= bkt_per_col + 1
   uint32_t R;                  // ring row width: the launch's largest bkt_per_col + 1
   uint32_t* parent;            // per vertex: DSU parent (vertex ids of the whole vertex space)
@@ -305,10 +320,22 @@ __device__ __forceinline__ void unite(const Graph& G, uint64_t e, uint32_t* s_ho
   if (G.edge) G.edge[hooked] = e;
 }
 
+// Several graphs in one launch over one vertex range: a flag per graph says that its round was modified.  It
+// is read before it is written: thousands of unions of one graph's round would queue on its line otherwise.
+__device__ __forceinline__ void mark(uint32_t* flag) {
+  if (!ld_volatile(flag)) *reinterpret_cast<volatile uint32_t*>(flag) = 1u;
+}
+__device__ __forceinline__ void unite_many(const BorArgs& A, const Graph& G, uint64_t e, uint32_t* tmod) {
+  if (e == ~0ull) return;
+  const uint32_t hooked = cached_union(G.parent, (uint32_t)(e >> 32), (uint32_t)e, G.span + 64, G.err);
+  if (hooked != 0xffffffffu) mark(tmod + A.vtenant[hooked]);
+}
+
 // Round 0: every vertex samples its own sketch, an octet of lanes for two; the edges of `per` passes are
 // collected one per lane and unioned together.
-__device__ __forceinline__ void round_zero(const Graph& G, const GsBucket* sk, const GsBorTenant& T, uint32_t gwarp,
-                                           uint32_t gwarps, uint32_t* s_mod, uint32_t* s_hooked) {
+__device__ __forceinline__ void round_zero(const Graph& G, const GsBucket* sk, const GsBorTenant& T, uint32_t* rank,
+                                           bool complement, uint32_t gwarp, uint32_t gwarps, uint32_t* s_mod,
+                                           uint32_t* s_hooked) {
   const uint32_t lane = lane_id(), span = G.span;
   const uint32_t per = min(4u, max(1u, (span + 8 * gwarps - 1) / (8 * gwarps)));
   for (uint32_t base = gwarp * 8 * per; base < span; base += gwarps * 8 * per) {
@@ -319,6 +346,8 @@ __device__ __forceinline__ void round_zero(const Graph& G, const GsBucket* sk, c
       bool active[2];
       uint32_t code[2];
       uint64_t idx[2];
+      const uint32_t bkt[2] = {T.bkt, T.bkt};
+      const uint64_t csmix[2] = {T.csmix, T.csmix};
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const uint32_t k = base + 8 * i + 4 * u + (lane >> 3);
@@ -327,10 +356,12 @@ __device__ __forceinline__ void round_zero(const Graph& G, const GsBucket* sk, c
         col[u] = own + (size_t)T.round0_col * T.bkt;
         det[u] = own + (T.nb - 1);
       }
-      sample_octet2(col, det, T.bkt, T.csmix, active, code, idx);
+      sample_octet2(col, det, bkt, csmix, active, code, idx);
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         failed |= active[u] && code[u] == kFail;
+        if (active[u] && (lane & 7u) == 0)
+          rank[G.vlo + base + 8 * i + 4 * u + (lane >> 3)] = complement && code[u] == kZero ? kClosed : 0u;
         const uint64_t e = active[u] && code[u] == kGood ? edge_of(G, idx[u]) : ~0ull;
         const uint64_t x = __shfl_sync(0xffffffffu, e, (lane & 3u) * 8u);
         if ((lane >> 2) == 2 * i + u) mine = x;
@@ -338,6 +369,47 @@ __device__ __forceinline__ void round_zero(const Graph& G, const GsBucket* sk, c
     }
     if (failed) *s_mod = 1;
     unite(G, mine, s_hooked);
+  }
+}
+
+// The same for several graphs over one vertex range: octets of different graphs share a warp.
+__device__ __forceinline__ void round_zero_many(const BorArgs& A, const Graph& G, const uint8_t* s_state,
+                                                uint32_t gwarp, uint32_t gwarps) {
+  const uint32_t lane = lane_id(), span = G.span;
+  for (uint32_t base = gwarp * 32; base < span; base += gwarps * 32) {
+    uint64_t mine = ~0ull;
+    for (uint32_t i = 0; i < 4; i++) {
+      const GsBucket *col[2], *det[2];
+      bool active[2];
+      uint32_t code[2], bkt[2], t[2], vbase[2], V[2];
+      uint64_t idx[2], csmix[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const uint32_t k = base + 8 * i + 4 * u + (lane >> 3);
+        t[u] = k < span ? A.vtenant[G.vlo + k] : 0u;
+        active[u] = k < span && s_state[t[u]] == 0;
+        const GsBorTenant& T = A.tenants[t[u]];
+        const GsBucket* own = A.sk + T.sk_off + (active[u] ? (size_t)(G.vlo + k - T.vbase) * T.nb : (size_t)0);
+        bkt[u] = active[u] ? T.bkt : 0u;
+        csmix[u] = T.csmix;
+        vbase[u] = T.vbase;
+        V[u] = T.V;
+        col[u] = own + (size_t)T.round0_col * T.bkt;
+        det[u] = own + (T.nb - 1);
+      }
+      sample_octet2(col, det, bkt, csmix, active, code, idx);
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        uint64_t e = ~0ull;
+        if (active[u] && code[u] == kFail) mark(A.tmod + t[u]);
+        if (active[u] && (lane & 7u) == 0)
+          A.rank[G.vlo + base + 8 * i + 4 * u + (lane >> 3)] = A.complement && code[u] == kZero ? kClosed : 0u;
+        if (active[u] && code[u] == kGood) e = edge_of(Graph{vbase[u], V[u], nullptr, nullptr, nullptr}, idx[u]);
+        const uint64_t x = __shfl_sync(0xffffffffu, e, (lane & 3u) * 8u);
+        if ((lane >> 2) == 2 * i + u) mine = x;
+      }
+    }
+    unite_many(A, G, mine, A.tmod);
   }
 }
 
@@ -384,11 +456,16 @@ __device__ __forceinline__ unsigned long long block_scan(unsigned long long x, u
 
 // SLOTS: buckets of a row (bkt_per_col + 1) per lane; at most 64 registers in either scope.  Dynamic shared
 // memory: kRing rows of R buckets per warp.
-template <int SCOPE, int SLOTS>
-__global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k_boruvka(const BorArgs A) {
+// MANY (grid scope): the launch's graphs are the tenants whose tstate word 0 is zero; their vertices lie among
+// others' in one range, their rounds advance together, and a graph whose round was unmodified stops taking
+// part, so each one's partition, round count and out-of-samples status equal a query run alone.  Two more
+// tables in dynamic shared memory: every tenant's complement component and state.
+template <int SCOPE, int SLOTS, bool MANY = false>
+__global__ void __launch_bounds__(threads_of(SCOPE, MANY), SCOPE == kNarrow ? 2 : 1) k_boruvka(const BorArgs A) {
+  static_assert(!MANY || SCOPE == kGrid, "several graphs share a launch on clusters or on the whole grid");
   constexpr bool CLUSTER = SCOPE != kGrid;
-  constexpr uint32_t kThreads = threads_of(SCOPE), kWarps = kThreads / 32;
-  constexpr uint32_t kTable = 2 * kThreads;        // slots of a block's table of roots
+  constexpr uint32_t kThreads = threads_of(SCOPE, MANY), kWarps = kThreads / 32;
+  constexpr uint32_t kTable = CLUSTER ? 1024 : 2048;   // slots of a block's table of roots, at most kThreads of them
   extern __shared__ __align__(16) GsBucket s_ring[];
   __shared__ BorCounters s_ctr[2];                 // cluster scope: the first block's are the cluster's
   __shared__ uint32_t s_row[4][SLOTS * 32];        // the block's share of the largest component's row
@@ -411,9 +488,12 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
     ctr = A.ctr;
     t = A.tenant;
   }
-  const GsBorTenant T = A.tenants ? A.tenants[t] : A.t0;
-  const uint32_t vlo = T.vbase, span = T.V, vend = T.vbase + T.V;
-  const uint32_t bkt = T.bkt, W = A.W, R = A.R;
+  const GsBorTenant T = A.tenants ? A.tenants[t] : A.t0;   // MANY: not used
+  const uint32_t vlo = MANY ? A.vlo : T.vbase, vend = MANY ? A.vhi : T.vbase + T.V, span = vend - vlo;
+  const uint32_t W = A.W, R = A.R;
+  uint32_t bkt = T.bkt;                                    // MANY: of the component at hand
+  uint32_t* const s_comp = reinterpret_cast<uint32_t*>(s_ring + (size_t)kWarps * kRing * R);   // MANY: [T1]
+  uint8_t* const s_state = reinterpret_cast<uint8_t*>(s_comp + A.T1);   // MANY: [T1] 0 running, 1 done, 2 last round
   const uint32_t gtid = block * kThreads + threadIdx.x, gthreads = blocks * kThreads;
   const uint32_t gwarp = gtid >> 5, gwarps = gthreads >> 5;
   const uint32_t limit = span + 64;
@@ -462,15 +542,43 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
     for (int i = 0; i < 16; i++) A.status[i] = 0;
   }
   if (!meet(nullptr)) return;
-  uint32_t rounds = 0, oos = T.round0_col >= T.ns;   // OutOfSamplesException before the first round
-
-  if (!oos) round_zero(G, sk, T, gwarp, gwarps, &s_mod, &s_hooked);
+  uint32_t rounds = 0, oos = MANY ? 0 : T.round0_col >= T.ns;   // OutOfSamplesException before the first round
+  if constexpr (MANY) {
+    for (uint32_t i = threadIdx.x; i < A.T1; i += kThreads) s_state[i] = A.tstate[4 * i] ? 1 : 0;
+    __syncthreads();
+    round_zero_many(A, G, s_state, gwarp, gwarps);
+  } else {
+    if (!oos) round_zero(G, sk, T, A.rank, A.complement, gwarp, gwarps, &s_mod, &s_hooked);
+  }
 
   for (uint32_t round = 0; !oos || round;) {
-    if (!meet(&ctr[round & 1].modified)) return;
-    if (!ld_volatile(&ctr[round & 1].modified)) break;
-    rounds = ++round;
-    oos = rounds >= T.ns;
+    if constexpr (MANY) {
+      if (!meet(nullptr)) return;
+      // every block decides the same from the same flags
+      bool some = false;
+      for (uint32_t i = threadIdx.x; i < A.T1; i += kThreads) {
+        if (s_state[i] == 2) s_state[i] = 1;
+        if (s_state[i]) continue;
+        if (!ld_volatile(&A.tmod[(round & 1) * A.T1 + i])) {
+          s_state[i] = 1;
+          continue;
+        }
+        some = true;
+        const bool last = round + 1 >= A.tenants[i].ns;   // out of samples: only the labels are still compressed
+        if (last) s_state[i] = 2;
+        if (block == 0) {
+          A.tstate[4 * i + 2] = round + 1;
+          A.tstate[4 * i + 3] = last;
+        }
+      }
+      if (!__syncthreads_or(some)) break;
+      ++round;
+    } else {
+      if (!meet(&ctr[round & 1].modified)) return;
+      if (!ld_volatile(&ctr[round & 1].modified)) break;
+      rounds = ++round;
+      oos = rounds >= T.ns;
+    }
     BorCounters* const c = ctr + (round & 1);
 
     // ---- compress, sizes, ranks, largest.  A block counts the members of every root among 1024 vertices
@@ -485,7 +593,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       __syncthreads();
       const uint32_t v = vlo + base + threadIdx.x;
       uint32_t r = 0xffffffffu;
-      if (v < vend) {
+      if (v < vend && (!MANY || s_state[A.vtenant[v]] != 1) && !(A.complement && __ldcg(&A.rank[v]) == kClosed)) {
         r = cached_root(A.parent, v, limit, err);
         A.parent[v] = r;
       }
@@ -493,7 +601,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       const uint32_t lead = __ffs(peers) - 1;
       uint32_t h = 0, local = 0;
       if (r != 0xffffffffu && lane == lead) {
-        h = __umulhi(r * 0x9E3779B1u, kTable);   // at most kThreads roots: half full
+        h = __umulhi(r * 0x9E3779B1u, kTable);   
         for (;;) {
           const uint32_t k = atomicCAS(&s_key[h], 0xffffffffu, r);
           if (k == 0xffffffffu || k == r) break;
@@ -509,7 +617,11 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
         s_cnt[i] = old;
         // the last block to add to a component sees its full size
         const unsigned long long key = ((unsigned long long)(old + n) << 32) | (0xffffffffu - root);
-        best = key > best ? key : best;
+        if constexpr (MANY) {
+          if (old + n > 1) atomicMax(&A.tlargest[(round & 1) * A.T1 + A.vtenant[root]], key);
+        } else {
+          best = key > best ? key : best;
+        }
       }
       __syncthreads();
       if (r != 0xffffffffu && lane == lead) local += s_cnt[h];
@@ -517,21 +629,42 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       if (r != 0xffffffffu) A.rank[v] = local + __popc(peers & ((1u << lane) - 1u));
       __syncthreads();
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
-      best = other > best ? other : best;
-    }
-    if (lane == 0 && best) atomicMax(&s_best, best);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      if (s_best) atomicMax(&c->largest, s_best);
-      s_best = 0;
+    if constexpr (!MANY) {
+      for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other > best ? other : best;
+      }
+      if (lane == 0 && best) atomicMax(&s_best, best);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        if (s_best) atomicMax(&c->largest, s_best);
+        s_best = 0;
+      }
     }
     if (!meet(nullptr)) return;
     if (oos) break;   // the labels are compressed
-    const uint64_t top = ld_volatile64(&c->largest);
     // the component whose column is the XOR of everything outside it, or ~0: none
-    const uint32_t comp = A.complement && (top >> 32) > 1ull ? 0xffffffffu - (uint32_t)top : 0xffffffffu;
+    uint32_t comp = 0xffffffffu;
+    if constexpr (MANY) {
+      for (uint32_t i = threadIdx.x; i < A.T1; i += kThreads) {
+        const uint64_t top = ld_volatile64(&A.tlargest[(round & 1) * A.T1 + i]);
+        s_comp[i] = A.complement && s_state[i] == 0 && (top >> 32) > 1ull ? 0xffffffffu - (uint32_t)top : 0xffffffffu;
+      }
+      __syncthreads();
+    } else {
+      const uint64_t top = ld_volatile64(&c->largest);
+      if (A.complement && (top >> 32) > 1ull) comp = 0xffffffffu - (uint32_t)top;
+    }
+    // sizes that count: not those of the complement components, nor of graphs that are out of samples
+    const auto listed = [&](uint32_t v, uint32_t size) -> uint32_t {
+      if constexpr (MANY) {
+        if (!size) return 0u;
+        const uint32_t i = A.vtenant[v];
+        return s_state[i] == 0 && v != s_comp[i] ? size : 0u;
+      } else {
+        return v == comp ? 0u : size;
+      }
+    };
 
     // ---- allocate: member runs and tasks, one reservation per block; runs and tasks come in one order ----
     {
@@ -541,7 +674,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       const uint32_t first = v0 + threadIdx.x < v1 ? __ldcg(&A.size[v0 + threadIdx.x]) : 0u;
       unsigned long long mine = 0, total;
       for (uint32_t v = v0 + threadIdx.x; v < v1; v += kThreads) {
-        const uint32_t n = v == comp ? 0u : v == v0 + threadIdx.x ? first : __ldcg(&A.size[v]);
+        const uint32_t n = listed(v, v == v0 + threadIdx.x ? first : __ldcg(&A.size[v]));
         mine += ((unsigned long long)n << 32) | ((n + kPiece - 1) / kPiece);
       }
       unsigned long long at = block_scan<kWarps>(mine, s_sums, &total);
@@ -551,7 +684,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       for (uint32_t vb = v0 + (threadIdx.x & ~31u); vb < v1; vb += kThreads) {
         const uint32_t v = vb + lane;
         const uint32_t size = v >= v1 ? 0u : v == v0 + threadIdx.x ? first : __ldcg(&A.size[v]);
-        const uint32_t n = v == comp ? 0u : size, pieces = (n + kPiece - 1) / kPiece;
+        const uint32_t n = v < v1 ? listed(v, size) : 0u, pieces = (n + kPiece - 1) / kPiece;
         const uint32_t start = (uint32_t)(at >> 32), task = (uint32_t)at;
         if (n) A.off[v] = start;
         if (pieces == 1) tasks[task] = make_uint4(v, start, n, 1u);
@@ -563,7 +696,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
           for (uint32_t p = lane; p < hp; p += 32)
             tasks[ht + p] = make_uint4(vb + src, h0 + p * kPiece, min(kPiece, hn - p * kPiece), hp);
         }
-        const bool is_big = size && (v == comp || pieces > 1);
+        const bool is_big = pieces > 1 || (size && (MANY ? v == s_comp[A.vtenant[v]] : v == comp));
         const uint32_t bm = __ballot_sync(0xffffffffu, is_big);
         if (bm) {
           uint32_t b = 0;
@@ -577,12 +710,29 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
 
     // ---- place the members; clear the sizes and the other counter set for the next round ----
     for (uint32_t v = vlo + gtid; v < vend; v += gthreads) {
-      const uint32_t r = __ldcg(&A.parent[v]);
-      if (r != comp) list[__ldcg(&A.off[r]) + __ldcg(&A.rank[v])] = v;
+      uint32_t out_of = comp;
+      if constexpr (MANY) {
+        const uint32_t i = A.vtenant[v];
+        if (s_state[i] == 1) continue;
+        if (s_state[i] == 2) {
+          A.size[v] = 0;
+          continue;
+        }
+        out_of = s_comp[i];
+      }
+      const uint32_t r = __ldcg(&A.parent[v]), rank = __ldcg(&A.rank[v]);
+      if (A.complement && rank == kClosed) continue;
+      if (r != out_of) list[__ldcg(&A.off[r]) + rank] = v;
       if (r == v) A.size[v] = 0;
     }
     if (gtid < sizeof(BorCounters) / sizeof(uint32_t))
       reinterpret_cast<volatile uint32_t*>(ctr + ((round + 1) & 1))[gtid] = 0;
+    if constexpr (MANY) {
+      for (uint32_t i = gtid; i < A.T1; i += gthreads) {
+        A.tmod[((round + 1) & 1) * A.T1 + i] = 0;
+        A.tlargest[((round + 1) & 1) * A.T1 + i] = 0;
+      }
+    }
     if (!meet(nullptr)) return;
 
     // ---- gather: each warp a run of tasks, whose members are one run of the list.  The members' rows
@@ -596,12 +746,28 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       uint64_t ma[SLOTS] = {}, mb[SLOTS] = {};      // pieces of one larger component
       uint32_t mroot = 0xffffffffu, held = 0;
       uint64_t mine = ~0ull;
+      // MANY: the graph that ca and cb belong to, its complement component and its row width
+      uint32_t ct = 0xffffffffu, crow = 0xffffffffu, cbkt = 0, mbkt = 0;
+      auto flush_complement = [&]() {
+        if (crow == 0xffffffffu) return;
+#pragma unroll
+        for (int k = 0; k < SLOTS; k++) {
+          const uint32_t j = lane + 32u * k;
+          if (j <= cbkt && (ca[k] | cb[k])) xor_row(A.acc + (size_t)crow * W, j, ca[k], cb[k]);
+          ca[k] = cb[k] = 0;
+        }
+      };
+      uint32_t* const tmod = MANY ? A.tmod + (round & 1) * A.T1 : nullptr;
+      auto join = [&](uint64_t e) {
+        if constexpr (MANY) unite_many(A, G, e, tmod);
+        else unite(G, e, &s_hooked);
+      };
       auto flush_pieces = [&]() {
         if (mroot == 0xffffffffu) return;
 #pragma unroll
         for (int k = 0; k < SLOTS; k++) {
           const uint32_t j = lane + 32u * k;
-          if (j <= bkt && (ma[k] | mb[k])) xor_row(A.acc + (size_t)mroot * W, j, ma[k], mb[k]);
+          if (j <= (MANY ? mbkt : bkt) && (ma[k] | mb[k])) xor_row(A.acc + (size_t)mroot * W, j, ma[k], mb[k]);
           ma[k] = mb[k] = 0;
         }
         mroot = 0xffffffffu;
@@ -610,35 +776,81 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
         const uint4 last = __ldcg(&tasks[t1 - 1]);
         const uint32_t m0 = __ldcg(&tasks[t0].y), total = last.y + last.z - m0;
         // lane l holds list entries l of the current and the next 32
-        uint32_t now = lane < total ? __ldcg(&list[m0 + lane]) : 0u;
-        uint32_t then = 32 + lane < total ? __ldcg(&list[m0 + 32 + lane]) : 0u;
+        uint32_t now = lane < total ? __ldcg(&list[m0 + lane]) : vlo;
+        uint32_t then = 32 + lane < total ? __ldcg(&list[m0 + 32 + lane]) : vlo;
         uint32_t next = 0;   // the member whose row is asked for next
+        // MANY: first bucket of lane l's member, and its graph's bkt << 16 | nb
+        uint64_t now_at = 0;
+        uint32_t now_geo = 0;
+        auto look_up = [&]() {
+          if constexpr (MANY) {
+            const GsBorTenant& M = A.tenants[A.vtenant[now]];
+            now_at = M.sk_off + (uint64_t)(now - M.vbase) * M.nb;
+            now_geo = (M.bkt << 16) | M.nb;
+          }
+        };
+        look_up();
         auto ask = [&]() {   // kGroup rows, one commit
 #pragma unroll
           for (uint32_t u = 0; u < kGroup; u++) {
-            const uint32_t v = __shfl_sync(0xffffffffu, now, (next + u) & 31u) - vlo;
+            const GsBucket* vb;
+            uint32_t b = bkt, nb = T.nb;
+            if constexpr (MANY) {
+              vb = A.sk + __shfl_sync(0xffffffffu, now_at, (next + u) & 31u);
+              const uint32_t geo = __shfl_sync(0xffffffffu, now_geo, (next + u) & 31u);
+              b = geo >> 16;
+              nb = geo & 0xffffu;
+            } else {
+              vb = sk + (size_t)(__shfl_sync(0xffffffffu, now, (next + u) & 31u) - vlo) * T.nb;
+            }
             if (next + u >= total) continue;
-            const GsBucket* vb = sk + (size_t)v * T.nb;
             GsBucket* to = ring + ((next + u) % kRing) * R;
 #pragma unroll
             for (int k = 0; k < SLOTS; k++) {
               const uint32_t j = lane + 32u * k;
-              if (j <= bkt) cp_async16(to + j, vb + (j < bkt ? round * bkt + j : T.nb - 1));
+              if (j <= b) cp_async16(to + j, vb + (j < b ? round * b + j : nb - 1));
             }
           }
           cp_async_commit();
           next += kGroup;
           if ((next & 31u) == 0) {
             now = then;
-            then = next + 32 + lane < total ? __ldcg(&list[m0 + next + 32 + lane]) : 0u;
+            look_up();
+            then = next + 32 + lane < total ? __ldcg(&list[m0 + next + 32 + lane]) : vlo;
           }
         };
         ask();
         ask();
         uint32_t done = 0;
         uint4 batch = make_uint4(0, 0, 0, 0);
+        uint32_t batch_t = 0, batch_base = 0, batch_V = 0, batch_bkt = 0;   // MANY: the tasks' graphs
+        uint64_t batch_cs = 0, csmix = T.csmix;
+        Graph H = G;
         for (uint32_t tk = t0; tk < t1; tk++) {
-          if (((tk - t0) & 31u) == 0 && tk + lane < t1) batch = __ldcg(&tasks[tk + lane]);
+          if (((tk - t0) & 31u) == 0 && tk + lane < t1) {
+            batch = __ldcg(&tasks[tk + lane]);
+            if constexpr (MANY) {
+              batch_t = A.vtenant[batch.x];
+              const GsBorTenant& M = A.tenants[batch_t];
+              batch_base = M.vbase;
+              batch_V = M.V;
+              batch_bkt = M.bkt;
+              batch_cs = M.csmix;
+            }
+          }
+          if constexpr (MANY) {
+            const uint32_t src = (tk - t0) & 31u, tt = __shfl_sync(0xffffffffu, batch_t, src);
+            bkt = __shfl_sync(0xffffffffu, batch_bkt, src);
+            csmix = __shfl_sync(0xffffffffu, batch_cs, src);
+            H.vlo = __shfl_sync(0xffffffffu, batch_base, src);
+            H.span = __shfl_sync(0xffffffffu, batch_V, src);
+            if (tt != ct) {
+              flush_complement();
+              ct = tt;
+              crow = s_comp[tt];
+              cbkt = bkt;
+            }
+          }
           const uint32_t root = __shfl_sync(0xffffffffu, batch.x, (tk - t0) & 31u);
           const uint32_t n = __shfl_sync(0xffffffffu, batch.z, (tk - t0) & 31u);
           const uint32_t pieces = __shfl_sync(0xffffffffu, batch.w, (tk - t0) & 31u);
@@ -664,7 +876,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
               ask();
             }
           }
-          if (comp != 0xffffffffu) {
+          if ((MANY ? crow : comp) != 0xffffffffu) {
 #pragma unroll
             for (int k = 0; k < SLOTS; k++) { ca[k] ^= a[k]; cb[k] ^= g[k]; }
           }
@@ -672,6 +884,7 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
             if (root != mroot) {
               flush_pieces();
               mroot = root;
+              mbkt = bkt;
             }
 #pragma unroll
             for (int k = 0; k < SLOTS; k++) { ma[k] ^= a[k]; mb[k] ^= g[k]; }
@@ -687,38 +900,43 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
               da = __shfl_sync(0xffffffffu, a[k], bkt & 31u);
               dg = __shfl_sync(0xffffffffu, g[k], bkt & 31u);
             }
-            good[k] = __ballot_sync(0xffffffffu, j <= bkt && is_good(GsBucket{a[k], g[k]}, T.csmix));
+            good[k] = __ballot_sync(0xffffffffu, j <= bkt && is_good(GsBucket{a[k], g[k]}, csmix));
             if (bkt / 32u == (uint32_t)k) det_good = (good[k] >> (bkt & 31u)) & 1u;
           }
           uint64_t e = ~0ull;
-          if ((da | dg) != 0ull) {
+          if ((da | dg) == 0ull) {
+            // no edge out, now or later: its members are not looked at again
+            if (A.complement && lane < n) A.rank[__ldcg(&list[m0 + done - n + lane])] = kClosed;
+          } else {
             uint32_t at = 0xffffffffu;   // the first good depth, but the deterministic bucket before any
 #pragma unroll
             for (int k = SLOTS - 1; k >= 0; k--)
               if (good[k]) at = 32u * k + (__ffs(good[k]) - 1);
             if (det_good) at = bkt;
-            if (at == 0xffffffffu) {
-              s_mod = 1;                 // FAIL
+            if (at == 0xffffffffu) {     // FAIL
+              if constexpr (MANY) mark(tmod + ct);
+              else s_mod = 1;
             } else {
               uint64_t idx = 0;
 #pragma unroll
               for (int k = 0; k < SLOTS; k++)
                 if (at / 32u == (uint32_t)k) idx = __shfl_sync(0xffffffffu, a[k], at & 31u);
-              e = edge_of(G, idx);
+              e = edge_of(H, idx);
             }
           }
           if (lane == held) mine = e;
           if (++held == 32) {
-            unite(G, mine, &s_hooked);
+            join(mine);
             __syncwarp();
             mine = ~0ull;
             held = 0;
           }
         }
-        if (held) unite(G, mine, &s_hooked);
+        if (held) join(mine);
         flush_pieces();
+        if constexpr (MANY) flush_complement();
       }
-      if (comp != 0xffffffffu) {
+      if (!MANY && comp != 0xffffffffu) {
         // one warp's row at a time would queue on the row's L2 lines: combined per block first
         if (t0 < t1) {
 #pragma unroll
@@ -750,14 +968,28 @@ __global__ void __launch_bounds__(threads_of(SCOPE), SCOPE == kNarrow ? 2 : 1) k
       GsBucket* row = A.acc + (size_t)r * W;
       uint32_t code;
       uint64_t idx;
-      sample_warp(row, row + bkt, bkt, T.csmix, &code, &idx);
-      if (code == kFail) s_mod = 1;
-      __syncwarp();
-      for (uint32_t j = lane; j <= bkt; j += 32) row[j] = GsBucket{0, 0};
-      unite(G, lane == 0 && code == kGood ? edge_of(G, idx) : ~0ull, &s_hooked);
+      if constexpr (MANY) {
+        const uint32_t i = A.vtenant[r];
+        const GsBorTenant& M = A.tenants[i];
+        const uint32_t b = M.bkt;
+        sample_warp(row, row + b, b, M.csmix, &code, &idx);
+        if (code == kFail) mark(A.tmod + (round & 1) * A.T1 + i);
+        __syncwarp();
+        for (uint32_t j = lane; j <= b; j += 32) row[j] = GsBucket{0, 0};
+        if (lane == 0 && code == kGood)
+          unite_many(A, G, edge_of(Graph{M.vbase, M.V, nullptr, nullptr, nullptr}, idx), A.tmod + (round & 1) * A.T1);
+        __syncwarp();
+      } else {
+        sample_warp(row, row + bkt, bkt, T.csmix, &code, &idx);
+        if (code == kFail) s_mod = 1;
+        __syncwarp();
+        for (uint32_t j = lane; j <= bkt; j += 32) row[j] = GsBucket{0, 0};
+        unite(G, lane == 0 && code == kGood ? edge_of(G, idx) : ~0ull, &s_hooked);
+      }
     }
   }
 
+  if constexpr (MANY) return;
   if (gtid == 0) { ts[0] = 1; ts[2] = rounds; ts[3] = oos; }
   if (A.out) write_answer(A, G, gtid, gthreads, meet);
   // the first block's counters stay until every block has read them
@@ -817,7 +1049,7 @@ __global__ void __launch_bounds__(threads_of(kWide), 1) k_boruvka_flat(const Bor
   }
   meet(nullptr);
   uint32_t rounds = 0, oos = T.round0_col >= T.ns;
-  if (!oos) round_zero(G, sk, T, gwarp, gwarps, &s_mod, &s_hooked);
+  if (!oos) round_zero(G, sk, T, A.rank, A.complement, gwarp, gwarps, &s_mod, &s_hooked);
 
   for (uint32_t round = 0; !oos || round;) {
     meet(flag + (round & 1));
@@ -833,14 +1065,18 @@ __global__ void __launch_bounds__(threads_of(kWide), 1) k_boruvka_flat(const Bor
       uint64_t a[SLOTS] = {}, g[SLOTS] = {};
       for (uint32_t base = gwarp * take; base < span; base += gwarps * take) {
         const uint32_t n = min(take, span - base);
-        uint32_t r = 0;
+        uint32_t r = 0xffffffffu;
         if (lane < n) {
           const uint32_t v = vlo + base + lane;
-          r = cached_root(A.parent, v, limit, A.status);
-          A.parent[v] = r;
+          const bool closed = A.complement && __ldcg(&A.rank[v]) == kClosed;
+          if (!closed) {
+            r = cached_root(A.parent, v, limit, A.status);
+            A.parent[v] = r;
+          }
           A.size[v] = r == v;   // the roots that sample: a union of the sample phase may hook one before its turn
         }
         if (oos) continue;   // only the labels are still wanted
+        const uint32_t open = __ballot_sync(0xffffffffu, r != 0xffffffffu);
         GsBucket b[kTake][SLOTS];
 #pragma unroll
         for (uint32_t u = 0; u < kTake; u++) {
@@ -848,12 +1084,12 @@ __global__ void __launch_bounds__(threads_of(kWide), 1) k_boruvka_flat(const Bor
 #pragma unroll
           for (int k = 0; k < SLOTS; k++) {
             const uint32_t j = lane + 32u * k;
-            b[u][k] = u < n && j <= bkt ? ld_bucket_cg(vb + (j < bkt ? round * bkt + j : T.nb - 1)) : GsBucket{0, 0};
+            b[u][k] = ((open >> u) & 1u) && j <= bkt ? ld_bucket_cg(vb + (j < bkt ? round * bkt + j : T.nb - 1)) : GsBucket{0, 0};
           }
         }
 #pragma unroll
         for (uint32_t u = 0; u < kTake; u++) {
-          if (u >= n) break;
+          if (!((open >> u) & 1u)) continue;
           const uint32_t root = __shfl_sync(0xffffffffu, r, u);
           if (root != cur) {
             if (cur != 0xffffffffu) {
@@ -968,34 +1204,34 @@ __global__ void __launch_bounds__(256) k_forest(const uint32_t* __restrict__ par
   }
 }
 
-template <int SCOPE, int SLOTS>
+template <int SCOPE, int SLOTS, bool MANY>
 constexpr auto kernel_of() {
   if constexpr (SCOPE == kWide) return k_boruvka_flat<SLOTS>;
-  else return k_boruvka<SCOPE, SLOTS>;
+  else return k_boruvka<SCOPE, SLOTS, MANY>;
 }
 
-size_t dynamic_bytes(int scope, uint32_t R) {
-  return (size_t)(threads_of(scope) / 32) * (scope == kWide ? 1 : kRing) * R * sizeof(GsBucket);
+size_t dynamic_bytes(int scope, uint32_t R, uint32_t T1) {
+  return (size_t)(threads_of(scope, T1 != 0) / 32) * (scope == kWide ? 1 : kRing) * R * sizeof(GsBucket) + 5 * (size_t)T1;
 }
 
 // Launches of more than 48 KB of dynamic shared memory, and clusters of more than 8 blocks, are opted into
 // per device and kernel; what was opted into is remembered per host thread.
-template <int SCOPE, int SLOTS>
+template <int SCOPE, int SLOTS, bool MANY = false>
 gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s) {
-  struct Opted { uint32_t R = 0, blocks = 0; int sms = 0; };
+  struct Opted { size_t smem = 0; uint32_t blocks = 0; int sms = 0; };
   static thread_local Opted opted[64];
-  constexpr auto kernel = kernel_of<SCOPE, SLOTS>();
+  constexpr auto kernel = kernel_of<SCOPE, SLOTS, MANY>();
   int dev = 0;
   GS_CUDA_TRY(cudaGetDevice(&dev));
   Opted& o = opted[dev & 63];
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  cfg.blockDim = dim3(threads_of(SCOPE));
-  cfg.dynamicSmemBytes = dynamic_bytes(SCOPE, L.R);
+  cfg.blockDim = dim3(threads_of(SCOPE, MANY));
+  cfg.dynamicSmemBytes = dynamic_bytes(SCOPE, L.R, MANY ? L.T1 : 0);
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (o.R < L.R) {
+  if (o.smem < cfg.dynamicSmemBytes) {
     GS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
     GS_CUDA_TRY(cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev));
     o.blocks = 8;
@@ -1011,7 +1247,7 @@ gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s)
         o.blocks = 16;
       cudaGetLastError();
     }
-    o.R = L.R;
+    o.smem = cfg.dynamicSmemBytes;
   }
   if (SCOPE != kGrid) {
     const uint32_t blocks = std::min(L.scope.blocks, o.blocks);
@@ -1026,6 +1262,7 @@ gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s)
     attr[0].val.cooperative = 1;
     cfg.gridDim = dim3(o.sms);
     GS_CUDA_TRY(cudaMemsetAsync(A.ctr, 0, kGsBorCounterWords * sizeof(uint32_t), s));
+    if (MANY) GS_CUDA_TRY(cudaMemsetAsync(L.many, 0, gs_boruvka_many_bytes(L.T1), s));
   }
   GS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, A));
   return GS_OK;
@@ -1033,6 +1270,7 @@ gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s)
 
 template <int SLOTS>
 gs_status launch_scope(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s) {
+  if (L.T1) return launch_boruvka<kGrid, SLOTS, true>(A, L, s);
   if (!L.scope.blocks) return launch_boruvka<kGrid, SLOTS>(A, L, s);
   return L.scope.wide ? launch_boruvka<kWide, SLOTS>(A, L, s) : launch_boruvka<kNarrow, SLOTS>(A, L, s);
 }
@@ -1048,6 +1286,12 @@ gs_status gs_boruvka_launch(const GsBorLaunch& L, cudaStream_t s) {
   A.t0 = L.t0;
   A.qlist = L.qlist;
   A.tenant = L.tenant;
+  A.T1 = L.T1;
+  A.vtenant = L.vtenant;
+  A.vlo = L.vlo;
+  A.vhi = L.vhi;
+  A.tlargest = static_cast<unsigned long long*>(L.many);
+  A.tmod = reinterpret_cast<uint32_t*>(A.tlargest + 2 * (size_t)L.T1);
   A.W = L.W;
   A.R = L.R;
   A.parent = L.parent;
@@ -1120,7 +1364,7 @@ gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, c
   L.t0.round0_col = round0_col;
   L.t0.csmix = gs_seed_mix(g->seed);
   // a handle with a wait limit of its own keeps the scope whose waits have one
-  if (g->wait_ns == kGsDefaultWaitNs) L.scope = gs_boruvka_scope(V, 1);
+  if (g->wait_ns == kGsDefaultWaitNs) L.scope = gs_boruvka_scope(V);
   L.vertices = V;
   L.W = L.R = bkt + 1;
   L.parent = g->d_parent;
@@ -1148,13 +1392,35 @@ gs_status gs_boruvka_enqueue(gs_graph* g, uint32_t level, uint32_t round0_col, c
 
 // One graph: a cluster has 16 SMs and the hardware's barrier, the grid all of them and a barrier of about
 // 1.5 us; the two meet above 8192 vertices (us per query call, cluster / grid: V = 1024 88 / 178, 4096
-// 109 / 165, 8192 184 / 220, 16384 285 / 207).  Several graphs: clusters side by side.  Up to 18 graphs get
-// wide ones (8 graphs of up to 65536 vertices: 0.42 ms against 0.62 with narrow ones); of more, the rows
-// fall out of L2, so members are listed, on smaller clusters (256 graphs of up to 16384 vertices, narrow:
-// 1.57 ms with 2 blocks each, 1.08 with 4, 1.54 with 8; wide: 2.1 at best).
-GsBorScope gs_boruvka_scope(uint32_t V, uint32_t graphs) {
-  if (graphs == 1) return V <= 8192 ? GsBorScope{16, true} : GsBorScope{};
-  return graphs <= 18 ? GsBorScope{16, true} : GsBorScope{graphs > 36 ? 4u : 8u, false};
+// 109 / 165, 8192 184 / 220, 16384 285 / 207).
+GsBorScope gs_boruvka_scope(uint32_t V) { return V <= 8192 ? GsBorScope{16, true} : GsBorScope{}; }
+
+// Several graphs of at most kGsBorClusterV vertices, clusters side by side: the scope of the least estimated
+// time.  A graph of V vertices takes about a + b V / blocks us on its cluster (wide: a = 120, b = 0.19;
+// narrow: a = 170, b = 0.32, measured on R-MAT and Erdos-Renyi tenants of 256 to 65536 vertices), 148 wide or
+// 296 narrow blocks run at once, and the launch ends with its largest graph.  Measured (ms per query, chosen /
+// best of all): 256 graphs of 256 to 16384 vertices 1.2 / 1.2, 40 of 1024 to 20000 0.89 / 0.89, 10 of 1024 to
+// 8192 0.21 / 0.21.
+GsBorScope gs_boruvka_scope(const uint32_t* V, uint32_t graphs) {
+  double sum = 0, most = 0;
+  for (uint32_t i = 0; i < graphs; i++) {
+    sum += V[i];
+    most = std::max(most, (double)V[i]);
+  }
+  GsBorScope best;
+  double least = 1e300;
+  for (int wide = 0; wide < 2; wide++) {
+    const double a = wide ? 120 : 170, b = wide ? 0.19 : 0.32;
+    for (uint32_t blocks = 2; blocks <= 16; blocks *= 2) {
+      const double at_once = std::floor((wide ? 148.0 : 296.0) / blocks);
+      const double t = std::max(a + b * most / blocks, (a * graphs + b * sum / blocks) / at_once);
+      if (t < least) {
+        least = t;
+        best = GsBorScope{blocks, wide != 0};
+      }
+    }
+  }
+  return best;
 }
 
 gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, uint32_t* st) {

@@ -158,6 +158,7 @@ struct gs_engine {
   uint32_t* d_vtenant = nullptr; // [max_vertices]
   uint32_t* d_tstate = nullptr;  // [(max_tenants + 1) * 4] Boruvka per-tenant state
   uint32_t* h_tstate = nullptr;  // pinned mirror
+  void* d_many = nullptr;        // tables of a Boruvka launch over several large tenants
   uint32_t* d_qstatus = nullptr; // [16] Boruvka status words
   uint32_t* h_qstatus = nullptr; // pinned [16]
   uint32_t* d_q = nullptr;       // [3 * (max_tenants + 1)] query list, label offsets, query list by size
@@ -185,7 +186,7 @@ namespace {
 void free_engine(gs_engine* e) {
   if (!e) return;
   if (e->g) gs_free_graph(e->g);
-  cudaFree(e->d_ing); cudaFree(e->d_bor); cudaFree(e->d_vtenant); cudaFree(e->d_tstate);
+  cudaFree(e->d_ing); cudaFree(e->d_bor); cudaFree(e->d_vtenant); cudaFree(e->d_tstate); cudaFree(e->d_many);
   cudaFree(e->d_qstatus); cudaFree(e->d_q); cudaFree(e->d_ncc);
   for (auto& tb : e->tabs) {
     cudaFree(tb.d_off); cudaFree(tb.d_ten);
@@ -297,10 +298,7 @@ gs_status copy_slices(const gs_engine::SliceTables& tb, uint32_t ns, cudaStream_
   return GS_OK;
 }
 
-// Graphs too large for a cluster that a query still answers one after the other with the whole GPU.
-constexpr uint32_t kMaxGridQueries = 2;
-
-// Queues the multi-tenant Boruvka launch and the read-back of its results into pinned memory.
+// Queues the multi-tenant Boruvka launches and the read-back of its results into pinned memory.
 // The pinned query tables must not be read by queued work any more.
 gs_status enqueue_query(gs_engine* e, const QueryPlan& qp, const uint32_t* tenants, uint32_t count, cudaStream_t s) {
   gs_graph* g = e->g;
@@ -314,14 +312,18 @@ gs_status enqueue_query(gs_engine* e, const QueryPlan& qp, const uint32_t* tenan
   if (g->acc_dirty)
     GS_CUDA_TRY(cudaMemsetAsync(g->d_acc, 0, (size_t)e->max_vertices * e->W * sizeof(GsBucket), s));
   g->acc_dirty = true;
-  // one cluster per graph, the largest graphs first (the launch ends when the last cluster does); up to
-  // kMaxGridQueries graphs that would keep a cluster busy for longer get the whole GPU, one after the other
+  // the large graphs share the whole GPU, the others run on a cluster each, the largest first (a launch ends
+  // when its last cluster does)
   uint32_t* order = e->h_q + 2 * (size_t)T1;
   std::copy(tenants, tenants + count, order);
   std::stable_sort(order, order + count, [&](uint32_t a, uint32_t b) { return e->ten[a].V > e->ten[b].V; });
   uint32_t large = 0;
-  while (large < count && e->ten[order[large]].V > (count == 1 ? 8192u : 65536u)) large++;
-  if (large > kMaxGridQueries) large = 0;
+  while (large < count && e->ten[order[large]].V > (count == 1 ? 8192u : kGsBorClusterV)) large++;
+  if (large > 1) {
+    for (uint32_t t = 0; t < T1; t++) e->h_tstate[4 * t] = 1;
+    for (uint32_t i = 0; i < large; i++) std::memset(e->h_tstate + 4 * order[i], 0, 4 * sizeof(uint32_t));
+    GS_CUDA_TRY(cudaMemcpyAsync(e->d_tstate, e->h_tstate, (size_t)T1 * 4 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  }
   GS_CUDA_TRY(cudaMemsetAsync(e->d_qstatus, 0, 16 * sizeof(uint32_t), s));
   GS_CUDA_TRY(cudaMemcpyAsync(e->d_q, e->h_q, (size_t)3 * T1 * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   GS_CUDA_TRY(cudaMemsetAsync(e->d_ncc, 0, (size_t)count * sizeof(uint32_t), s));
@@ -343,16 +345,30 @@ gs_status enqueue_query(gs_engine* e, const QueryPlan& qp, const uint32_t* tenan
   // tenants only take edge records, which reach both endpoints: every tenant's sketches XOR to zero
   L.complement = 1;
   {
-    GsProfScope ps(g, GS_PROF_QUERY, s, large + (large < count) + 1);
-    for (uint32_t i = 0; i < large; i++) {
-      L.tenant = order[i];
+    GsProfScope ps(g, GS_PROF_QUERY, s, (large > 0) + (large < count) + 1);
+    if (large) {
+      if (large == 1) {
+        L.tenant = order[0];
+      } else {
+        L.T1 = T1;
+        L.vtenant = e->d_vtenant;
+        L.many = e->d_many;
+        L.vlo = 0xffffffffu;
+        for (uint32_t i = 0; i < large; i++) {
+          const EngTenant& t = e->ten[order[i]];
+          L.vlo = std::min(L.vlo, t.vbase);
+          L.vhi = std::max(L.vhi, t.vbase + t.V);
+        }
+      }
       GS_TRY(gs_boruvka_launch(L, s));
+      L.T1 = 0;
     }
     if (large < count) {
       L.count = count - large;
       L.qlist = e->d_q + 2 * (size_t)T1 + large;
-      L.scope = gs_boruvka_scope(e->ten[order[large]].V, L.count);
-      if (!L.scope.blocks) L.scope = GsBorScope{16, true};   // one graph left
+      std::vector<uint32_t> V(L.count);
+      for (uint32_t i = 0; i < L.count; i++) V[i] = e->ten[order[large + i]].V;
+      L.scope = gs_boruvka_scope(V.data(), L.count);
       GS_TRY(gs_boruvka_launch(L, s));
     }
     const dim3 grid((unsigned)std::min<uint64_t>((qp.maxv + 255) / 256, 64), count);
@@ -490,6 +506,7 @@ gs_status gs_engine_create(const gs_engine_config* cfg, gs_engine** out) {
   GS_CUDA_TRY(cudaGetLastError());
   GS_CUDA_TRY(cudaMalloc(&e->d_tstate, (size_t)T1 * 4 * sizeof(uint32_t)));
   GS_CUDA_TRY(cudaMallocHost(&e->h_tstate, (size_t)T1 * 4 * sizeof(uint32_t)));
+  GS_CUDA_TRY(cudaMalloc(&e->d_many, gs_boruvka_many_bytes(T1)));
   GS_CUDA_TRY(cudaMalloc(&e->d_qstatus, 32 * sizeof(uint32_t)));
   GS_CUDA_TRY(cudaMallocHost(&e->h_qstatus, 16 * sizeof(uint32_t)));
   GS_CUDA_TRY(cudaMalloc(&e->d_q, (size_t)3 * T1 * sizeof(uint32_t)));

@@ -282,6 +282,11 @@ struct GsBorLaunch {
   uint32_t count = 1;                    // graphs (cluster scope)
   const uint32_t* qlist = nullptr;       // device [count] tenants (cluster scope with a table)
   uint32_t tenant = 0;                   // the tenant (grid scope with a table)
+  uint32_t T1 = 0;                       // several graphs in grid scope: entries of the tenant tables; the
+                                         // graphs are those whose tstate word 0 is zero
+  const uint32_t* vtenant = nullptr;     //   device: tenant of every vertex
+  uint32_t vlo = 0, vhi = 0;             //   the graphs' vertices lie in [vlo, vhi)
+  void* many = nullptr;                  //   device scratch of gs_boruvka_many_bytes(T1)
   uint64_t vertices = 0;                 // length of the per-vertex arrays
   uint32_t W = 0;                        // accumulator row width
   uint32_t R = 0;                        // largest bkt_per_col + 1 of the launch's graphs
@@ -302,8 +307,12 @@ struct GsBorLaunch {
   uint32_t complement = 0;
 };
 
-// The scope of a query of `graphs` graphs of at most V vertices.
-GsBorScope gs_boruvka_scope(uint32_t V, uint32_t graphs);
+// The scope of a query of one graph of V vertices, and of several of at most kGsBorClusterV each.
+constexpr uint32_t kGsBorClusterV = 16384;
+GsBorScope gs_boruvka_scope(uint32_t V);
+GsBorScope gs_boruvka_scope(const uint32_t* V, uint32_t graphs);
+// Bytes of GsBorLaunch::many for tables of T1 tenants.
+inline size_t gs_boruvka_many_bytes(uint32_t T1) { return (size_t)T1 * 2 * (sizeof(uint64_t) + sizeof(uint32_t)); }
 // The Boruvka scratch of a handle over `vertices` vertices with accumulator rows of `width` buckets.
 gs_status gs_alloc_boruvka(gs_graph* g, uint64_t vertices, uint32_t width, bool forest);
 // The last query's last_forest_edges forest edges into g->d_forest (queued on s).
