@@ -94,9 +94,6 @@ gs_status order_after(gs_graph* g, cudaStream_t s) {
   return GS_OK;
 }
 
-// Host input moves in slices of at most 2^24 pairs.  Per phase the first copy and the last slice's
-// ingest overlap nothing and every slice carries a fixed ingest cost (about 0.5 ms at V = 2^17);
-// 2^24 balances the two (1 GiB phases: 202.6 ms per 8 phases at 2^25, 189.1 at 2^24, 211.9 at 2^23).
 // (src[i], dst[i]) -> pair i
 __global__ void k_interleave(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint2* __restrict__ out,
                              uint64_t n) {
@@ -104,21 +101,19 @@ __global__ void k_interleave(const uint32_t* __restrict__ a, const uint32_t* __r
     out[i] = make_uint2(a[i], b[i]);
 }
 
-// Host input moves through two staging slots of at most 2^25 pairs (256 MB each side): a slice's
-// copy overlaps the ingest of the previous slice, and larger slices carry the sketch update's fixed
-// per-launch cost (every touched vertex's rows merged once per launch) less often.
+// The most pairs in one staging slot (256 MB on each side); what a call asks for depends on its input.
 uint64_t staging_limit(const gs_graph* g) { return std::min<uint64_t>(g->max_batch_edges, 1ull << 25); }
 
 }  // namespace
 
-gs_status gs_ensure_pair_staging(gs_graph* g, uint64_t want) {
+gs_status gs_ensure_pair_staging(gs_graph* g, uint64_t want, bool host) {
   // the ring is sized for the largest host slice asked for so far (at least 2^20 pairs, a power of
   // two, at most the limit); small graphs fed small batches keep a small ring
   uint64_t target = 1ull << 20;
   while (target < want && target < staging_limit(g)) target <<= 1;
   target = std::min(target, staging_limit(g));
-  if (g->d_pairs && g->pairs_cap >= target) return GS_OK;
-  if (g->d_pairs) {
+  if (g->d_pairs && g->pairs_cap >= target && (g->h_pin || !host)) return GS_OK;
+  if (g->d_pairs && g->pairs_cap < target) {
     // growing: every copy into and every reader of the old slots must be done
     GS_CUDA_TRY(cudaStreamSynchronize(g->copy_stream));
     for (int i = 0; i < 2; i++) GS_CUDA_TRY(cudaEventSynchronize(g->ev_done[i]));
@@ -131,8 +126,6 @@ gs_status gs_ensure_pair_staging(gs_graph* g, uint64_t want) {
     g->d_file_pairs = nullptr;
     g->pairs_cap = 0;
   }
-  GS_CUDA_TRY(cudaMalloc(&g->d_pairs, 2 * target * 2 * sizeof(uint32_t)));
-  GS_CUDA_TRY(cudaMallocHost(&g->h_pin, 2 * target * 2 * sizeof(uint32_t)));
   if (!g->copy_stream) {
     GS_CUDA_TRY(cudaStreamCreateWithFlags(&g->copy_stream, cudaStreamNonBlocking));
     for (int i = 0; i < 2; i++) {
@@ -140,7 +133,11 @@ gs_status gs_ensure_pair_staging(gs_graph* g, uint64_t want) {
       GS_CUDA_TRY(cudaEventCreateWithFlags(&g->ev_done[i], cudaEventDisableTiming));
     }
   }
-  g->pairs_cap = target;
+  if (!g->d_pairs) {
+    GS_CUDA_TRY(cudaMalloc(&g->d_pairs, 2 * target * 2 * sizeof(uint32_t)));
+    g->pairs_cap = target;
+  }
+  if (host && !g->h_pin) GS_CUDA_TRY(cudaMallocHost(&g->h_pin, 2 * g->pairs_cap * 2 * sizeof(uint32_t)));
   return GS_OK;
 }
 
@@ -258,9 +255,22 @@ uint64_t gs_desired_updates_per_batch(const gs_graph* g) {
 namespace {
 
 // Host batches of at most this many records are read by the kernels where they lie in the page-locked ring
-// (us per call of 100 records: 27 with the copy, 12 without; the eager DSU's and the exact tier's passes read
-// them again).
+// instead of being copied on the copy stream, with two events and a wait around them (two batches of 100 records
+// and a query whose kernel writes the labels itself: 173 -> 115 us for both together); each of the few passes
+// over them reads at most 8 KB over PCIe.
 constexpr uint64_t kZeroCopyPairs = 1024;
+
+// Records in one slice of host input: 64 per vertex, rounded up to a power of two.  A slice's copy overlaps the
+// ingest of the one before, so small slices leave little to do when the last copy lands; but each slice merges
+// the rows of all vertices that it touches, and toggles that cancel are only found within one.  ms for 2^25 R-MAT
+// records and the query with slices of 2^22 / 2^23 / 2^24 / 2^25:
+//   V = 2^14: 5.55 / 5.65 / 5.91 / 6.31    V = 2^17: 6.33 / 6.25 / 6.67 / 7.40
+//   V = 2^18: 8.79 / 7.00 / 7.54 / 8.65    V = 2^20: 15.23 / 12.20 / 10.47 / 11.70
+uint64_t host_slice(const gs_graph* g) {
+  uint64_t m = 1ull << 22;
+  while (m < 64ull * g->V && m < (1ull << 24)) m <<= 1;
+  return m;
+}
 
 // Host input moves through the staging slots: slice k is copied on the copy stream into device slot
 // k % 2 (from the caller's memory when it is page-locked, else through the pinned ring) while the
@@ -269,7 +279,14 @@ constexpr uint64_t kZeroCopyPairs = 1024;
 // stays in use until the handle's work is done, and every wait on a slot's earlier slice happens on
 // the device, so copies of this call can run ahead of queries queued before it.
 gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cudaStream_t s, bool wait_copies) {
-  GS_TRY(gs_ensure_pair_staging(g, n));
+  bool pinned = false;
+  if (n > kZeroCopyPairs) {
+    cudaPointerAttributes attr{};
+    pinned = cudaPointerGetAttributes(&attr, pairs) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+  }
+  const uint64_t slice = host_slice(g);
+  GS_TRY(gs_ensure_pair_staging(g, std::min(n, slice), !pinned));
   if (n <= kZeroCopyPairs) {
     // a few records: copied into the ring by the host and read from there by the update's kernel, instead of
     // a copy on another stream and the two events and the wait that tie it to this one
@@ -283,13 +300,10 @@ gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cuda
     GS_CUDA_TRY(cudaEventRecord(g->ev_copy[slot], s));   // who waits for either may write the slot
     return order_after(g, s);
   }
-  cudaPointerAttributes attr{};
-  const bool pinned = cudaPointerGetAttributes(&attr, pairs) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-  cudaGetLastError();
   const uint64_t cap = g->pairs_cap;
   uint32_t* hp = static_cast<uint32_t*>(g->h_pin);
   for (uint64_t done = 0, k = 0; done < n; k++) {
-    const uint64_t m = std::min(cap, n - done);
+    const uint64_t m = std::min({n - done, cap, slice});
     const int slot = (int)(k & 1);
     uint32_t* dslot = g->d_pairs + (size_t)slot * cap * 2;
     const uint32_t* src = pairs + 2 * done;
@@ -299,8 +313,6 @@ gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cuda
       GS_CUDA_TRY(cudaEventSynchronize(wait_copies ? g->ev_done[slot] : g->ev_copy[slot]));
       std::memcpy(hp + (size_t)slot * cap * 2, src, (size_t)m * 2 * sizeof(uint32_t));
       src = hp + (size_t)slot * cap * 2;
-    } else if (wait_copies) {
-      GS_CUDA_TRY(cudaEventSynchronize(g->ev_done[slot]));
     }
     GS_CUDA_TRY(cudaStreamWaitEvent(g->copy_stream, g->ev_done[slot], 0));
     GS_CUDA_TRY(cudaMemcpyAsync(dslot, src, (size_t)m * 2 * sizeof(uint32_t), cudaMemcpyHostToDevice,

@@ -97,7 +97,7 @@ struct gs_graph {
   uint32_t part_lb = 9;        // low key bits resolved by the second pass
   uint32_t* d_pairs = nullptr; // staging for host-resident input pairs, 2 x [pairs_cap] u32 pairs
   uint64_t pairs_cap = 0;
-  void* h_pin = nullptr;       // 2 pinned staging buffers of pairs_cap pairs
+  void* h_pin = nullptr;       // 2 pinned staging buffers of pairs_cap pairs (null until host memory needs them)
   uint2* d_file_pairs = nullptr; // decoded records of one stream-file slice (gs_ingest_stream_file)
   cudaStream_t copy_stream = nullptr;               // H2D of host input slices
   uint64_t zero_copy_next = 0;                      // ring slot of the next small host batch
@@ -210,9 +210,9 @@ struct GsProfScope {
 
 // Partial-support helpers implemented in the .cu files.
 gs_status gs_ensure_ingest_scratch(gs_graph* g, uint64_t records);
-// The page-locked staging ring (two slots) for host slices of up to `want` pairs, grown as needed up to
-// min(max_batch_edges, 2^25); UINT64_MAX sizes it at that limit.
-gs_status gs_ensure_pair_staging(gs_graph* g, uint64_t want = ~0ull);
+// The staging ring (two slots, with `host` also its page-locked side) for host slices of up to `want` pairs, grown
+// as needed up to min(max_batch_edges, 2^25); UINT64_MAX sizes it at that limit.
+gs_status gs_ensure_pair_staging(gs_graph* g, uint64_t want = ~0ull, bool host = true);
 // Sizes the single-level ingest scratch for batches of `edges` records, so that a later ingest of
 // at most that many records allocates nothing (required while a stream is being captured).
 gs_status gs_reserve_ingest(gs_graph* g, uint64_t edges);

@@ -144,3 +144,25 @@ def test_toggles_that_cancel_in_tenants_and_levels(restatement):
     sk = restatement.new_sketches(V, 1.0, levels)
     restatement.ingest_levels(sk, V, levels, L, seed, pairs)
     assert got == sk.tobytes()
+
+
+@pytest.mark.parametrize("n", [1024, 1025, (1 << 22) - 1, 1 << 22, (1 << 22) + 1, 3 * (1 << 22) + 5])
+def test_host_slices(n):
+    """Host batches: read in place up to 1024 records, else in slices (of 2^22 records at this V) through the
+    two slots; ordinary and page-locked memory, into a fresh handle and one whose slots are in use."""
+    torch = pytest.importorskip("torch")
+    V, seed = 1500, 0xC0FFEE
+    pairs = torch.from_numpy(_random(V, n, n).view(np.int32))
+    with gs.GraphSketch(V, seed) as g:
+        g.ingest_pairs(pairs.cuda())
+        g.synchronize()
+        want = g.download().tobytes()
+    for first in (pairs.pin_memory(), pairs):
+        with gs.GraphSketch(V, seed) as g:
+            g.ingest_pairs(first.numpy().view(np.uint32))
+            g.synchronize()
+            assert g.download().tobytes() == want
+            g.ingest_pairs(pairs.numpy().view(np.uint32))      # the same records again: all cancel
+            g.ingest_pairs(first.numpy().view(np.uint32))
+            g.synchronize()
+            assert g.download().tobytes() == want
