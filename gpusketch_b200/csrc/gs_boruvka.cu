@@ -11,16 +11,18 @@
 //   the round as modified; the loop stops at the first unmodified round, and a round
 //   r >= num_samples is the reference's OutOfSamplesException (src/sketch.cpp:111-113,173-177).
 //
-// All rounds run inside one persistent kernel (k_boruvka), so a query is one launch and one
-// read-back instead of a host round trip per round.  A graph's blocks meet at a barrier between
-// phases, in one of two scopes:
+// All rounds run inside one persistent kernel, so a query is one launch and one read-back instead of
+// a host round trip per round.  A graph's blocks meet at a barrier between phases, in one of two scopes:
 //   cluster   one thread-block cluster per graph: the barrier is the hardware's, and any number of
-//             graphs share a launch without waiting for one another;
-//   grid      one graph, or the large ones of several, over the whole GPU (cooperative launch); the
-//             barrier is a counter in global memory, and every wait on it is bounded and reports
-//             GS_DEV_ERR_TIMEOUT.
+//             graphs share a launch without waiting for one another.  One or few graphs take wide
+//             clusters (k_boruvka_flat, at the end: a round in two phases), many take narrow ones
+//             (k_boruvka);
+//   grid      one graph, or the large ones of several, over the whole GPU (k_boruvka, a cooperative
+//             launch); the barrier is a counter in global memory, and every wait on it is bounded and
+//             reports GS_DEV_ERR_TIMEOUT.
+// gs_boruvka_scope chooses, and says with which figures.
 //
-// A round after round 0 (barriers between the phases):
+// A round of k_boruvka after round 0 (barriers between the phases):
 //   compress  parent[v] = root(v); in the same pass every component's size, every vertex's rank in
 //             its component and the largest component
 //   allocate  a root takes a run of the member list and one task per kPiece members
@@ -44,9 +46,11 @@
 // and cost a load per round from then on (isolated vertices are most of a sparse R-MAT graph).
 //
 // Bound: latency.  A round is a chain of about a dozen dependent loads and five barriers, whatever the
-// graph's size, until the graph is large enough for the member columns' bytes to matter.
-// Measured (one query, us): V = 1024 199 -> 84, 16384 345 -> 195, 100003 835 -> 400, 131072 (R-MAT) 1062 ->
-// 560, 1000003 4810 -> 2020; 256 graphs of 256 to 16384 vertices 2230 -> 1080.  Before, every phase of every
+// graph's size, until the graph is large enough for the member columns' bytes to matter: at V = 10^6 the
+// rounds in which most vertices are still gathered take 150 to 350 us each, of which reading the columns
+// is about 140, and listing the members 110.
+// Measured (one query, us): V = 1024 199 -> 62, 16384 345 -> 188, 100003 835 -> 400, 131072 (R-MAT) 1062 ->
+// 518, 1000003 4810 -> 1970; 256 graphs of 256 to 16384 vertices 2230 -> 1050.  Before, every phase of every
 // graph was a grid phase of 444 blocks, all members were XORed into their component's row by atomics (82 of
 // them per vertex and round at V = 10^6), and roots were appended to a list, so that a round had six barriers.
 // DSU: CAS hooking of the larger root under the smaller (include/dsu.h:155-167 unions by random

@@ -1,15 +1,22 @@
 // gs_ingest.cu - edge-record ingest: device-side endpoint bucketing + per-vertex sketch update.
 //
 // Replaces the reference's host gutters + CudaStream double buffering + sketchUpdate kernel
-// (include/cuda_stream.h:146-276, src/cuda_kernel.cu:197-257).  One ingest pass over n records:
+// (include/cuda_stream.h:146-276, src/cuda_kernel.cu:197-257).  A batch of at most kDirectEdges edge
+// records is XORed into the sketches as it comes (k_ingest_direct, one launch).  A larger one is grouped
+// by vertex first:
 //
 //   1. k_part_count / k_part_scan    per block, a shared-memory histogram of the records' keys
-//                                    (level*V + v) >> lb; one global atomic per non-empty bucket
+//                                    (level*V + v) >> lb; one global atomic per non-empty bucket; a
+//                                    sample of the edges is counted as well
 //   2. k_part_scatter(_staged)       records placed by bucket: sorted per block in shared memory,
 //                                    then written as coalesced runs
-//   3. k_vert_count, k_scan_*        per-vertex record counts and work chunks ceil(count / chunk)
+//   3. k_vert_count, k_vert_offsets  per-vertex record counts; each vertex's run, and the list that it
+//                                    goes to.  The edge sample says whether toggles cancel
 //   4. k_vert_scatter(_sorted)       neighbours placed by vertex inside each chunk of a bucket
-//   5. k_ingest_packed / k_ingest    one warp per work chunk of one vertex.  A lane hashes the edge
+//   5. k_parity                      (when toggles cancel) leaves the neighbours that occur an odd
+//                                    number of times in the runs of the vertices of many records
+//   6. k_ingest_few                  the vertices of few records: a warp takes several of them
+//   7. k_ingest_packed / k_ingest    one warp per work chunk of one vertex.  A lane hashes the edge
 //                                    for one column (XXH3 with the column constant folded,
 //                                    gs_common.cuh) and XORs {mix(edge), checksum} into the
 //                                    shared-memory row of that column and depth (depths < 10);
@@ -21,6 +28,9 @@
 //                                    the non-zero rows and the deterministic bucket are merged into
 //                                    the vertex sketch (plain read-modify-write when the vertex is
 //                                    one chunk, atomic XOR when several warps share it).
+//
+// Batches that come per vertex (directed) are grouped by k_count_batches, k_scan_* and
+// k_scatter_batches, and take steps 6 and 7.
 //
 // XOR is commutative and associative, so the result is bit-identical to the reference's
 // sequential Sketch::update over the same records (src/sketch.cpp:85-99), whatever the order.
@@ -658,6 +668,10 @@ __global__ void k_scatter_batches(const uint32_t* __restrict__ srcs, const uint6
 // cut into work chunks of at most `chunk` records, work[i] = {vertex, chunk of the vertex}.  When toggles
 // cancel, a vertex of more than kParityMin records is first cut into parity items of at most kParityRecords,
 // and listed by k_parity with the records that are left.  All lists are in any order.
+// us of k_ingest_packed and k_ingest_few together for limits of 32 / 64 / 128 / 256 records: R-MAT V = 16384 404
+// 411 410 431, 64 tenants 1147 1134 1205 1258, V = 10^6 and 256 tenants the same within 1%.
+// kParityMin 512, 1024 and 2048 are equal on R-MAT streams; 64 takes a random graph's vertices of 250 records
+// through k_parity, which costs 392 us at V = 100003 and saves 110.
 constexpr uint32_t kFewRecords = 64;
 constexpr uint32_t kParityMin = 1024, kParityRecords = 65536;
 
@@ -802,7 +816,7 @@ __global__ void __launch_bounds__(kPartThreads) k_vert_offsets(const uint32_t* _
 // words, twice over) list the bitmap's set bits instead.  The items of a vertex that has several XOR their
 // bitmaps into one in memory, and the last of them lists that one.
 // Bound by the shared-memory atomics and one read of the records.  R-MAT of 2^27 edge records, V = 2^17:
-// @PARITY@
+// 0.56 ms, after which the packed kernel takes 2.84 ms instead of 8.06 (the phase 11.3 -> 6.7 ms).
 constexpr uint32_t kParityThreads = 256;
 constexpr uint32_t kParityTile = kParityThreads * 8;
 constexpr uint32_t kParityMaxVertices = 1u << 18;   // 32 KB of bitmap: six blocks per SM
@@ -1469,12 +1483,21 @@ __global__ void __launch_bounds__(kPackMaxThreads, 2) k_ingest_packed(const Inge
 // vertex, so rows hold edge ids instead of mixed keys (no inverse mix per bucket), a bit per depth says which
 // rows hold something, and only those are merged, four 16-byte loads of the sketch on their way at once, as
 // plain read-modify-writes: the vertex is this warp's alone.
-// Bound by instruction issue and the latency of the touched sectors together.  @FEW@
+// Bound by the memory's handling of scattered 64-byte runs: reading and writing the first four depths of 28
+// columns per vertex, with nothing computed, takes 1.5 ns a vertex, and this kernel 1.87 (10^6 vertices of 8
+// records each; k_ingest_packed 6.3).  24 warps on an SM matter more than anything that costs registers: 20
+// warps are slower by a tenth, and a spill of 64 bytes makes it five times as slow, because shared memory leaves
+// no L1 for it.
 constexpr uint32_t kFewStride = (kSlabDepth + 1) * 32;   // rows of one column group, with the discard row
 constexpr int few_threads(int cg) { return cg == 1 ? 256 : 128; }
 constexpr uint32_t few_warp_words(int cg) { return cg * kFewStride + 32 + 16; }   // uint4: rows, records, mixed keys
 
-__device__ __forceinline__ uint4 ld_bucket(const GsBucket* p) { return __ldcg(reinterpret_cast<const uint4*>(p)); }
+// A miss of a plain load brings 128 bytes into L2, of which a column's first buckets need half.
+__device__ __forceinline__ uint4 ld_bucket(const GsBucket* p) {
+  uint4 t;
+  asm volatile("ld.global.cg.L2::64B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(t.x), "=r"(t.y), "=r"(t.z), "=r"(t.w) : "l"(p) : "memory");
+  return t;
+}
 __device__ __forceinline__ void st_bucket(GsBucket* p, const uint4& t) { __stcg(reinterpret_cast<uint4*>(p), t); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
