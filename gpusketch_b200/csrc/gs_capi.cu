@@ -260,15 +260,18 @@ namespace {
 // over them reads at most 8 KB over PCIe.
 constexpr uint64_t kZeroCopyPairs = 1024;
 
-// Records in one slice of host input: 64 per vertex, rounded up to a power of two.  A slice's copy overlaps the
-// ingest of the one before, so small slices leave little to do when the last copy lands; but each slice merges
-// the rows of all vertices that it touches, and toggles that cancel are only found within one.  ms for 2^25 R-MAT
+// Records in one slice of host input: 64 per vertex or an eighth of the call's, rounded up to a power of two.
+// A slice's copy overlaps the ingest of the one before, so small slices leave little to do when the last copy
+// lands; but each slice merges the rows of all vertices that it touches, toggles that cancel are only found
+// within one, and copies that follow one another without end (asynchronous calls of 2^27 records) lose about
+// 30 us to each: 157.7 ms per 2^30 records in slices of 2^23, 155.5 of 2^24, 155.7 of 2^25.  ms for 2^25 R-MAT
 // records and the query with slices of 2^22 / 2^23 / 2^24 / 2^25:
 //   V = 2^14: 5.55 / 5.65 / 5.91 / 6.31    V = 2^17: 6.33 / 6.25 / 6.67 / 7.40
 //   V = 2^18: 8.79 / 7.00 / 7.54 / 8.65    V = 2^20: 15.23 / 12.20 / 10.47 / 11.70
-uint64_t host_slice(const gs_graph* g) {
+uint64_t host_slice(const gs_graph* g, uint64_t n) {
+  const uint64_t want = std::max<uint64_t>(64ull * g->V, n / 8);
   uint64_t m = 1ull << 22;
-  while (m < 64ull * g->V && m < (1ull << 24)) m <<= 1;
+  while (m < want && m < (1ull << 24)) m <<= 1;
   return m;
 }
 
@@ -285,7 +288,7 @@ gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cuda
     pinned = cudaPointerGetAttributes(&attr, pairs) == cudaSuccess && attr.type == cudaMemoryTypeHost;
     cudaGetLastError();
   }
-  const uint64_t slice = host_slice(g);
+  const uint64_t slice = host_slice(g, n);
   GS_TRY(gs_ensure_pair_staging(g, std::min(n, slice), !pinned));
   if (n <= kZeroCopyPairs) {
     // a few records: copied into the ring by the host and read from there by the update's kernel, instead of
