@@ -612,8 +612,7 @@ def run_gs(args):
     Sv = geo.bytes_per_vertex
     alg_step = 8.0 * U + V * Sv * (2 * P - 1)
     alg_per_launch = alg_step / P
-    launches = max(1, prof["ingest_launches"])
-    ingest_ms_avg = prof["ingest_ms"] / launches
+    ingest_ms_avg = prof["ingest_ms"] / (args.steps * P)     # a phase's update: k_ingest_few and k_ingest_packed
     achieved = alg_per_launch / (ingest_ms_avg / 1e3) / 1e9
     peak, peak_kind = measured_peak_hbm()
     traffic, traffic_current = ncu_traffic_per_launch()

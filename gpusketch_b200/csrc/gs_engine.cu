@@ -234,7 +234,6 @@ gs_status globalize(gs_engine* e, const uint32_t* in, uint32_t* out, uint64_t fi
 
 struct QueryPlan {
   std::vector<uint8_t> seen;
-  uint32_t vlo = 0xffffffffu, vhi = 0, max_rounds = 0;
   uint64_t total = 0, maxv = 0;
 };
 
@@ -249,9 +248,6 @@ gs_status plan_query(const gs_engine* e, const uint32_t* tenants, uint32_t count
     }
     qp->seen[t] = 1;
     const EngTenant& T = e->ten[t];
-    qp->vlo = std::min(qp->vlo, T.vbase);
-    qp->vhi = std::max(qp->vhi, T.vbase + T.V);
-    qp->max_rounds = std::max(qp->max_rounds, T.geom.num_samples);
     qp->total += T.V;
     qp->maxv = std::max<uint64_t>(qp->maxv, T.V);
   }

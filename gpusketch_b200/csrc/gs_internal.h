@@ -103,8 +103,9 @@ struct gs_graph {
   uint64_t zero_copy_next = 0;                      // ring slot of the next small host batch
   cudaEvent_t ev_copy[2] = {nullptr, nullptr};      // slice copied into d_pairs[slot]
   cudaEvent_t ev_done[2] = {nullptr, nullptr};      // slice in d_pairs[slot] consumed
-  uint32_t* d_status = nullptr;  // [0] error bits [1] records [2] chunks [3] modified [4] forest [5] part chunks
-                                 // ... [16] ingest error bits carried across a query (32 words)
+  uint32_t* d_status = nullptr;  // [0] error bits [1] records, rounds [2] work chunks [3] vertices of few records
+                                 // [4] forest edges [5] part chunks [13] [14] next of [3] and [2] [16] ingest error
+                                 // bits carried across a query [17] components [20..22] parity lists (32 words)
   uint32_t* h_status = nullptr;  // pinned mirror (32 words)
   uint64_t changes = 0;          // count of calls that changed the sketches
   uint64_t changes_at_clear = 0; // `changes` right after the last gs_clear (0: none since creation)
