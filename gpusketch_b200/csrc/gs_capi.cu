@@ -15,7 +15,6 @@ using DeviceGuard = GsDeviceGuard;
   DeviceGuard _guard((g)->device);                                        \
   if (!_guard.ok) { gs_set_error("cannot select CUDA device"); return GS_ERR_NO_DEVICE; }
 
-cudaStream_t pick_stream(gs_graph* g, void* s) { return s ? static_cast<cudaStream_t>(s) : g->stream; }
 
 }  // namespace
 
@@ -83,14 +82,6 @@ gs_status ensure_query_buffers(gs_graph* g) {
   if (!g->h_qstatus) GS_CUDA_TRY(cudaMallocHost(&g->h_qstatus, 32 * sizeof(uint32_t)));
   if (!g->ev_query) GS_CUDA_TRY(cudaEventCreateWithFlags(&g->ev_query, cudaEventDisableTiming));
   GS_CUDA_TRY(cudaMallocHost(&g->h_qlabels, (size_t)g->V * sizeof(uint32_t)));
-  return GS_OK;
-}
-
-// work queued on a caller stream s must finish before the handle's own stream touches the sketches
-gs_status order_after(gs_graph* g, cudaStream_t s) {
-  if (s == g->stream) return GS_OK;
-  GS_CUDA_TRY(cudaEventRecord(g->ev_order, s));
-  GS_CUDA_TRY(cudaStreamWaitEvent(g->stream, g->ev_order, 0));
   return GS_OK;
 }
 
@@ -281,7 +272,8 @@ uint64_t host_slice(const gs_graph* g, uint64_t n) {
 // caller may reuse its buffer); without, it returns at once for page-locked input, whose buffer then
 // stays in use until the handle's work is done, and every wait on a slot's earlier slice happens on
 // the device, so copies of this call can run ahead of queries queued before it.
-gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cudaStream_t s, bool wait_copies) {
+gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, bool wait_copies) {
+  const cudaStream_t s = g->stream;
   bool pinned = false;
   if (n > kZeroCopyPairs) {
     cudaPointerAttributes attr{};
@@ -301,7 +293,7 @@ gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cuda
     GS_TRY(gs_ingest_device_pairs(g, h, n, -1, s));
     GS_CUDA_TRY(cudaEventRecord(g->ev_done[slot], s));
     GS_CUDA_TRY(cudaEventRecord(g->ev_copy[slot], s));   // who waits for either may write the slot
-    return order_after(g, s);
+    return GS_OK;
   }
   const uint64_t cap = g->pairs_cap;
   uint32_t* hp = static_cast<uint32_t*>(g->h_pin);
@@ -328,7 +320,7 @@ gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, cuda
   }
   // the caller's buffer may be reused once every copy has landed
   if (wait_copies) GS_CUDA_TRY(cudaStreamSynchronize(g->copy_stream));
-  return order_after(g, s);
+  return GS_OK;
 }
 
 constexpr uint64_t al16(uint64_t x) { return (x + 15) & ~15ull; }
@@ -339,7 +331,8 @@ constexpr uint64_t al16(uint64_t x) { return (x + 15) & ~15ull; }
 // gathered into the slot's page-locked half - starts rebased to the gathered destinations - copied to
 // the device half and ingested while the next chunk is gathered.
 gs_status ingest_host_batches(gs_graph* g, uint32_t level, const uint32_t* srcs, const uint64_t* starts,
-                              const uint64_t* sizes, uint32_t nbat, const uint32_t* dsts, cudaStream_t s) {
+                              const uint64_t* sizes, uint32_t nbat, const uint32_t* dsts) {
+  const cudaStream_t s = g->stream;
   uint64_t ndst = 0;
   for (uint32_t b = 0; b < nbat; b++) ndst += sizes[b];
   GS_TRY(gs_ensure_pair_staging(g, ndst / 2 + 3 * (uint64_t)nbat));
@@ -382,7 +375,7 @@ gs_status ingest_host_batches(gs_graph* g, uint32_t level, const uint32_t* srcs,
                                     reinterpret_cast<const uint32_t*>(d + off_dsts), s, std::max<uint64_t>(nd, 1)));
     GS_CUDA_TRY(cudaEventRecord(g->ev_done[slot], s));
   }
-  return order_after(g, s);
+  return GS_OK;
 }
 
 }  // namespace
@@ -404,28 +397,24 @@ gs_status gs_ingest_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, int on
   if (!g || (n && !pairs)) { gs_set_error("gs_ingest_pairs: null argument"); return GS_ERR_BAD_ARG; }
   if (n == 0) return GS_OK;
   GS_GUARD(g);
-  cudaStream_t s = pick_stream(g, stream);
   g->labels_valid = false;
   g->changes++;
-  if (on_device) {
-    GS_TRY(gs_ingest_device_pairs(g, pairs, n, -1, s));
-    return order_after(g, s);
-  }
-  return ingest_host_pairs(g, pairs, n, s, true);
+  GsCallerOrder order(g, stream);
+  GS_TRY(order.begin());
+  GS_TRY(on_device ? gs_ingest_device_pairs(g, pairs, n, -1, g->stream) : ingest_host_pairs(g, pairs, n, true));
+  return order.end();
 }
 
 gs_status gs_ingest_pairs_async(gs_graph* g, const uint32_t* pairs, uint64_t n, int on_device, void* stream) {
   if (!g || (n && !pairs)) { gs_set_error("gs_ingest_pairs_async: null argument"); return GS_ERR_BAD_ARG; }
   if (n == 0) return GS_OK;
   GS_GUARD(g);
-  cudaStream_t s = pick_stream(g, stream);
   g->labels_valid = false;
   g->changes++;
-  if (on_device) {
-    GS_TRY(gs_ingest_device_pairs(g, pairs, n, -1, s));
-    return order_after(g, s);
-  }
-  return ingest_host_pairs(g, pairs, n, s, false);
+  GsCallerOrder order(g, stream);
+  GS_TRY(order.begin());
+  GS_TRY(on_device ? gs_ingest_device_pairs(g, pairs, n, -1, g->stream) : ingest_host_pairs(g, pairs, n, false));
+  return order.end();
 }
 
 gs_status gs_ingest_edges(gs_graph* g, const uint32_t* src, const uint32_t* dst, uint64_t n, int on_device,
@@ -439,10 +428,12 @@ gs_status gs_ingest_edges(gs_graph* g, const uint32_t* src, const uint32_t* dst,
     return gs_ingest_pairs(g, host.data(), n, 0, stream);
   }
   // device arrays: interleaved on the device into the staging slots, one slice at a time
-  cudaStream_t s = pick_stream(g, stream);
+  const cudaStream_t s = g->stream;
   g->labels_valid = false;
   g->changes++;
   GS_TRY(gs_ensure_pair_staging(g, n));
+  GsCallerOrder order(g, stream);
+  GS_TRY(order.begin());
   const uint64_t cap = g->pairs_cap;
   for (uint64_t done = 0, k = 0; done < n; k++) {
     const uint64_t m = std::min(cap, n - done);
@@ -457,7 +448,7 @@ gs_status gs_ingest_edges(gs_graph* g, const uint32_t* src, const uint32_t* dst,
     GS_CUDA_TRY(cudaEventRecord(g->ev_done[slot], s));
     done += m;
   }
-  return order_after(g, s);
+  return order.end();
 }
 
 gs_status gs_ingest_vertex_batches(gs_graph* g, uint32_t level, const uint32_t* srcs, const uint64_t* starts,
@@ -470,13 +461,14 @@ gs_status gs_ingest_vertex_batches(gs_graph* g, uint32_t level, const uint32_t* 
   if (level >= g->num_levels) { gs_set_error("level out of range"); return GS_ERR_BAD_ARG; }
   if (nbat == 0) return GS_OK;
   GS_GUARD(g);
-  cudaStream_t s = pick_stream(g, stream);
   g->labels_valid = false;
   g->changes++;
   g->sketches_symmetric = false;  // one-sided updates: the XOR of all vertex sketches is no longer zero
+  GsCallerOrder order(g, stream);
+  GS_TRY(order.begin());
   if (on_device) {
-    GS_TRY(gs_ingest_device_batches(g, level, srcs, starts, sizes, nbat, dsts, s));
-    return order_after(g, s);
+    GS_TRY(gs_ingest_device_batches(g, level, srcs, starts, sizes, nbat, dsts, g->stream));
+    return order.end();
   }
   for (uint32_t b = 0; b < nbat; b++) {
     if (starts[b] > ndst || sizes[b] > ndst - starts[b]) {
@@ -484,7 +476,8 @@ gs_status gs_ingest_vertex_batches(gs_graph* g, uint32_t level, const uint32_t* 
       return GS_ERR_BAD_ARG;
     }
   }
-  return ingest_host_batches(g, level, srcs, starts, sizes, nbat, dsts, s);
+  GS_TRY(ingest_host_batches(g, level, srcs, starts, sizes, nbat, dsts));
+  return order.end();
 }
 
 gs_status gs_synchronize(gs_graph* g) {

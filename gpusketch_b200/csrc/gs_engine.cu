@@ -671,9 +671,11 @@ gs_status gs_engine_ingest(gs_engine* e, const uint32_t* slice_tenants, const ui
   if (!pairs) { gs_set_error("gs_engine_ingest: null pairs"); return GS_ERR_BAD_ARG; }
   GS_ENGINE_GUARD(e);
   gs_graph* g = e->g;
-  cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
+  const cudaStream_t s = g->stream;
   g->labels_valid = false;
   GS_TRY(gs_ensure_pair_staging(g));
+  GsCallerOrder order(g, stream);
+  GS_TRY(order.begin());
   gs_engine::SliceTables& tb = e->tabs[e->tab_next++ & 1];
   GS_CUDA_TRY(cudaEventSynchronize(tb.ev_free));
   GS_TRY(stage_slices(tb, slice_tenants, slice_offsets, num_slices));
@@ -710,11 +712,7 @@ gs_status gs_engine_ingest(gs_engine* e, const uint32_t* slice_tenants, const ui
   }
   GS_CUDA_TRY(cudaEventRecord(tb.ev_free, s));
   if (!pairs_on_device) GS_CUDA_TRY(cudaStreamSynchronize(g->copy_stream));
-  if (s != g->stream) {
-    GS_CUDA_TRY(cudaEventRecord(g->ev_order, s));
-    GS_CUDA_TRY(cudaStreamWaitEvent(g->stream, g->ev_order, 0));
-  }
-  return GS_OK;
+  return order.end();
 }
 
 gs_status gs_engine_ingest_slices(gs_engine* e, uint32_t num_slices, const uint32_t* slice_tenants,
@@ -739,9 +737,11 @@ gs_status gs_engine_ingest_slices(gs_engine* e, uint32_t num_slices, const uint3
   if (total == 0) return GS_OK;
   GS_ENGINE_GUARD(e);
   gs_graph* g = e->g;
-  cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g->stream;
+  const cudaStream_t s = g->stream;
   g->labels_valid = false;
   GS_TRY(gs_ensure_pair_staging(g));
+  GsCallerOrder order(g, stream);
+  GS_TRY(order.begin());
   const uint64_t cap = g->pairs_cap;
   uint32_t* hp = static_cast<uint32_t*>(g->h_pin);
   bool direct = false;  // some slice was copied straight from caller memory
@@ -794,11 +794,7 @@ gs_status gs_engine_ingest_slices(gs_engine* e, uint32_t num_slices, const uint3
   }
   // caller memory read in place must have landed before the caller may reuse it
   if (direct) GS_CUDA_TRY(cudaStreamSynchronize(g->copy_stream));
-  if (s != g->stream) {
-    GS_CUDA_TRY(cudaEventRecord(g->ev_order, s));
-    GS_CUDA_TRY(cudaStreamWaitEvent(g->stream, g->ev_order, 0));
-  }
-  return GS_OK;
+  return order.end();
 }
 
 gs_status gs_engine_synchronize(gs_engine* e) {

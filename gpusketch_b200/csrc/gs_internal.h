@@ -56,9 +56,9 @@ struct gs_graph {
   int num_sms = 148;
   uint64_t max_batch_edges = 1ull << 27;
   GsTuning tune{};
-  cudaStream_t stream = nullptr;      // stream every kernel of this handle is launched on
+  cudaStream_t stream = nullptr;      // stream that every kernel of this handle is launched on
   cudaStream_t own_stream = nullptr;  // created with the handle
-  cudaEvent_t ev_order = nullptr;     // orders the handle's stream after a caller-stream ingest
+  cudaEvent_t ev_order = nullptr;     // orders the handle's stream and a caller's (GsCallerOrder)
 
   // ---- resident state ----
   GsBucket* d_sk = nullptr;    // [num_levels][V][num_buckets]
@@ -191,6 +191,33 @@ struct GsDeviceGuard {
   ~GsDeviceGuard() {
     int cur = -1;
     if (prev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev) cudaSetDevice(prev);
+  }
+};
+
+// A call's place in the order of the stream that its caller names.  All work of a handle runs on the handle's
+// stream; begin() makes that wait for what the caller has queued (the records may be written just before the
+// call), and end(), or leaving the call early, makes the caller's stream wait for the work (the records' memory
+// may be used again right after it).  Null, or the handle's own stream: nothing to order.
+struct GsCallerOrder {
+  gs_graph* const g;
+  const cudaStream_t caller;
+  bool open = false;
+  GsCallerOrder(gs_graph* g_, void* stream)
+      : g(g_), caller(stream && stream != g_->stream ? static_cast<cudaStream_t>(stream) : nullptr) {}
+  ~GsCallerOrder() { end(); }
+  gs_status begin() {
+    if (!caller) return GS_OK;
+    GS_CUDA_TRY(cudaEventRecord(g->ev_order, caller));
+    GS_CUDA_TRY(cudaStreamWaitEvent(g->stream, g->ev_order, 0));
+    open = true;
+    return GS_OK;
+  }
+  gs_status end() {
+    if (!open) return GS_OK;
+    open = false;
+    GS_CUDA_TRY(cudaEventRecord(g->ev_order, g->stream));
+    GS_CUDA_TRY(cudaStreamWaitEvent(caller, g->ev_order, 0));
+    return GS_OK;
   }
 };
 

@@ -109,9 +109,9 @@ class SketchEngine:
         so = np.ascontiguousarray(slice_offsets, dtype=np.uint64)
         if so.size != st.size + 1:
             raise ValueError("slice_offsets needs one entry more than slice_tenants")
-        p, _, dev, keep = _as_pairs(pairs)
+        p, _, dev, keep = _as_pairs(pairs, stream)
         check(self._lib.gs_engine_ingest(self._h, st.ctypes.data, so.ctypes.data, st.size, p, int(dev),
-                                         _device_stream(stream, dev)), "gs_engine_ingest")
+                                         _device_stream(stream, keep if dev else None)), "gs_engine_ingest")
         del keep
 
     def ingest_batches(self, batches, stream=None) -> None:
@@ -164,7 +164,7 @@ class SketchEngine:
             # gs_engine_phase takes no stream: the records' producer (and a .contiguous() copy) must be
             # complete before the engine's own stream reads them
             import torch
-            torch.cuda.current_stream().synchronize()
+            torch.cuda.current_stream(keep.device).synchronize()
         qt = np.ascontiguousarray(list(query_tenants), dtype=np.uint32)
         ncc = np.zeros(max(qt.size, 1), np.uint32)
         rounds = np.zeros(max(qt.size, 1), np.uint32)

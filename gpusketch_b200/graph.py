@@ -43,14 +43,26 @@ def hash64(key: int, seed: int) -> int:
     return int(lib().gs_hash64(key & (2**64 - 1), seed & (2**64 - 1)))
 
 
-def _as_pairs(pairs):
+def _contiguous(t, stream):
+    """t.contiguous(); with an explicit stream, a copy of a CUDA tensor is made (and its memory reused) in the
+    order of that stream."""
+    if stream is None or not t.is_cuda or t.is_contiguous():
+        return t.contiguous()
+    import torch
+    ptr = _named_stream(stream).value
+    s = torch.cuda.default_stream(t.device) if ptr == CUDA_STREAM_LEGACY else torch.cuda.ExternalStream(ptr, t.device)
+    with torch.cuda.stream(s):
+        return t.contiguous()
+
+
+def _as_pairs(pairs, stream=None):
     """(pointer, count, on_device, keepalive) for an (n, 2) uint32 array or tensor."""
     try:
         import torch
         if isinstance(pairs, torch.Tensor):
             if pairs.dtype not in (torch.int32, torch.uint32):
                 raise TypeError("edge records must be 32-bit integers")
-            t = pairs.contiguous()
+            t = _contiguous(pairs, stream)
             return C.c_void_p(t.data_ptr()), t.numel() // 2, bool(t.is_cuda), t
     except ImportError:  # pragma: no cover
         pass
@@ -58,14 +70,14 @@ def _as_pairs(pairs):
     return C.c_void_p(a.ctypes.data), a.size // 2, False, a
 
 
-def _as_u32(values):
+def _as_u32(values, stream=None):
     """(pointer, count, on_device, keepalive) for a 1-D uint32 array or 32-bit tensor."""
     try:
         import torch
         if isinstance(values, torch.Tensor):
             if values.dtype not in (torch.int32, torch.uint32):
                 raise TypeError("vertex ids must be 32-bit integers")
-            t = values.contiguous()
+            t = _contiguous(values, stream)
             return C.c_void_p(t.data_ptr()), t.numel(), bool(t.is_cuda), t
     except ImportError:  # pragma: no cover
         pass
@@ -79,15 +91,25 @@ def _stream_ptr(stream) -> C.c_void_p:
     return C.c_void_p(int(getattr(stream, "cuda_stream", stream)))
 
 
-def _device_stream(stream, on_device: bool) -> C.c_void_p:
-    """The stream a call with device operands runs on.  With no explicit stream, torch's current
-    stream: the library's work is then ordered after the torch kernels that produced the operands, and
-    torch's caching allocator, which reuses a freed block only after the work queued on that stream,
-    cannot hand a temporary (a .contiguous() copy) to another tensor while the library still reads it."""
-    if stream is None and on_device:
-        import torch
-        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
-    return _stream_ptr(stream)
+CUDA_STREAM_LEGACY = 1   # cudaStreamLegacy: the default stream by name (a null pointer names none)
+
+
+def _named_stream(stream) -> C.c_void_p:
+    return C.c_void_p(_stream_ptr(stream).value or CUDA_STREAM_LEGACY)
+
+
+def _device_stream(stream, operand) -> C.c_void_p:
+    """The stream that orders a call; `operand` is its device operand, or None.  With no explicit stream, torch's
+    current stream on the operand's device: the library's work is ordered after the torch kernels that
+    produced the operand, and torch's caching allocator, which reuses a freed block only after the work
+    queued on that stream, cannot hand a temporary (a .contiguous() copy) to another tensor while the
+    library still reads it.  Torch's default stream is a null pointer, which would name no stream."""
+    if stream is not None:
+        return _named_stream(stream)
+    if operand is None:
+        return C.c_void_p(0)
+    import torch
+    return _named_stream(torch.cuda.current_stream(operand.device))
 
 
 class GraphSketch:
@@ -140,8 +162,9 @@ class GraphSketch:
 
     # ---- ingest ----
     def ingest_pairs(self, pairs, stream=None) -> None:
-        p, n, dev, keep = _as_pairs(pairs)
-        check(self._lib.gs_ingest_pairs(self._h, p, n, int(dev), _device_stream(stream, dev)), "gs_ingest_pairs")
+        p, n, dev, keep = _as_pairs(pairs, stream)
+        check(self._lib.gs_ingest_pairs(self._h, p, n, int(dev), _device_stream(stream, keep if dev else None)),
+              "gs_ingest_pairs")
         del keep
 
     def prepare_host_input(self, records: int) -> None:
@@ -152,10 +175,10 @@ class GraphSketch:
         """gs_ingest_pairs_async: queue the copies and the ingest without waiting.  A page-locked host
         buffer (a pinned CPU tensor) stays in use until the handle's queued work is done: keep it alive
         and unchanged until synchronize(), query_wait() or a synchronous query."""
-        p, n, dev, keep = _as_pairs(pairs)
+        p, n, dev, keep = _as_pairs(pairs, stream)
         if keep is not pairs and not dev:
             raise ValueError("ingest_pairs_async needs a C-contiguous uint32/int32 buffer the caller keeps alive")
-        check(self._lib.gs_ingest_pairs_async(self._h, p, n, int(dev), _device_stream(stream, dev)),
+        check(self._lib.gs_ingest_pairs_async(self._h, p, n, int(dev), _device_stream(stream, keep if dev else None)),
               "gs_ingest_pairs_async")
 
     def ingest_stream_file(self, path: str, first: int = 0, count: int | None = None) -> int:
@@ -170,11 +193,12 @@ class GraphSketch:
     def ingest_edges(self, src, dst, stream=None) -> None:
         """gs_ingest_edges: record i toggles edge {src[i], dst[i]}; both arrays on the host or both on
         the device."""
-        a, na, da, ka = _as_u32(src)
-        b, nb, db, kb = _as_u32(dst)
+        a, na, da, ka = _as_u32(src, stream)
+        b, nb, db, kb = _as_u32(dst, stream)
         if na != nb or da != db:
             raise ValueError("src and dst need the same length and the same side (host or device)")
-        check(self._lib.gs_ingest_edges(self._h, a, b, na, int(da), _device_stream(stream, da)), "gs_ingest_edges")
+        check(self._lib.gs_ingest_edges(self._h, a, b, na, int(da), _device_stream(stream, ka if da else None)),
+              "gs_ingest_edges")
         del ka, kb
 
     def ingest_vertex_batches(self, srcs, starts, sizes, dsts, level: int = 0) -> None:
@@ -332,5 +356,5 @@ def rmat_stream(log2_v: int, n: int, seed: int, first: int = 0, a: float = 0.57,
     if cnt < n:
         raise ValueError("output too small")
     check(lib().gs_gen_rmat_stream(log2_v, a, b, c, delete_frac, seed, first, n, p, int(dev),
-                                   _device_stream(stream, dev)), "gs_gen_rmat_stream")
+                                   _device_stream(stream, keep if dev else None)), "gs_gen_rmat_stream")
     return out

@@ -113,8 +113,13 @@ uint64_t gs_desired_updates_per_batch(const gs_graph* g);
  * tags into (one level for connected-components graphs).  Self-loops are no-ops, as in
  * the reference where the two updates of sketch src cancel.  pairs_on_device != 0 means
  * `pairs` is a device pointer; otherwise it is host memory (pinned or pageable) staged
- * through the library's pinned ring.  `cuda_stream` (cudaStream_t, may be NULL) orders the
- * work after the caller's stream.  Replaces the GPU worker path
+ * through the library's pinned ring.  The work runs on the handle's stream, after what is
+ * queued on `cuda_stream` (cudaStream_t) at the call and before what is queued there after it: in
+ * that stream's order, device records may be written just before the call and their memory used
+ * again right after it.  So may they for every entry point with a stream and device operands.
+ * NULL names no stream and orders nothing: the caller makes sure that device records are complete
+ * before the call and stay until the handle's work is done.  The default stream is named by
+ * cudaStreamLegacy (1) or cudaStreamPerThread (2).  Replaces the GPU worker path
  * GraphSketchDriver::batch_callback -> CCGPUSketchAlg::apply_update_batch ->
  * CudaStream::process_batch -> CudaKernel::sketchUpdate (include/graph_sketch_driver.h:204-208,
  * src/cc_gpu_sketch_alg.cpp:7-19, include/cuda_stream.h:146-202, src/cuda_kernel.cu:242-257). */
