@@ -302,6 +302,11 @@ __global__ void __launch_bounds__(kPartThreads) k_part_scatter(const uint2* __re
   }
 }
 
+// The records are read once to be counted and again to be placed.  A record that changes in between (a caller's
+// buffer that is written while the library reads it) leaves counts and records apart, so every index that a
+// record gives after the count is checked against what it indexes: shared stages, the buckets of staged records,
+// vertices past the last one, parity bitmaps.  What does not fit sets GS_DEV_ERR_CAPACITY.
+
 // Pass 1 placement when every edge makes exactly two records (one level).  Pass A counts the block's
 // records per bucket in shared memory; after the block scan and the global range
 // reservation, pass B reads the edges again (from L2: the block read them a moment ago) and takes each
@@ -386,9 +391,11 @@ __global__ void __launch_bounds__(kPartThreads, 3) k_part_scatter_staged(const u
       const uint32_t ku = lvl * t.V + p.x, kv = lvl * t.V + p.y;
       const uint32_t pu = slot_inc(cur, ku >> lb, ok);
       const uint32_t pv = slot_inc(cur, kv >> lb, ok);
-      if (ok) {
+      if (ok && max(pu, pv) < 2u * kPartEdges) {
         stage[pu] = make_uint2(ku, p.y);
         stage[pv] = make_uint2(kv, p.x);
+      } else if (ok) {
+        atomicOr(status, (uint32_t)GS_DEV_ERR_CAPACITY);
       }
     }
   }
@@ -397,7 +404,7 @@ __global__ void __launch_bounds__(kPartThreads, 3) k_part_scatter_staged(const u
   for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
     const uint2 r = stage[i];
     const uint32_t b = r.x >> lb;
-    const uint64_t pos = (uint64_t)gbase[b] + (i - loff[b]);
+    const uint64_t pos = b < H ? (uint64_t)gbase[b] + (i - loff[b]) : cap;
     if (pos >= cap) atomicOr(status, (uint32_t)GS_DEV_ERR_CAPACITY);
     else if (COMPACT) reinterpret_cast<uint32_t*>(part)[pos] = ((r.x & ((1u << lb) - 1u)) << (32u - lb)) | r.y;
     else part[pos] = r;
@@ -426,8 +433,8 @@ __device__ __forceinline__ uint32_t chunk_bucket(const uint32_t* choff, uint32_t
 // sorted placement of the same chunk need not count it again
 template <bool COMPACT>
 __global__ void __launch_bounds__(kPartThreads) k_vert_count(const uint2* __restrict__ part, const uint32_t* __restrict__ bkt,
-                                                             uint32_t H, uint32_t lb, uint32_t* __restrict__ cnt,
-                                                             const uint32_t* __restrict__ status,
+                                                             uint32_t H, uint32_t lb, uint32_t nv,
+                                                             uint32_t* __restrict__ cnt, uint32_t* __restrict__ status,
                                                              uint32_t* __restrict__ chunkhist, const Sample sample) {
   extern __shared__ uint32_t hist[];
   __shared__ uint32_t s_d;
@@ -462,7 +469,10 @@ __global__ void __launch_bounds__(kPartThreads) k_vert_count(const uint2* __rest
     }
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < nk; k += blockDim.x) {
-      if (hist[k]) atomicAdd(&cnt[(d << lb) + k], hist[k]);
+      if (hist[k]) {
+        if ((d << lb) + k < nv) atomicAdd(&cnt[(d << lb) + k], hist[k]);
+        else atomicOr(status, (uint32_t)GS_DEV_ERR_CAPACITY);
+      }
       if (chunkhist) chunkhist[((size_t)c << lb) + k] = hist[k];
     }
     __syncthreads();
@@ -472,7 +482,8 @@ __global__ void __launch_bounds__(kPartThreads) k_vert_count(const uint2* __rest
 // pass 2, placement: each record's neighbour goes to its vertex's slice of nbr
 template <bool COMPACT>
 __global__ void __launch_bounds__(kPartThreads) k_vert_scatter(const uint2* __restrict__ part, const uint32_t* __restrict__ bkt,
-                                                               uint32_t H, uint32_t lb, uint32_t* __restrict__ cursor,
+                                                               uint32_t H, uint32_t lb, uint32_t nv,
+                                                               uint32_t* __restrict__ cursor,
                                                                uint32_t* __restrict__ nbr, uint64_t cap,
                                                                uint32_t* __restrict__ status) {
   extern __shared__ uint32_t sh[];
@@ -504,7 +515,7 @@ __global__ void __launch_bounds__(kPartThreads) k_vert_scatter(const uint2* __re
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < nk; k += blockDim.x) {
       const uint32_t h = hist[k];
-      base[k] = h ? atomicAdd(&cursor[(d << lb) + k], h) : 0u;
+      base[k] = h && (d << lb) + k < nv ? atomicAdd(&cursor[(d << lb) + k], h) : 0xffffffffu;   // k_vert_count reported
       hist[k] = 0;
     }
     __syncthreads();
@@ -556,7 +567,8 @@ size_t vert_scatter_sorted_smem(uint32_t lb) {
 // block scans, and a third resident block keeps loads in flight meanwhile
 __global__ void __launch_bounds__(kPartThreads, 3) k_vert_scatter_sorted(const uint32_t* __restrict__ part,
                                                                       const uint32_t* __restrict__ bkt, uint32_t H,
-                                                                      uint32_t lb, uint32_t* __restrict__ cursor,
+                                                                      uint32_t lb, uint32_t nv,
+                                                                      uint32_t* __restrict__ cursor,
                                                                       uint32_t* __restrict__ nbr, uint64_t cap,
                                                                       uint32_t* __restrict__ status,
                                                                       const uint32_t* __restrict__ chunkhist) {
@@ -608,14 +620,18 @@ __global__ void __launch_bounds__(kPartThreads, 3) k_vert_scatter_sorted(const u
         const uint32_t h = hist[k];
         loff[k] = run;
         cur[k] = run;
-        base[k] = h ? atomicAdd(&cursor[(d << lb) + k], h) : 0u;
+        base[k] = h && (d << lb) + k < nv ? atomicAdd(&cursor[(d << lb) + k], h) : 0xffffffffu;   // k_vert_count reported
         run += h;
       }
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kVertPer; j++)
-      if (r0 + threadIdx.x + j * blockDim.x < r1) stage[atomicAdd(&cur[rec[j] >> shift], 1u)] = rec[j];
+      if (r0 + threadIdx.x + j * blockDim.x < r1) {
+        const uint32_t at = atomicAdd(&cur[rec[j] >> shift], 1u);
+        if (at < (uint32_t)kVertChunk) stage[at] = rec[j];
+        else atomicOr(&status[0], (uint32_t)GS_DEV_ERR_CAPACITY);
+      }
     __syncthreads();
     const uint32_t n = r1 - r0;
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -874,11 +890,16 @@ __global__ void __launch_bounds__(kParityThreads) k_parity(const ParityArgs A) {
         u[k] = i < r1 ? A.nbr[i] : 0xffffffffu;
       }
 #pragma unroll
-      for (int k = 0; k < 8; k++)
-        if (u[k] != 0xffffffffu) {
-          const uint2 w = parity_place(u[k] - vb);
+      for (int k = 0; k < 8; k++) {
+        if (u[k] == 0xffffffffu) continue;
+        const uint32_t id = u[k] - vb;
+        if (id < 32u * A.words) {
+          const uint2 w = parity_place(id);
           atomicXor(&bm[w.x], w.y);
+        } else {
+          atomicOr(A.lists.status, (uint32_t)GS_DEV_ERR_CAPACITY);
         }
+      }
     }
     __syncthreads();
     bool list = true;   // this block lists what is left of the vertex
@@ -896,7 +917,7 @@ __global__ void __launch_bounds__(kParityThreads) k_parity(const ParityArgs A) {
 #pragma unroll
         for (int k = 0; k < 8; k++) {
           bool keep = false;
-          if (u[k] != 0xffffffffu) {
+          if (u[k] != 0xffffffffu && u[k] - vb < 32u * A.words) {
             const uint2 w = parity_place(u[k] - vb);
             keep = atomicAnd(&bm[w.x], ~w.y) & w.y;
           }
@@ -1885,9 +1906,9 @@ gs_status launch_part_scatter_staged(const uint2* p, uint64_t m, const PairTag& 
   return GS_OK;
 }
 
-gs_status launch_vert_scatter_sorted(const uint2* part, const uint32_t* bkt, uint32_t H, uint32_t lb, uint32_t* cursor,
-                                     uint32_t* nbr, uint64_t cap, uint32_t* status, const uint32_t* chunkhist, int grid,
-                                     cudaStream_t s) {
+gs_status launch_vert_scatter_sorted(const uint2* part, const uint32_t* bkt, uint32_t H, uint32_t lb, uint32_t nv,
+                                     uint32_t* cursor, uint32_t* nbr, uint64_t cap, uint32_t* status,
+                                     const uint32_t* chunkhist, int grid, cudaStream_t s) {
   const size_t smem = vert_scatter_sorted_smem(lb);
   static thread_local size_t smem_set[64] = {};
   int dev = 0;
@@ -1896,8 +1917,8 @@ gs_status launch_vert_scatter_sorted(const uint2* part, const uint32_t* bkt, uin
     GS_CUDA_TRY(cudaFuncSetAttribute(k_vert_scatter_sorted, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     smem_set[dev & 63] = smem;
   }
-  k_vert_scatter_sorted<<<grid, kPartThreads, smem, s>>>(reinterpret_cast<const uint32_t*>(part), bkt, H, lb, cursor,
-                                                          nbr, cap, status, chunkhist);
+  k_vert_scatter_sorted<<<grid, kPartThreads, smem, s>>>(reinterpret_cast<const uint32_t*>(part), bkt, H, lb, nv,
+                                                          cursor, nbr, cap, status, chunkhist);
   GS_CUDA_TRY(cudaGetLastError());
   return GS_OK;
 }
@@ -2157,19 +2178,19 @@ static gs_status ingest_edges_grouped(gs_graph* g, const uint2* p, uint64_t m, c
     uint32_t* chunkhist = nullptr;
     if (compact) {
       GS_TRY(ensure_chunkhist(g, 2 * m, &chunkhist));
-      k_vert_count<true><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
+      k_vert_count<true><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, nv, g->d_cnt, g->d_status,
                                                              chunkhist, sample);
     } else {
-      k_vert_count<false><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_status,
+      k_vert_count<false><<<grid2, kPartThreads, vc_smem, s>>>(g->d_part, g->d_bkt, H, lb, nv, g->d_cnt, g->d_status,
                                                               nullptr, sample);
     }
     GS_TRY(ensure_work(g, parity_possible(g), s));
     k_vert_offsets<<<H, kPartThreads, 0, s>>>(g->d_bkt, H, lb, nv, g->d_off, g->d_cnt, work_lists(g), sample);
     if (compact) {
-      GS_TRY(launch_vert_scatter_sorted(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_nbr, g->nbr_cap, g->d_status,
+      GS_TRY(launch_vert_scatter_sorted(g->d_part, g->d_bkt, H, lb, nv, g->d_cnt, g->d_nbr, g->nbr_cap, g->d_status,
                                         chunkhist, g->num_sms * 3, s));
     } else {
-      k_vert_scatter<false><<<grid2, kPartThreads, vs_smem, s>>>(g->d_part, g->d_bkt, H, lb, g->d_cnt, g->d_nbr,
+      k_vert_scatter<false><<<grid2, kPartThreads, vs_smem, s>>>(g->d_part, g->d_bkt, H, lb, nv, g->d_cnt, g->d_nbr,
                                                                  g->nbr_cap, g->d_status);
     }
     GS_CUDA_TRY(cudaGetLastError());
