@@ -92,8 +92,17 @@ __global__ void k_interleave(const uint32_t* __restrict__ a, const uint32_t* __r
     out[i] = make_uint2(a[i], b[i]);
 }
 
-// The most pairs in one staging slot (256 MB on each side); what a call asks for depends on its input.
-uint64_t staging_limit(const gs_graph* g) { return std::min<uint64_t>(g->max_batch_edges, 1ull << 25); }
+// Host batches of at most this many records are read by the kernels where they lie in the page-locked ring
+// instead of being copied on the copy stream, with two events and a wait around them (two batches of 100 records
+// and a query whose kernel writes the labels itself: 173 -> 115 us for both together); each of the few passes
+// over them reads at most 8 KB over PCIe.
+constexpr uint64_t kZeroCopyPairs = 1024;
+
+// The most pairs in one staging slot (256 MB on each side); what a call asks for depends on its input.  However
+// small max_batch_edges is, a slot holds such a batch, a batch header with destinations, a file record.
+uint64_t staging_limit(const gs_graph* g) {
+  return std::max(kZeroCopyPairs, std::min<uint64_t>(g->max_batch_edges, 1ull << 25));
+}
 
 }  // namespace
 
@@ -244,12 +253,6 @@ uint64_t gs_desired_updates_per_batch(const gs_graph* g) {
 }  // extern "C"
 
 namespace {
-
-// Host batches of at most this many records are read by the kernels where they lie in the page-locked ring
-// instead of being copied on the copy stream, with two events and a wait around them (two batches of 100 records
-// and a query whose kernel writes the labels itself: 173 -> 115 us for both together); each of the few passes
-// over them reads at most 8 KB over PCIe.
-constexpr uint64_t kZeroCopyPairs = 1024;
 
 // Records in one slice of host input: 64 per vertex or an eighth of the call's, rounded up to a power of two.
 // A slice's copy overlaps the ingest of the one before, so small slices leave little to do when the last copy

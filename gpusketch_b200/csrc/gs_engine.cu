@@ -847,9 +847,9 @@ gs_status gs_engine_phase(gs_engine* e, const uint32_t* slice_tenants, const uin
   gs_graph* g = e->g;
   cudaStream_t s = g->stream;
   GS_TRY(gs_ensure_pair_staging(g));
-  if (n > g->pairs_cap) {
-    gs_set_error("gs_engine_phase: at most " + std::to_string(g->pairs_cap) + " records per phase, got " +
-                 std::to_string(n));
+  const uint64_t most = std::min(g->pairs_cap, g->max_batch_edges);
+  if (n > most) {
+    gs_set_error("gs_engine_phase: at most " + std::to_string(most) + " records per phase, got " + std::to_string(n));
     return GS_ERR_BAD_ARG;
   }
   // everything the recorded work touches exists before recording starts, and nothing queued on the
