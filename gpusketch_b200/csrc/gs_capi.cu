@@ -372,6 +372,7 @@ gs_status ingest_host_batches(gs_graph* g, uint32_t level, const uint32_t* srcs,
     uint8_t* d = dp + slot * slot_bytes;
     GS_CUDA_TRY(cudaMemcpyAsync(d, h, off_sizes + nb * 8, cudaMemcpyHostToDevice, s));
     if (nd) GS_CUDA_TRY(cudaMemcpyAsync(d + off_dsts, hd, nd * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    GS_CUDA_TRY(cudaEventRecord(g->ev_copy[slot], s));   // who waits for it may write the page-locked slot
     GS_TRY(gs_ingest_device_batches(g, level, reinterpret_cast<const uint32_t*>(d),
                                     reinterpret_cast<const uint64_t*>(d + off_starts),
                                     reinterpret_cast<const uint64_t*>(d + off_sizes), (uint32_t)nb,
