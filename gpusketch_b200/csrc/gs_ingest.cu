@@ -1604,12 +1604,14 @@ __global__ void __launch_bounds__(few_threads(CG), 3) k_ingest_few(const IngestA
         rb = __shfl_sync(0xffffffffu, first, i + 1);
         n = __shfl_sync(0xffffffffu, count, i + 1);
         nu = lane < n ? A.nbr[rb + lane] : 0u;
-        // and its columns' first four depths, which most vertices touch, are asked into L2 (a hint: the tenant's
-        // geometry may be another; 3% of the kernel's time)
+        // and its columns' first four depths, which most vertices touch, are asked into L2 (3% of the kernel's
+        // time).  C and bkt are this vertex's: a vertex of another tenant, whose sketch may be smaller and the
+        // arena's last, is not asked for
         const GsBucket* col = A.sk + __shfl_sync(0xffffffffu, mysk, i + 1) + (size_t)lane * bkt;
-        if (lane < C) {
+        const bool same = !TEN || __shfl_sync(0xffffffffu, myt, i + 1) == cur_t;
+        if (same && lane < C) {
           prefetch_l2(col);
-          prefetch_l2(col + 2);
+          if (bkt > 2) prefetch_l2(col + 2);
         }
       }
       // depths below cap are rows, row cap is the discard row; a geometry with more buckets per column than
