@@ -1219,7 +1219,7 @@ size_t dynamic_bytes(int scope, uint32_t R, uint32_t T1) {
 }
 
 // Launches of more than 48 KB of dynamic shared memory, and clusters of more than 8 blocks, are opted into
-// per device and kernel; what was opted into is remembered per host thread.
+// per device and kernel; that it was done, and the cluster size that fits, are remembered per host thread.
 template <int SCOPE, int SLOTS, bool MANY = false>
 gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s) {
   struct Opted { size_t smem = 0; uint32_t blocks = 0; int sms = 0; };
@@ -1236,7 +1236,7 @@ gs_status launch_boruvka(const BorArgs& A, const GsBorLaunch& L, cudaStream_t s)
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (o.smem < cfg.dynamicSmemBytes) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+    GS_TRY(gs_allow_shared_memory(kernel, dev));
     GS_CUDA_TRY(cudaDeviceGetAttribute(&o.sms, cudaDevAttrMultiProcessorCount, dev));
     o.blocks = 8;
     if (SCOPE != kGrid) {

@@ -1794,13 +1794,12 @@ template <int CG, int R, bool SMALL, bool TEN>
 gs_status launch_ingest(gs_graph* g, const IngestArgs& A, cudaStream_t s) {
   const int warps = (int)g->tune.warps_per_block;
   const size_t smem = ingest_smem_bytes(CG, R, warps);
-  // the opt-in shared-memory limit is a per-device function attribute; the persistent grid fills
-  // every SM with as many blocks as registers and shared memory allow
+  // the persistent grid fills every SM with as many blocks as registers and shared memory allow
   struct Cache { size_t smem = 0; int warps = 0; int blocks = 0; };
   static thread_local Cache cache[64];  // per host thread, device and kernel instantiation
   Cache& cc = cache[g->device < 64 ? g->device : 63];
   if (cc.smem != smem || cc.warps != warps) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(k_ingest<CG, R, SMALL, TEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GS_TRY(gs_allow_shared_memory(k_ingest<CG, R, SMALL, TEN>, g->device));
     int nb = 0;
     GS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ingest<CG, R, SMALL, TEN>, warps * 32, smem));
     cc.smem = smem;
@@ -1830,7 +1829,7 @@ gs_status launch_ingest_packed(gs_graph* g, IngestArgs A, cudaStream_t s) {
   static thread_local Cache cache[64];  // per host thread, device and kernel instantiation
   Cache& cc = cache[g->device < 64 ? g->device : 63];
   if (cc.smem != smem || cc.warps != warps) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(k_ingest_packed<TEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GS_TRY(gs_allow_shared_memory(k_ingest_packed<TEN>, g->device));
     int nb = 0;
     GS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ingest_packed<TEN>, warps * 32, smem));
     cc.smem = smem;
@@ -1851,7 +1850,7 @@ gs_status launch_ingest_few(const IngestArgs& A, int num_sms, cudaStream_t s) {
   int dev = 0;
   GS_CUDA_TRY(cudaGetDevice(&dev));
   if (!opted[dev & 63]) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(k_ingest_few<CG, TEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GS_TRY((gs_allow_shared_memory(k_ingest_few<CG, TEN>, dev)));
     opted[dev & 63] = true;
   }
   k_ingest_few<CG, TEN><<<grid, few_threads(CG), smem, s>>>(A);
@@ -1895,12 +1894,12 @@ gs_status launch_part_scatter_staged(const uint2* p, uint64_t m, const PairTag& 
                                      uint32_t* bkt, uint2* part, uint64_t cap, uint32_t* status,
                                      const uint32_t* blockhist, cudaStream_t s) {
   const size_t smem = part_scatter_staged_smem(H);
-  static thread_local size_t smem_set[64] = {};
+  static thread_local bool opted[64] = {};
   int dev = 0;
   GS_CUDA_TRY(cudaGetDevice(&dev));
-  if (smem_set[dev & 63] < smem) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(k_part_scatter_staged<COMPACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    smem_set[dev & 63] = smem;
+  if (!opted[dev & 63]) {
+    GS_TRY(gs_allow_shared_memory(k_part_scatter_staged<COMPACT>, dev));
+    opted[dev & 63] = true;
   }
   const unsigned tiles = (unsigned)((m + kPartEdges - 1) / kPartEdges);
   k_part_scatter_staged<COMPACT><<<tiles, kPartThreads, smem, s>>>(p, m, t, lb, H, bkt, part, cap, status, blockhist);
@@ -1912,12 +1911,12 @@ gs_status launch_vert_scatter_sorted(const uint2* part, const uint32_t* bkt, uin
                                      uint32_t* cursor, uint32_t* nbr, uint64_t cap, uint32_t* status,
                                      const uint32_t* chunkhist, int grid, cudaStream_t s) {
   const size_t smem = vert_scatter_sorted_smem(lb);
-  static thread_local size_t smem_set[64] = {};
+  static thread_local bool opted[64] = {};
   int dev = 0;
   GS_CUDA_TRY(cudaGetDevice(&dev));
-  if (smem_set[dev & 63] < smem) {
-    GS_CUDA_TRY(cudaFuncSetAttribute(k_vert_scatter_sorted, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    smem_set[dev & 63] = smem;
+  if (!opted[dev & 63]) {
+    GS_TRY(gs_allow_shared_memory(k_vert_scatter_sorted, dev));
+    opted[dev & 63] = true;
   }
   k_vert_scatter_sorted<<<grid, kPartThreads, smem, s>>>(reinterpret_cast<const uint32_t*>(part), bkt, H, lb, nv,
                                                           cursor, nbr, cap, status, chunkhist);

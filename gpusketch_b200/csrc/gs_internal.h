@@ -221,6 +221,19 @@ struct GsCallerOrder {
   }
 };
 
+// Lets a kernel use all the dynamic shared memory that the current device has for it.  The limit belongs to the
+// kernel on that device, not to a handle or a host thread: every launcher asks for the same most, so that no
+// thread ever lowers what another one's launches need.
+template <typename Kernel>
+gs_status gs_allow_shared_memory(Kernel* kernel, int device) {
+  int most = 0;
+  cudaFuncAttributes fa{};
+  GS_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  GS_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
+  GS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes));
+  return GS_OK;
+}
+
 // Frees every buffer a handle owns, then the handle.
 void gs_free_graph(gs_graph* g);
 
