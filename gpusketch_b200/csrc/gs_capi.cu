@@ -580,7 +580,8 @@ gs_status gs_query_wait(gs_graph* g, uint32_t* labels, uint32_t* num_cc, uint32_
   g->last_answer_eager = false;
   // the partition stays valid for point queries only while no later call has changed the sketches
   g->labels_valid = g->changes == g->query_changes;
-  if (g->query_level == 0 && g->eager_on) GS_TRY(gs_eager_rebuild(g, g->stream));
+  // so does the DSU: when the sketches changed behind the query, its partition and forest are not theirs
+  if (g->query_level == 0 && g->eager_on && g->labels_valid) GS_TRY(gs_eager_rebuild(g, g->stream));
   if (rounds) *rounds = g->last_rounds;
   if (labels) std::memcpy(labels, g->h_qlabels, (size_t)V * sizeof(uint32_t));
   if (num_cc) *num_cc = g->last_components;
