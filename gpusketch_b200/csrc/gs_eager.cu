@@ -157,8 +157,9 @@ gs_status gs_eager_enable(gs_graph* g, bool on, cudaStream_t s) {
   }
   g->eager_on = true;
   // a handle that has ingested nothing is the empty graph, whose DSU is all singletons; otherwise the
-  // next query rebuilds the DSU with a Boruvka run
-  if (g->records_total == 0) return gs_eager_reset_empty(g, s);
+  // next query rebuilds the DSU with a Boruvka run.  (records_total alone does not tell: it starts again with
+  // the profile, and sketches can be uploaded.)
+  if (g->records_total == 0 && g->changes == g->changes_at_clear) return gs_eager_reset_empty(g, s);
   GS_CUDA_TRY(cudaMemsetAsync(g->d_eager_status, 0, 4 * sizeof(uint32_t), s));
   return gs_eager_invalidate(g, s);
 }

@@ -47,3 +47,36 @@ def test_switched_on_between_a_query_and_its_answer(restatement, between):
         _check(restatement, g, *parts, half)
         g.ingest_pairs(half)
         _check(restatement, g, *parts)
+
+
+@pytest.mark.parametrize("how", ["uploaded", "profiled", "read", "batches"])
+def test_switched_on_over_sketches_that_are_there(restatement, tmp_path, how):
+    """A handle whose record count says zero is not an empty graph when its sketches were uploaded or read from a
+    file, or when the profile was reset after the ingest."""
+    a = _path(0, 100)
+    with gs.GraphSketch(V, 9) as g:
+        g.ingest_pairs(a)
+        if how == "profiled":
+            g.synchronize()
+            g.profile_enable(False)
+            g.set_eager_dsu(True)
+            assert not g.has_cached_query()
+            _check(restatement, g, a)
+            return
+        g.write_binary(str(tmp_path / "g"))
+        sketches = g.download()
+    if how == "read":
+        h = gs.GraphSketch.read_binary(str(tmp_path / "g"))
+    else:
+        h = gs.GraphSketch(V, 9)
+        if how == "uploaded":
+            h.upload(sketches)
+        else:
+            src, dst = np.concatenate([a[:, 0], a[:, 1]]), np.concatenate([a[:, 1], a[:, 0]])
+            h.ingest_vertex_batches(src, np.arange(len(src), dtype=np.uint64), np.ones(len(src), np.uint64), dst)
+            h.synchronize()
+            h.profile_enable(False)
+    with h:
+        h.set_eager_dsu(True)
+        assert not h.has_cached_query()
+        _check(restatement, h, a)
