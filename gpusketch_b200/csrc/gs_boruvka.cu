@@ -1429,10 +1429,15 @@ GsBorScope gs_boruvka_scope(const uint32_t* V, uint32_t graphs) {
 
 gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, uint32_t* st) {
   if (st[0] & GS_DEV_ERR_TIMEOUT) {
-    // the words are still on the device
-    GS_CUDA_TRY(cudaMemcpy(st, g->d_status, 18 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    GS_CUDA_TRY(cudaMemset(g->d_status, 0, sizeof(uint32_t)));
+    // the words are still on the device, among them the error bits of calls queued behind the query, which stay
+    constexpr uint32_t kOwn = GS_DEV_ERR_TIMEOUT | GS_DEV_ERR_DSU_LIMIT;
+    GS_CUDA_TRY(cudaMemcpyAsync(st, g->d_status, 18 * sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream));
+    GS_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    const uint32_t later = st[0] & ~kOwn;
+    GS_CUDA_TRY(cudaMemcpyAsync(g->d_status, &later, sizeof(uint32_t), cudaMemcpyHostToDevice, g->stream));
+    GS_CUDA_TRY(cudaStreamSynchronize(g->stream));
     st[0] |= GS_DEV_ERR_TIMEOUT;
+    st[16] &= ~kOwn;   // a block gave up before the first one had moved the earlier calls' bits there
   }
   // records skipped by the ingest calls before the query are reported first
   if (st[16]) {

@@ -54,7 +54,8 @@ namespace {
 gs_status check_status(gs_graph* g, cudaStream_t s) {
   GS_CUDA_TRY(cudaMemcpyAsync(g->h_status, g->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   GS_CUDA_TRY(cudaStreamSynchronize(s));
-  const uint32_t bits = g->h_status[0];
+  uint32_t bits = g->h_status[0];
+  if (g->query_pending) bits &= ~(uint32_t)GS_DEV_ERR_TIMEOUT;   // the queued query's own: gs_query_wait reports it
   if (bits) {
     GS_CUDA_TRY(cudaMemsetAsync(g->d_status, 0, sizeof(uint32_t), s));
     GS_CUDA_TRY(cudaStreamSynchronize(s));
