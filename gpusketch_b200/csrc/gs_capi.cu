@@ -279,16 +279,18 @@ uint64_t host_slice(const gs_graph* g, uint64_t n) {
 gs_status ingest_host_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, bool wait_copies) {
   const cudaStream_t s = g->stream;
   bool pinned = false;
-  if (n > kZeroCopyPairs) {
+  if (n > kZeroCopyPairs || !wait_copies) {
     cudaPointerAttributes attr{};
     pinned = cudaPointerGetAttributes(&attr, pairs) == cudaSuccess && attr.type == cudaMemoryTypeHost;
     cudaGetLastError();
   }
   const uint64_t slice = host_slice(g, n);
   GS_TRY(gs_ensure_pair_staging(g, std::min(n, slice), !pinned));
-  if (n <= kZeroCopyPairs) {
+  if (n <= kZeroCopyPairs && !(pinned && !wait_copies)) {
     // a few records: copied into the ring by the host and read from there by the update's kernel, instead of
-    // a copy on another stream and the two events and the wait that tie it to this one
+    // a copy on another stream and the two events and the wait that tie it to this one.  A slot is free once the
+    // batch before the last one is ingested; asynchronous calls with page-locked input, which wait for nothing
+    // on the host, take the copies below
     const int slot = (int)(g->zero_copy_next++ & 1);
     GS_CUDA_TRY(cudaEventSynchronize(g->ev_done[slot]));
     GS_CUDA_TRY(cudaEventSynchronize(g->ev_copy[slot]));
