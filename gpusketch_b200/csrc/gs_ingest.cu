@@ -1707,8 +1707,16 @@ __global__ void __launch_bounds__(few_threads(CG), 3) k_ingest_few(const IngestA
 // Sketch update of a small batch, without grouping it: a warp per edge record, a lane per bucket (column j,
 // or the deterministic bucket at j = C), both endpoints' buckets XORed in HBM.  The depths are hashed once
 // for both endpoints.
+// Bound by L2 atomics; those on one bucket queue (1.3 ns each), and every record of a hub vertex meets at its
+// deterministic bucket, half of them at each column's first.  So a warp keeps the buckets of a vertex that the
+// next of its records names too - the deterministic one and the columns' first hub_depths depths - in shared
+// memory until another vertex repeats.  us per star of 65536 records without that, with it, and grouped: V = 8192
+// 174 65 147, V = 131072 474 177 272; random records as before (30, 119).  Holding them in registers is the same.
+constexpr int kDirectWarps = 8;
+constexpr uint32_t hub_depths(int cg) { return cg == 1 ? 4 : 2; }
+
 template <int CG, bool TEN>
-__global__ void __launch_bounds__(256) k_ingest_direct(const uint2* __restrict__ pairs, uint32_t n, PairTag tag,
+__global__ void __launch_bounds__(kDirectWarps * 32) k_ingest_direct(const uint2* __restrict__ pairs, uint32_t n, PairTag tag,
                                                        const IngestArgs A) {
   const uint32_t lane = lane_id();
   uint32_t C = A.C, bkt = A.bkt, nb = A.nb, cur_t = 0xffffffffu;
@@ -1727,12 +1735,30 @@ __global__ void __launch_bounds__(256) k_ingest_direct(const uint2* __restrict__
       for (int g = 0; g < CG; g++) cm[g] = gs_seed_mix(A.seed + 5ull * (lane + 32u * g));
     }
   }
+  constexpr uint32_t kNone = 0xffffffffu;
+  uint32_t hub = kNone;               // the vertex held, in the first level that its records reach
+  GsBucket* hub_sk = nullptr;
+  constexpr uint32_t kHubDepths = hub_depths(CG);
+  __shared__ ulonglong2 s_hub[kDirectWarps][CG * kHubDepths][32];   // its buckets, each lane its own
+  ulonglong2 (*const held)[32] = s_hub[threadIdx.x >> 5];
+  for (uint32_t r = 0; r < CG * kHubDepths; r++) held[r][lane] = make_ulonglong2(0, 0);
+  auto flush_hub = [&]() {
+    if (hub == kNone) return;
+#pragma unroll 1
+    for (uint32_t r = 0; r < CG * kHubDepths; r++) {
+      const uint32_t j = lane + 32u * (r / kHubDepths), k = r % kHubDepths;
+      const ulonglong2 b = held[r][lane];
+      if (!(b.x | b.y)) continue;
+      xor_bucket_global(hub_sk + (j < C ? j * bkt + k : nb - 1), b.x, b.y);
+      held[r][lane] = make_ulonglong2(0, 0);
+    }
+  };
   const uint32_t step = (gridDim.x * blockDim.x) >> 5;
   uint32_t e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  uint2 next = e < n ? pairs[e] : make_uint2(0u, 0u);
+  uint2 next = e < n ? pairs[e] : make_uint2(kNone, kNone);
   for (; e < n; e += step) {
     const uint2 p = next;
-    if (e + step < n) next = pairs[e + step];
+    next = e + step < n ? pairs[e + step] : make_uint2(kNone, kNone);
     int lo = 0, hi = -1;
     if (!record_levels(tag, p.x, p.y, &lo, &hi, A.status)) continue;
     uint32_t vb = 0;
@@ -1741,6 +1767,8 @@ __global__ void __launch_bounds__(256) k_ingest_direct(const uint2* __restrict__
       const uint32_t t = A.vtenant[p.x];
       const GsIngTenant T = A.tenants[t];
       if (t != cur_t) {
+        flush_hub();                  // in its own tenant's geometry
+        hub = kNone;
         cur_t = t;
         C = T.C;
         bkt = T.bkt;
@@ -1752,23 +1780,39 @@ __global__ void __launch_bounds__(256) k_ingest_direct(const uint2* __restrict__
     }
     const uint32_t u = p.x - vb, v = p.y - vb;
     const uint64_t id = gs_concat(u, v), E = gs_key_mix(id), cs = gs_hash_tail(E ^ csmix);
-    uint32_t at[CG];
+    uint32_t at[CG], depth[CG];       // depth: of the hub's held buckets, kHubDepths or more for none
 #pragma unroll
     for (int g = 0; g < CG; g++) {
       const uint32_t j = lane + 32u * g;
       const uint32_t d = gs_depth_from_mixed(E ^ cm[g], bkt);
-      at[g] = j < C ? (d < bkt ? j * bkt + d : 0xffffffffu) : j == C ? nb - 1 : 0xffffffffu;
+      at[g] = j < C ? (d < bkt ? j * bkt + d : kNone) : j == C ? nb - 1 : kNone;
+      depth[g] = j < C ? d : 0u;
     }
+    if (p.x != hub && p.y != hub && next.x != hub && next.y != hub) {
+      const bool x = p.x == next.x || p.x == next.y, y = p.y == next.x || p.y == next.y;
+      if (x || y) {
+        flush_hub();
+        hub = x ? p.x : p.y;
+        hub_sk = sk + ((size_t)lo * A.V + (hub - vb)) * nb;
+      }
+    }
+    const bool hold_u = p.x == hub, hold_v = p.y == hub;
     for (int l = lo; l <= hi; l++) {
       GsBucket* const lvl = sk + (size_t)l * A.V * nb;
 #pragma unroll
       for (int g = 0; g < CG; g++) {
-        if (at[g] == 0xffffffffu) continue;
-        xor_bucket_global(lvl + (size_t)u * nb + at[g], id, cs);
-        xor_bucket_global(lvl + (size_t)v * nb + at[g], id, cs);
+        if (at[g] == kNone) continue;
+        const bool keep = (hold_u || hold_v) && l == lo && depth[g] < kHubDepths;
+        if (keep) {
+          ulonglong2* const b = &held[g * kHubDepths + depth[g]][lane];
+          *b = make_ulonglong2(b->x ^ id, b->y ^ cs);
+        }
+        if (!(keep && hold_u)) xor_bucket_global(lvl + (size_t)u * nb + at[g], id, cs);
+        if (!(keep && hold_v)) xor_bucket_global(lvl + (size_t)v * nb + at[g], id, cs);
       }
     }
   }
+  flush_hub();
 }
 
 size_t ingest_smem_bytes(int cg, int r, int warps) {
@@ -1861,11 +1905,14 @@ gs_status launch_ingest_few(const IngestArgs& A, int num_sms, cudaStream_t s) {
 template <bool TEN>
 gs_status launch_ingest_direct(const IngestArgs& A, uint32_t cols, const uint2* p, uint32_t n, const PairTag& t,
                                int num_sms, cudaStream_t s) {
-  const unsigned grid = std::min<uint32_t>((n + 7) / 8, (uint32_t)num_sms * 8);
+  // half as many blocks for narrow sketches: a warp then meets a hub's records twice as often (a star of 65536
+  // records, V = 131072: 245 -> 177 us; random records the same)
+  const unsigned grid = std::min<uint32_t>((n + kDirectWarps - 1) / kDirectWarps, (uint32_t)num_sms * (cols < 32 ? 4 : 8));
+  constexpr int threads = kDirectWarps * 32;
   // a lane per bucket: the columns and the deterministic bucket
-  if (cols < 32) k_ingest_direct<1, TEN><<<grid, 256, 0, s>>>(p, n, t, A);
-  else if (cols < 64) k_ingest_direct<2, TEN><<<grid, 256, 0, s>>>(p, n, t, A);
-  else k_ingest_direct<3, TEN><<<grid, 256, 0, s>>>(p, n, t, A);
+  if (cols < 32) k_ingest_direct<1, TEN><<<grid, threads, 0, s>>>(p, n, t, A);
+  else if (cols < 64) k_ingest_direct<2, TEN><<<grid, threads, 0, s>>>(p, n, t, A);
+  else k_ingest_direct<3, TEN><<<grid, threads, 0, s>>>(p, n, t, A);
   GS_CUDA_TRY(cudaGetLastError());
   return GS_OK;
 }
@@ -2114,8 +2161,10 @@ static gs_status ingest_grouped(gs_graph* g, uint32_t nv, cudaStream_t s) {
 
 // Batches of at most this many edge records are not grouped by vertex.  Grouping costs about ten launches
 // and the smallest of its kernels' times (50 us) whatever the batch; a direct update costs four 64-bit
-// atomics per column.  us per batch of 2^13 / 2^16 / 2^18 records, grouped and direct: V = 8192 62 76 107 and
-// 9 31 111, V = 131072 71 150 246 and 8 113 460, V = 1000003 109 251 615 and 9 157 638.
+// atomics per column.  us per batch of 2^13 / 2^16 / 2^18 random records, grouped and direct: V = 8192 62 76 107
+// and 9 31 111, V = 131072 71 150 246 and 8 113 460, V = 1000003 109 251 615 and 9 157 638.  Hubs are the direct
+// update's worst: 2^16 records over V = 131072 with one, two and four of them 272 296 304 and 177 287 235, over
+// V = 1000003 435 437 438 and 212 335 280.
 constexpr uint64_t kDirectEdges = 65536;
 
 static int grid_for(gs_graph* g, uint64_t work_items, int threads) {
