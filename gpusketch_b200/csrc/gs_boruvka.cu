@@ -1427,6 +1427,15 @@ GsBorScope gs_boruvka_scope(const uint32_t* V, uint32_t graphs) {
   return best;
 }
 
+// A cluster holds its SMs for about 45 + 0.11 V us however small its graph is, and 148 run at once; one grid launch
+// over all graphs takes about 230 us and 1 us for 1000 ids of its range.  Measured (us, clusters / grid): 4096
+// graphs of 64 vertices 1574 / 522, of 256 2187 / 1235; 2048 of 64 797 / 324; 1024 of 64 423 / 285, of 256 599 /
+// 518, of 1000 1061 / 1256; 512 of 64 238 / 243; 256 of 64 147 / 232.  (The launch before, one grid for all: 834,
+// 1771, 568, 534, 793, 1872, 462, 392.)
+bool gs_boruvka_shares_grid(uint32_t graphs, uint64_t vertices, uint64_t span) {
+  return (45.0 * graphs + 0.11 * (double)vertices) / 148 > 230 + 0.001 * (double)span;
+}
+
 gs_status gs_boruvka_finish(gs_graph* g, uint32_t level, uint32_t* st) {
   if (st[0] & GS_DEV_ERR_TIMEOUT) {
     // the words are still on the device, among them the error bits of calls queued behind the query, which stay

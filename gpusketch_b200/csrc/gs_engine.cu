@@ -309,12 +309,21 @@ gs_status enqueue_query(gs_engine* e, const QueryPlan& qp, const uint32_t* tenan
     GS_CUDA_TRY(cudaMemsetAsync(g->d_acc, 0, (size_t)e->max_vertices * e->W * sizeof(GsBucket), s));
   g->acc_dirty = true;
   // the large graphs share the whole GPU, the others run on a cluster each, the largest first (a launch ends
-  // when its last cluster does)
+  // when its last cluster does); when there are very many of them, they share the grid launch as well
   uint32_t* order = e->h_q + 2 * (size_t)T1;
   std::copy(tenants, tenants + count, order);
   std::stable_sort(order, order + count, [&](uint32_t a, uint32_t b) { return e->ten[a].V > e->ten[b].V; });
   uint32_t large = 0;
   while (large < count && e->ten[order[large]].V > (count == 1 ? 8192u : kGsBorClusterV)) large++;
+  uint32_t vlo = 0xffffffffu, vhi = 0;
+  uint64_t small_vertices = 0;
+  for (uint32_t i = 0; i < count; i++) {
+    const EngTenant& t = e->ten[order[i]];
+    vlo = std::min(vlo, t.vbase);
+    vhi = std::max(vhi, t.vbase + t.V);
+    if (i >= large) small_vertices += t.V;
+  }
+  if (gs_boruvka_shares_grid(count - large, small_vertices, vhi - vlo)) large = count;
   if (large > 1) {
     for (uint32_t t = 0; t < T1; t++) e->h_tstate[4 * t] = 1;
     for (uint32_t i = 0; i < large; i++) std::memset(e->h_tstate + 4 * order[i], 0, 4 * sizeof(uint32_t));

@@ -352,6 +352,8 @@ struct GsBorLaunch {
 constexpr uint32_t kGsBorClusterV = 16384;
 GsBorScope gs_boruvka_scope(uint32_t V);
 GsBorScope gs_boruvka_scope(const uint32_t* V, uint32_t graphs);
+// Whether several such graphs, of `vertices` vertices together and within `span` ids, share one grid launch instead.
+bool gs_boruvka_shares_grid(uint32_t graphs, uint64_t vertices, uint64_t span);
 // Bytes of GsBorLaunch::many for tables of T1 tenants.
 inline size_t gs_boruvka_many_bytes(uint32_t T1) { return (size_t)T1 * 2 * (sizeof(uint64_t) + sizeof(uint32_t)); }
 // The Boruvka scratch of a handle over `vertices` vertices with accumulator rows of `width` buckets.
