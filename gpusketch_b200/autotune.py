@@ -14,6 +14,10 @@ from ._native import check, lib
 
 _CACHE: dict[tuple, tuple] = {}
 
+# Batches of at most this many records are XORed in without the kernels that are tuned here (kDirectEdges in
+# csrc/gs_ingest.cu): no candidate differs on them, and the fastest would be the noise's choice.
+DIRECT_RECORDS = 65536
+
 
 class GsTuning(C.Structure):
     _fields_ = [("chunk", C.c_uint32), ("warps_per_block", C.c_uint32), ("reg_depth", C.c_uint32),
@@ -46,11 +50,16 @@ def set_tuning(g, chunk: int, warps_per_block: int, reg_depth: int) -> None:
 def autotune(g, sample_pairs, chunks=(256, 512, 1024, 2048), warps=(8, 12, 16), reg_depths=(0, 1),
              repeats: int = 2, table: list | None = None) -> dict:
     """Times every candidate on `sample_pairs` (a CUDA tensor of records) and applies the fastest.
-    The sketches are restored afterwards: each candidate ingests the sample twice (XOR cancels)."""
+    The sketches are restored afterwards: each candidate ingests the sample twice (XOR cancels).
+    A sample that the tuned kernels do not see (DIRECT_RECORDS records or fewer, or a handle whose passes are
+    that small) leaves the handle's parameters as they are and returns them."""
+    if int(sample_pairs.shape[0]) <= DIRECT_RECORDS:
+        return get_tuning(g)
     key = (g.geometry.num_columns, g.geometry.bkt_per_col, int(sample_pairs.shape[0]))
     if key in _CACHE:
         set_tuning(g, *_CACHE[key])
         return dict(zip(("chunk", "warps_per_block", "reg_depth"), _CACHE[key]))
+    kept = get_tuning(g)
     best, best_ms = None, float("inf")
     for chunk, w, r in itertools.product(chunks, warps, reg_depths):
         set_tuning(g, chunk, w, r)
@@ -58,7 +67,12 @@ def autotune(g, sample_pairs, chunks=(256, 512, 1024, 2048), warps=(8, 12, 16), 
         for _ in range(repeats):
             g.ingest_pairs(sample_pairs)
             g.ingest_pairs(sample_pairs)
-        ms = g.profile_read()["ingest_ms"]
+        profile = g.profile_read()
+        if profile["bucket_launches"] == 0:      # nothing was grouped by vertex
+            g.profile_enable(False)
+            set_tuning(g, **kept)
+            return kept
+        ms = profile["ingest_ms"]
         if table is not None:
             table.append({"chunk": chunk, "warps_per_block": w, "reg_depth": r, "ingest_ms": ms / (2 * repeats)})
         if ms < best_ms:
@@ -74,7 +88,9 @@ def autotune_engine(e, slice_tenants, slice_offsets, pairs, chunks=(128, 256, 51
     """Engine variant: times the multi-tenant sketch update on one batch of device-resident slices
     (ingested twice per candidate, so the tenants' sketches are unchanged) and applies the fastest.
     Tile size = records per work item, vertices per block = warps per block (a warp owns one vertex
-    chunk), update-buffer depth = bucket depths kept in registers."""
+    chunk), update-buffer depth = bucket depths kept in registers.  Few records: as in autotune."""
+    if int(slice_offsets[-1]) - int(slice_offsets[0]) <= DIRECT_RECORDS:
+        return get_tuning(e)
     best, best_ms = None, float("inf")
     for chunk, w, r in itertools.product(chunks, warps, reg_depths):
         set_tuning(e, chunk, w, r)
