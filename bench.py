@@ -607,20 +607,26 @@ def run_gs(args):
     ms_per_step = ms_max / args.steps
     value = whole_job_rate(sum_over_ranks(U * args.steps, dist, dev), ms_max)
 
-    # roofline of the dominant kernel (the sketch update), per launch: B_edge = 8 + 2*V*S_v/U_phase
-    # bytes per edge update (the read half dropped for the first phase of a step, whose sketches are 0)
+    # roofline of a phase's sketch update: B_edge = 8 + 2*V*S_v/U_phase bytes per edge update (the read half
+    # dropped for the first phase of a step, whose sketches are 0) over the time of every kernel between the
+    # records and the sketches, because records that cancel are read and dropped before the update kernels
     Sv = geo.bytes_per_vertex
     alg_step = 8.0 * U + V * Sv * (2 * P - 1)
     alg_per_launch = alg_step / P
-    ingest_ms_avg = prof["ingest_ms"] / (args.steps * P)     # a phase's update: k_ingest_few and k_ingest_packed
-    achieved = alg_per_launch / (ingest_ms_avg / 1e3) / 1e9
+    ingest_ms_avg = prof["ingest_ms"] / (args.steps * P)     # k_ingest_few and k_ingest_packed of a phase
+    update_ms_avg = ingest_ms_avg + prof["bucket_ms"] / (args.steps * P)
+    achieved = alg_per_launch / (update_ms_avg / 1e3) / 1e9
     peak, peak_kind = measured_peak_hbm()
     traffic, traffic_current = ncu_traffic_per_launch()
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "traffic_source": "committed ncu capture (profiles/k_ingest_rmat17_traffic.txt)",
-                "traffic_capture_matches_source": traffic_current, "peak_source": peak_kind,
-                "kernel": "k_ingest_packed (sketch update)", "alg_bytes_per_launch": alg_per_launch,
-                "avg_launch_ms": ingest_ms_avg, "path_frac": value / world * (alg_step / U) / 1e9 / peak}
+                "kernel": "a phase's sketch update: bucketing, k_parity, k_ingest_few, k_ingest_packed",
+                "alg_bytes_per_launch": alg_per_launch, "avg_launch_ms": update_ms_avg, "peak_source": peak_kind,
+                "traffic": traffic, "traffic_kernel": "k_ingest_packed",
+                "traffic_frac": traffic / (ingest_ms_avg / 1e3) / 1e9 / peak if traffic else None,
+                "traffic_ms": ingest_ms_avg,
+                "traffic_source": "committed ncu capture (profiles/k_ingest_rmat17_traffic.txt)",
+                "traffic_capture_matches_source": traffic_current,
+                "path_frac": value / world * (alg_step / U) / 1e9 / peak}
     # the sketch update is bound by instruction issue: its measured warp instructions per launch
     # (one-pass ncu count of this workload's launch) against 4 schedulers x SMs x the sampled SM clock
     issue = None
@@ -631,7 +637,7 @@ def run_gs(args):
         pk = 4.0 * sms * clocks["sm_mhz"] * 1e6
         issue = {"bound": "issue", "achieved": ach, "peak": pk, "unit": "warp_inst/s", "frac": ach / pk,
                  "inst_per_launch": inst, "inst_source": "committed ncu capture (profiles/k_ingest_rmat17_issue.txt)",
-                 "inst_capture_matches_source": inst_current, "kernel": "k_ingest_packed (sketch update)",
+                 "inst_capture_matches_source": inst_current, "kernel": "k_ingest_packed (its time with k_ingest_few's)",
                  "peak_source": f"4 schedulers x {sms} SMs x median sampled SM clock"}
     # ... and by shared-memory bandwidth: every (record, column) reads and writes a 16-byte row and every
     # record is broadcast from the warp's stage; one wavefront (128 B) per SM and clock is the peak
@@ -644,7 +650,8 @@ def run_gs(args):
         smem = {"bound": "shared-memory wavefronts", "achieved": ach, "peak": pk, "unit": "wavefronts/s",
                 "frac": ach / pk, "wavefronts_per_launch": wf,
                 "wavefront_source": "committed ncu capture (profiles/k_ingest_rmat17_issue.txt)",
-                "wavefront_capture_matches_source": wf_current, "kernel": "k_ingest_packed (sketch update)",
+                "wavefront_capture_matches_source": wf_current,
+                "kernel": "k_ingest_packed (its time with k_ingest_few's)",
                 "peak_source": f"one 128-byte wavefront per SM and clock x {sms} SMs x median sampled SM clock"}
     split = {"ingest_ms_per_step": prof["ingest_ms"] / args.steps, "bucket_ms_per_step": prof["bucket_ms"] / args.steps,
              "query_ms_per_step": prof["query_ms"] / args.steps}
