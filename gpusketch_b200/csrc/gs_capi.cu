@@ -255,14 +255,15 @@ uint64_t gs_desired_updates_per_batch(const gs_graph* g) {
 
 namespace {
 
-// Records in one slice of host input: 64 per vertex or an eighth of the call's, rounded up to a power of two.
-// A slice's copy overlaps the ingest of the one before, so small slices leave little to do when the last copy
-// lands; but each slice merges the rows of all vertices that it touches, toggles that cancel are only found
-// within one, and copies that follow one another without end (asynchronous calls of 2^27 records) lose about
-// 30 us to each: 157.7 ms per 2^30 records in slices of 2^23, 155.5 of 2^24, 155.7 of 2^25.  ms for 2^25 R-MAT
-// records and the query with slices of 2^22 / 2^23 / 2^24 / 2^25:
+// Records in one slice of host input: 64 per vertex or an eighth of the call's, rounded up to a power of two,
+// from 2^22 to 2^24.  A slice's copy overlaps the ingest of the one before, so small slices leave little to do
+// when the last copy lands; but each slice merges the rows of all vertices that it touches, toggles that cancel
+// are only found within one, and copies that follow one another without end (asynchronous calls of 2^27 records)
+// lose about 30 us to each: 157.7 ms per 2^30 records in slices of 2^23, 155.5 of 2^24, 155.7 of 2^25.  ms for
+// 2^25 R-MAT records and the query with slices of 2^22 / 2^23 / 2^24 / 2^25:
 //   V = 2^14: 5.55 / 5.65 / 5.91 / 6.31    V = 2^17: 6.33 / 6.25 / 6.67 / 7.40
 //   V = 2^18: 8.79 / 7.00 / 7.54 / 8.65    V = 2^20: 15.23 / 12.20 / 10.47 / 11.70
+// (At V = 2^18 the rule takes 2^24, half a millisecond behind 2^23; 64 per vertex fits the other three.)
 uint64_t host_slice(const gs_graph* g, uint64_t n) {
   const uint64_t want = std::max<uint64_t>(64ull * g->V, n / 8);
   uint64_t m = 1ull << 22;
@@ -334,8 +335,10 @@ constexpr uint64_t al16(uint64_t x) { return (x + 15) & ~15ull; }
 // Host per-vertex batches move through the same staging slots as host pairs, so a call allocates
 // nothing: the batches are cut into chunks that fit one slot (a batch longer than the room left is
 // split; XOR makes the pieces equivalent to the whole), each chunk's headers and destinations are
-// gathered into the slot's page-locked half - starts rebased to the gathered destinations - copied to
-// the device half and ingested while the next chunk is gathered.
+// gathered into the slot's page-locked half - starts rebased to the gathered destinations - and then
+// copied to the device half and ingested.  The ring grows with the calls, so most calls are one chunk,
+// whose gather, copy and ingest follow one another; the copy of the headers covers all that a slot has
+// room for.
 gs_status ingest_host_batches(gs_graph* g, uint32_t level, const uint32_t* srcs, const uint64_t* starts,
                               const uint64_t* sizes, uint32_t nbat, const uint32_t* dsts) {
   const cudaStream_t s = g->stream;

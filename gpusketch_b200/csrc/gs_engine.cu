@@ -7,8 +7,9 @@
 // sketch-update kernel's tenant variant reads each work chunk's geometry, column constants and
 // arena offset from the tenant table, so a tenant's buckets get exactly the XORs a gs_graph with
 // the same V, seed and sketches_factor would get (src/cc_sketch_alg.cpp:154-160, src/sketch.cpp:
-// 110-131 of the reference).  A query runs the persistent Boruvka kernel over the listed tenants
-// in one cooperative launch; the others are marked done before it starts.
+// 110-131 of the reference).  A query runs the persistent Boruvka kernels over the listed tenants in at most
+// two launches: one for the small ones, on a thread-block cluster each, and a cooperative one for the large
+// ones (or for all, when there are very many), which share the whole GPU.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -158,7 +159,7 @@ struct gs_engine {
   uint32_t* d_vtenant = nullptr; // [max_vertices]
   uint32_t* d_tstate = nullptr;  // [(max_tenants + 1) * 4] Boruvka per-tenant state
   uint32_t* h_tstate = nullptr;  // pinned mirror
-  void* d_many = nullptr;        // tables of a Boruvka launch over several large tenants
+  void* d_many = nullptr;        // tables of a Boruvka grid launch over several tenants
   uint32_t* d_qstatus = nullptr; // [16] Boruvka status words
   uint32_t* h_qstatus = nullptr; // pinned [16]
   uint32_t* d_q = nullptr;       // [3 * (max_tenants + 1)] query list, label offsets, query list by size

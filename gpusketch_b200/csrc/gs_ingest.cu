@@ -26,8 +26,8 @@
 //                                    records with 32 lanes in three steps; k_ingest (wider sketches,
 //                                    register depths) keeps lane = column.  At the end of the chunk
 //                                    the non-zero rows and the deterministic bucket are merged into
-//                                    the vertex sketch (plain read-modify-write when the vertex is
-//                                    one chunk, atomic XOR when several warps share it).
+//                                    the vertex sketch (k_ingest_packed: atomic XOR; k_ingest: plain
+//                                    read-modify-write when the vertex is one chunk, else atomic XOR).
 //
 // Batches that come per vertex (directed) are grouped by k_count_batches, k_scan_* and
 // k_scatter_batches, and take steps 6 and 7.
@@ -1256,7 +1256,8 @@ __global__ void __launch_bounds__(512) k_ingest(const IngestArgs A) {
 }
 
 // Sketch update with the packed lane layout (reg_depth 0, at most 32 columns); chunk lookup, record
-// staging, deep-bucket path and merge as in k_ingest.
+// staging and deep-bucket path as in k_ingest.  The merge is by atomic XORs always: no load waits for a
+// bucket's old value, and vertices small enough to saturate the L2 atomics are k_ingest_few's.
 template <bool TEN>
 __global__ void __launch_bounds__(kPackMaxThreads, 2) k_ingest_packed(const IngestArgs A) {
   extern __shared__ uint4 smem[];

@@ -252,7 +252,7 @@ struct GsProfScope {
 // Partial-support helpers implemented in the .cu files.
 gs_status gs_ensure_ingest_scratch(gs_graph* g, uint64_t records);
 // The staging ring (two slots, with `host` also its page-locked side) for host slices of up to `want` pairs, grown
-// as needed up to min(max_batch_edges, 2^25); UINT64_MAX sizes it at that limit.
+// as needed up to max(1024, min(max_batch_edges, 2^25)); UINT64_MAX sizes it at that limit.
 gs_status gs_ensure_pair_staging(gs_graph* g, uint64_t want = ~0ull, bool host = true);
 // Sizes the single-level ingest scratch for batches of `edges` records, so that a later ingest of
 // at most that many records allocates nothing (required while a stream is being captured).
@@ -348,7 +348,8 @@ struct GsBorLaunch {
   uint32_t complement = 0;
 };
 
-// The scope of a query of one graph of V vertices, and of several of at most kGsBorClusterV each.
+// The scope of a query of one graph of V vertices, and of several of at most kGsBorClusterV each.  (Only the grid's
+// waits have a limit: a cluster's blocks are resident together, and its barrier is the hardware's.)
 constexpr uint32_t kGsBorClusterV = 16384;
 GsBorScope gs_boruvka_scope(uint32_t V);
 GsBorScope gs_boruvka_scope(const uint32_t* V, uint32_t graphs);

@@ -5,7 +5,8 @@
 // started), so every cudaMalloc would step outside the budget they were given.  This entry point
 // serves them: the caller passes the records and its own sketch buffer.  A call has at most
 // GS_NOALLOC_MAX_EDGES records, which the direct update XORs into the sketches without grouping them by
-// vertex (65536 records, V = 8191, and the clearing of its buffer: 115 us grouped, 61 direct), so all that is kept in device memory is one file-scope error word.
+// vertex (65536 records, V = 8191, and the clearing of its buffer: 119 us grouped, 60 direct), so all that
+// is kept in device memory is one file-scope error word.
 //
 // In host code the name g_noalloc_status is only a host-side stand-in for the word: every call asks the
 // runtime for its device address on the current device (cudaGetSymbolAddress, with that device current)

@@ -4,7 +4,7 @@ Binds the gs_engine_* entry points of include/gpusketch.h.  Every tenant's sketc
 to a GraphSketch (and the reference's CCSketchAlg) with the same num_vertices, seed and
 sketches_factor fed the same records; an ingest call carries record slices of many tenants and
 runs the bucketing and the sketch update once for all of them, and a query answers
-connected_components() for a list of tenants with one device Boruvka launch.
+connected_components() for a list of tenants with one or two device Boruvka launches.
 """
 from __future__ import annotations
 

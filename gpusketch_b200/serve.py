@@ -8,7 +8,7 @@ host records, connectivity queries) are admitted as they arrive:
   budget) into ONE engine ingest call: one host->device copy, one bucketing pass and one sketch
   update over all of them, the copies of the next slice overlapping the kernels of the previous;
 * queries waiting at that point are answered between batches, all of them with ONE multi-tenant
-  Boruvka launch;
+  query;
 * a tenant whose last request was served is checkpointed (optional) and removed, freeing its
   arena range for tenants still waiting for admission.
 
@@ -181,7 +181,7 @@ class SketchServer:
                     remaining[t] -= 1
                     if remaining[t] == 0:
                         done_tenants.append(t)
-            # ---- queries between batches: one multi-tenant Boruvka launch ----
+            # ---- queries between batches: one multi-tenant query ----
             if queries:
                 tens = sorted({reqs[i].tenant for i in queries})
                 res = eng.connected_components([slot[t] for t in tens], with_labels=self.keep_labels)

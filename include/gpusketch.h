@@ -127,8 +127,10 @@ gs_status gs_ingest_pairs(gs_graph* g, const uint32_t* pairs, uint64_t n, int pa
                           void* cuda_stream);
 
 /* Allocates now what host input needs - the page-locked staging ring for slices of up to `records`
- * records (at most min(max_batch_edges, 2^25)) and the stream-file decode buffer - instead of at the
- * first host ingest; page-locking hundreds of megabytes takes tens of milliseconds.  Library extension
+ * records (at most min(max_batch_edges, 2^25), at least 1024) and the stream-file decode buffer -
+ * instead of at the first host ingest; page-locking hundreds of megabytes takes tens of milliseconds.
+ * Record pairs move in slices of at most 2^24, stream files in slices as large as the ring: for pairs
+ * alone, more than 2^24 records ask for memory that is not used.  Library extension
  * (the reference's CCGPUSketchAlg constructor sets up its CudaStream buffers the same way,
  * include/cc_gpu_sketch_alg.h:36-95). */
 gs_status gs_prepare_host_input(gs_graph* g, uint64_t records);
@@ -276,12 +278,16 @@ gs_status gs_set_eager_dsu(gs_graph* g, int enable);
 gs_status gs_has_cached_query(gs_graph* g, int* cached);
 
 /* ---- bounded device-side waits ----
- * Every wait of a device kernel on other blocks (the grid barriers of the persistent Boruvka kernel)
- * gives up after a limit, sets a device error bit and lets the kernel return, so a wait that cannot
- * end leaves the context usable: the query then fails with GS_ERR_TIMEOUT and the next query starts
- * from scratch.  Sets that limit for this handle's queries (summed sleep time of one wait; default
- * about one second; 0 restores the default).  Library extension without a reference counterpart;
- * the tests set a limit far below one barrier's normal wait to make a wait run out. */
+ * Every wait of a device kernel on blocks of the whole GPU (the grid barriers of the persistent Boruvka
+ * kernel) gives up after a limit, sets a device error bit and lets the kernel return, so a wait that
+ * cannot end leaves the context usable: the query then fails with GS_ERR_TIMEOUT and the next query
+ * starts from scratch.  Graphs of up to 8192 vertices, and engine tenants of up to 16384, are queried on
+ * thread-block clusters instead: a cluster's blocks are resident together and meet at the hardware's
+ * barrier, which has no limit to set.  Sets the limit for this handle's queries (summed sleep time of
+ * one wait; default about one second; 0 restores the default); with a limit of its own a handle is
+ * queried on the whole GPU whatever its size, so that the limit holds.  Library extension without a
+ * reference counterpart; the tests set a limit far below one barrier's normal wait to make a wait run
+ * out. */
 gs_status gs_set_device_wait_limit(gs_graph* g, uint64_t nanoseconds);
 
 /* ---- tuning (set by the autotuner, gpusketch_b200/autotune.py) ---- */
@@ -395,7 +401,7 @@ gs_status gs_engine_ingest_slices(gs_engine* e, uint32_t num_slices, const uint3
                                   const uint64_t* slice_counts, const uint32_t* const* slice_pairs,
                                   void* cuda_stream);
 gs_status gs_engine_synchronize(gs_engine* e);
-/* connected_components() of `count` distinct tenants in one device Boruvka launch.  labels
+/* connected_components() of `count` distinct tenants in one or two device Boruvka launches.  labels
  * (host, may be NULL) receives each listed tenant's V labels back to back in list order, each the
  * smallest tenant-local vertex id of its component; num_cc[i] and rounds[i] (may be NULL) are the
  * component count and Boruvka rounds of tenants[i].  GS_ERR_SKETCH_FAIL when a listed tenant ran
