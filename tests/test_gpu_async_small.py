@@ -15,14 +15,17 @@ def test_small_page_locked_batches_wait_for_nothing(restatement, n):
     r = np.random.default_rng(n)
     pairs = r.integers(0, V, size=(20 * n, 2), dtype=np.uint32)
     host = torch.from_numpy(pairs.view(np.int32)).pin_memory()
-    side = torch.cuda.Stream()
+    side, big = torch.cuda.Stream(), torch.zeros(1 << 28, device="cuda")
+    torch.cuda.synchronize()
     with gs.GraphSketch(V, seed) as g:
         g.set_stream(side)
         for _ in range(4):
             g.ingest_pairs_async(host[:n])
         g.synchronize()
-        for _ in range(2000):                       # the device is at least ten milliseconds behind
-            g.clear()
+        g.clear()
+        with torch.cuda.stream(side):
+            for _ in range(60):                     # 2 GB each: the device is at least ten milliseconds behind
+                big.add_(1)
         behind = torch.cuda.Event()
         behind.record(side)
         for i in range(20):

@@ -12,7 +12,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("second", ["pairs", "small", "file", "batches"])
 @pytest.mark.parametrize("first", ["pairs", "small", "file", "batches"])
 def test_a_queued_copy_is_made_before_its_slot_is_written(restatement, tmp_path, first, second):
+    import torch
     V, seed = 4096, 0x5EED5300
+    side, big = torch.cuda.Stream(), torch.zeros(1 << 28, device="cuda")
+    torch.cuda.synchronize()
     r = np.random.default_rng(53)
     data = []
     for i in range(2):
@@ -30,6 +33,8 @@ def test_a_queued_copy_is_made_before_its_slot_is_written(restatement, tmp_path,
 
     made = [batches(p) for p in data]
     with gs.GraphSketch(V, seed) as g:
+        g.set_stream(side)
+
         def put(i):
             kind = (first, second)[i]
             if kind == "file":
@@ -42,8 +47,9 @@ def test_a_queued_copy_is_made_before_its_slot_is_written(restatement, tmp_path,
         for i in (0, 1, 0, 1):                # everything is allocated; all of it cancels
             put(i)
         g.synchronize()
-        for _ in range(200):                  # the device is some milliseconds behind
-            g.clear()
+        with torch.cuda.stream(side):
+            for _ in range(60):               # 2 GB each: the device is at least ten milliseconds behind
+                big.add_(1)
         g.connected_components_async()
         put(0)
         put(1)
